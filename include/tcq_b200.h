@@ -67,10 +67,11 @@ TCQ_API const char *tcq_last_cuda_error(void);
 
 /*
  * Scratch sizing.  tcq_workspace_bytes(): the size with which tcq_encode_tb /
- * tcq_viterbi_pass process n_tiles at full speed (backpointers of up to one
- * chunk of tiles, K bits per trellis edge per step, plus per-tile hand-off
- * words).  tcq_workspace_min_bytes(): the smallest accepted size (one tile per
- * SM-resident group); anything in between just means smaller chunks.
+ * tcq_viterbi_pass process n_tiles at full speed (path metrics of every fifth,
+ * third or second step (K = 2, 3, 4) of up to one chunk of tiles, plus per-tile
+ * hand-off words).  tcq_workspace_min_bytes(): the smallest accepted size (one
+ * tile); anything in between means smaller chunks, or metrics of a half or a
+ * quarter of the path at a time, for which the sweep is repeated.
  * Replaces the per-batch torch.empty scratch of
  * src/trellis/viterbi_triton.py:96-102.  Returns 0 for invalid K.
  */
@@ -133,7 +134,7 @@ TCQ_API int tcq_viterbi_pass(const float *w, int64_t n_tiles, int K, int codeboo
  * tcq_encode_tb for callers that cannot allocate device memory (no counterpart in the
  * reference, which allocates its scratch with torch.empty on every call).
  * Same inputs, outputs and results as tcq_encode_tb, but no workspace argument: the
- * backpointer scratch is a fixed TCQ_STATIC_SCRATCH_BYTES array inside the library's device
+ * scratch is a fixed TCQ_STATIC_SCRATCH_BYTES array inside the library's device
  * image, so the call performs no cudaMalloc / cudaFree and uses no allocating library.
  *   - at most tcq_encode_tb_static_max_tiles(K) tiles per call (31 / 42 / 63 for K = 2 / 3 / 4);
  *     more returns TCQ_E_TOO_MANY_TILES and launches nothing;
@@ -156,12 +157,13 @@ TCQ_API int tcq_encode_tb_static_status(void *stream);
 
 /*
  * The forward sweep of one pass alone (no traceback): runs the Viterbi step kernel
- * exactly as tcq_encode_tb does for one chunk and leaves the packed backpointers of
- * the last bp_steps steps (256, or 128 as in the encoder's first pass) in `ws`.
+ * exactly as tcq_encode_tb does, chunk by chunk, each leaving what a walk over
+ * the last bp_steps steps (256, or 128 as in the encoder's first pass) needs in `ws`.
  * For profiling and roofline measurements of the step kernel; it replaces the
  * same reference code as tcq_viterbi_pass (src/trellis/qtip.py:177-182,
- * src/trellis/viterbi_triton.py:24-78).  n_tiles must fit one chunk of the
- * workspace (otherwise TCQ_E_WORKSPACE).
+ * src/trellis/viterbi_triton.py:24-78).  The workspace must hold n_tiles *
+ * tcq_workspace_min_bytes(K) or so, and n_tiles be at most 24 per SM (otherwise
+ * TCQ_E_WORKSPACE).
  */
 TCQ_API int tcq_forward_pass(const float *w, int64_t n_tiles, int K, int codebook, const int32_t *overlap, int roll,
                              int bp_steps, void *ws, size_t ws_bytes, void *stream);
@@ -189,7 +191,8 @@ TCQ_API int tcq_selftest_wait_timeout(const float *w, int64_t n_tiles, int K, vo
 
 /*
  * Number of kernel launches tcq_encode_tb issues for n_tiles with a workspace of
- * ws_bytes (four per chunk: step kernel and traceback for each of the two passes),
+ * ws_bytes (four per chunk: step kernel and traceback for each of the two passes;
+ * six or twelve where the workspace holds a half or a quarter of a path only),
  * or a negative TCQ_E_* code.  No reference counterpart; used for accounting.
  */
 TCQ_API int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes);

@@ -4,7 +4,9 @@
 #include "../../include/tcq_b200.h"
 
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <iterator>
 
 #include "tcq_forward.cuh"
 #include "tcq_traceback.cuh"
@@ -35,67 +37,248 @@ int current_num_sms(int* out) {
     return TCQ_OK;
 }
 
+// How many clusters of C CTAs of the step kernel the current device runs at once (one CTA per SM); 0: none.
+int clusters_at_once(int C) {
+    static int cache[64][17] = {};                 // per device ordinal and C: 0 not known yet, -1 none
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || C < 2 || C > 16) return 0;
+    const bool cached = dev >= 0 && dev < 64;
+    int n = cached ? cache[dev][C] : 0;
+    if (n == 0) {
+        ClusterArgs ca{};                          // no tiles: a query.  One CTA fits an SM whatever K and the tiles per group are.
+        ca.at_once = &n;
+        const cudaError_t err = launch_forward_cluster<2>(kCbMcg, ca, C, 1, nullptr);
+        if (err != cudaSuccess) (void)cudaGetLastError();
+        if (err == cudaErrorNotSupported) n = -1;
+        if (cached) cache[dev][C] = n;             // a failed query leaves 0: it says nothing about the device
+    }
+    return n > 0 ? n : 0;
+}
+
+// Whether the cluster step kernel runs on the current device (TCQ_FORWARD_KERNEL=cta: the single-CTA form is asked for).
+bool cluster_available() {
+    const char* v = std::getenv("TCQ_FORWARD_KERNEL");
+    return !(v != nullptr && std::strcmp(v, "cta") == 0) && clusters_at_once(2) > 0;
+}
+
+// How a batch is spread over the chip: clusters of C CTAs, G tiles each, and the time of one round of a 256-step sweep with
+// all SMs of a B200 at work, measured.  A larger cluster divides a tile's step over more SMs, which shortens the step for
+// the few tiles that then fit, no further than the exchange of metrics between SMs allows (0.4 us a step); more tiles per
+// cluster share the step's fixed cost (0.35 us with two SMs; 0.45 us a tile beyond that at K = 3).
+struct ClusterShape { int C, G; double us; };
+constexpr ClusterShape kShapes2[] = {{16, 1, 100}, {8, 1, 124}, {8, 2, 175}, {4, 1, 181}, {4, 2, 260}, {2, 1, 240}, {2, 2, 398}, {2, 3, 532}};
+constexpr ClusterShape kShapes3[] = {{8, 1, 107}, {8, 2, 150}, {4, 1, 152}, {4, 2, 205}, {2, 1, 223}, {2, 2, 337}, {2, 3, 460}, {2, 4, 558}, {2, 5, 690}, {2, 6, 804}};
+constexpr ClusterShape kShapes4[] = {{8, 1, 105}, {8, 2, 150}, {4, 1, 142}, {4, 2, 213}, {2, 1, 205}, {2, 2, 338}, {2, 3, 447}, {2, 4, 548}, {2, 5, 680}, {2, 6, 804}};
+
+// The shape that finishes n tiles soonest, counting whole rounds; *us its time for one pass.  (Clusters of 4, 8 and 16 leave SMs of
+// some GPCs over: 33, 15 and 7 of them run at once on a B200's 148 SMs.)
+// TCQ_FORWARD_KERNEL = cluster2 | cluster4 | cluster8 | cluster16 fixes the cluster size, for comparison runs.
+ClusterShape pick_cluster(long long n, int K, double* us) {
+    const ClusterShape* s = K == 2 ? kShapes2 : K == 3 ? kShapes3 : kShapes4;
+    const int ns = int(K == 2 ? std::size(kShapes2) : K == 3 ? std::size(kShapes3) : std::size(kShapes4));
+    const char* v = std::getenv("TCQ_FORWARD_KERNEL");
+    const int only = v != nullptr && std::strncmp(v, "cluster", 7) == 0 ? std::atoi(v + 7) : 0;
+    ClusterShape best{2, 2, 0};
+    double best_t = 1e300;
+    for (int i = 0; i < ns; ++i) {
+        if (only != 0 && s[i].C != only) continue;
+        const long long at_once = clusters_at_once(s[i].C);
+        if (at_once < 1) continue;
+        const long long groups = (n + s[i].G - 1) / s[i].G, rounds = (groups + at_once - 1) / at_once;
+        if (double(rounds) * s[i].us < best_t) {
+            best_t = double(rounds) * s[i].us;
+            best = s[i];
+        }
+    }
+    if (us != nullptr) *us = best_t;
+    return best;
+}
+
 size_t rowb(int K) { return (size_t(1) << (kL - K)) * size_t(K) / 8; }
 size_t bp_bytes_per_tile(int K) { return size_t(kT) * rowb(K); }
 constexpr size_t kAlign = 256;
 size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
-constexpr int kMaxKeys = 4;   // partial minima per tile left by the cluster kernel (one per CTA of a cluster)
+constexpr int kMaxKeys = 16;   // partial minima per tile left by the cluster kernel (one per CTA of a cluster)
 
-// Workspace for `chunk` tiles: backpointers of one whole pass, two int32 hand-off arrays and the
-// per-CTA partial minima of the final metrics.
-size_t ws_bytes_for_chunk(long long chunk, int K) {
-    return align_up(size_t(chunk) * bp_bytes_per_tile(K)) + 2 * align_up(size_t(chunk) * sizeof(int)) +
-           align_up(size_t(chunk) * kMaxKeys * sizeof(unsigned long long)) + kAlign /* status word */;
+// Scratch comes in two forms.  The cluster step kernel leaves metric rows (MetricRows), the single-CTA kernel packed
+// argmins of every step ("backpointers"), which are a quarter of the size.  The status word lies at the front in both.
+int rows_for(int K, int steps) {
+    return K == 2 ? MetricRows<2>::rows_for(steps) : K == 3 ? MetricRows<3>::rows_for(steps) : MetricRows<4>::rows_for(steps);
 }
 
-// Tiles per chunk at full speed: eight rounds of the largest tile group on every SM.
-long long default_chunk(int num_sms) { return 8LL * 3 * num_sms; }
+size_t rows_bytes_per_tile(int K, int part) { return size_t(rows_for(K, part)) * (size_t(1) << (kL - K)) * 4; }
+constexpr size_t kSmallBytes = kMaxKeys * sizeof(unsigned long long) + 2 * sizeof(int);     // per tile, beside the rows
+
+// Bytes for `chunk` tiles with backpointers: those of one whole pass and two int32 hand-off arrays (and a part that is no longer used:
+// what callers were told to bring stays the same).
+size_t bp_ws_bytes(long long chunk, int K) {
+    return align_up(size_t(chunk) * bp_bytes_per_tile(K)) + 2 * align_up(size_t(chunk) * sizeof(int)) +
+           align_up(size_t(chunk) * 4 * sizeof(unsigned long long)) + kAlign /* status word */;
+}
+// ... with metric rows for walks over `part` steps at a time, the overlaps, the edges handed from part to part and the partial
+// minima of the final metrics.
+size_t rows_ws_bytes(long long chunk, int K, int part) {
+    return align_up(kSmallBytes * size_t(chunk) + 64) + size_t(chunk) * rows_bytes_per_tile(K, part);
+}
+
+// Tiles per chunk at full speed.  Backpointers: eight rounds of the largest tile group on every SM.  Metric rows: two
+// rounds of the largest group on every cluster, which takes no more memory.
+long long bp_chunk(int num_sms) { return 8LL * 3 * num_sms; }
+long long rows_chunk(int num_sms) { return 6LL * num_sms; }
 
 struct Workspace {
+    bool clustered;             // metric rows and the cluster step kernel; else backpointers and the single-CTA kernel
+    int part;                   // steps whose metric rows the workspace holds for a chunk (256, or 128 or 64: see plan_rows)
     unsigned char* bp;
+    float* rows;
     int* e_final;
     int* overlap;
+    int* edge;
     unsigned long long* keys;
     unsigned int* status;
     long long chunk;
 };
 
+// Largest chunk of at most `want` tiles; `need(chunk)` bytes, about per_tile each.
+template <typename Need>
+long long largest_chunk(long long want, size_t ws_bytes, size_t per_tile, long long wave, Need need) {
+    if (need(want) <= ws_bytes) return want;
+    // solve conservatively, then step down
+    long long chunk = (long long)((ws_bytes > 5 * kAlign ? ws_bytes - 5 * kAlign : 0) / per_tile) + 1;
+    if (chunk > want) chunk = want;
+    while (chunk > 0 && need(chunk) > ws_bytes) --chunk;
+    // whole rounds of full groups avoid a ragged last wave inside every chunk
+    if (chunk > wave) chunk = chunk / wave * wave;
+    return chunk;
+}
+
+long long bp_chunk_for(long long n, size_t ws_bytes, int K, int num_sms) {
+    return largest_chunk(n < bp_chunk(num_sms) ? n : bp_chunk(num_sms), ws_bytes, bp_bytes_per_tile(K), 3LL * num_sms,
+                         [K](long long c) { return bp_ws_bytes(c, K); });
+}
+
+// Sweeps of a pass whose path is walked in parts of `part` steps, last part first: the whole pass, then again up to each
+// earlier part.  In steps, for the two passes of an encode (the first needs the second half of its path only).
+int swept_steps(int part) { return part == 256 ? 512 : part == 128 ? 256 + 256 + 128 : (256 + 192) + (256 + 192 + 128 + 64); }
+
+// Chunk and part for metric rows in ws_bytes: the whole path at once if that many tiles fit; a workspace too small for it holds
+// half or a quarter of a path for two or four times the tiles, which pays (and for one tile may be all that fits) although
+// the sweep is repeated for each part.  80 us: the walks and launches of a chunk.
+void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chunk, int* part) {
+    *chunk = 0;
+    *part = 256;
+    double best = 1e300;
+    for (int p = 256; p >= 64; p /= 2) {
+        const long long want = n < rows_chunk(num_sms) ? n : rows_chunk(num_sms);
+        long long c = largest_chunk(want, ws_bytes, rows_bytes_per_tile(K, p), 3LL * num_sms,
+                                    [K, p](long long m) { return rows_ws_bytes(m, K, p); });
+        if (c < 1) continue;
+        const bool all = c >= want;
+        if (!all) c = (n + (n + c - 1) / c - 1) / ((n + c - 1) / c);        // as many chunks, of equal size
+        double us = 0.0, rest = 0.0;
+        pick_cluster(c, K, &us);
+        if (n % c != 0) pick_cluster(n % c, K, &rest);
+        const double total = (double(n / c) * us + rest) * swept_steps(p) / 256.0 + double((n + c - 1) / c) * (80.0 + 40.0 * (256 / p - 1));
+        if (total < best) {
+            best = total;
+            *chunk = c;
+            *part = p;
+        }
+        if (all) break;                            // smaller parts gain nothing
+    }
+}
+
 int carve(void* ws, size_t ws_bytes, long long n, int K, int num_sms, Workspace* out) {
     if (ws == nullptr) return TCQ_E_NULL_POINTER;
     if (reinterpret_cast<uintptr_t>(ws) % kAlign) return TCQ_E_MISALIGNED;
-    long long chunk = n < default_chunk(num_sms) ? n : default_chunk(num_sms);
-    if (ws_bytes_for_chunk(chunk, K) > ws_bytes) {
-        // largest chunk that fits: solve conservatively, then step down
-        chunk = (long long)((ws_bytes > 5 * kAlign ? ws_bytes - 5 * kAlign : 0) / (bp_bytes_per_tile(K) + 2 * sizeof(int) + kMaxKeys * sizeof(unsigned long long)));
-        while (chunk > 0 && ws_bytes_for_chunk(chunk, K) > ws_bytes) --chunk;
-        if (chunk < 1) return TCQ_E_WORKSPACE;
-        // whole rounds of full groups avoid a ragged last wave inside every chunk
-        const long long wave = 3LL * num_sms;
-        if (chunk > wave) chunk = chunk / wave * wave;
-    }
-    unsigned char* base = static_cast<unsigned char*>(ws);
-    out->bp = base;
-    base += align_up(size_t(chunk) * bp_bytes_per_tile(K));
-    out->e_final = reinterpret_cast<int*>(base);
-    base += align_up(size_t(chunk) * sizeof(int));
-    out->overlap = reinterpret_cast<int*>(base);
-    base += align_up(size_t(chunk) * sizeof(int));
-    out->keys = reinterpret_cast<unsigned long long*>(base);
-    base += align_up(size_t(chunk) * kMaxKeys * sizeof(unsigned long long));
+    *out = Workspace{};
+    out->chunk = bp_chunk_for(n, ws_bytes, K, num_sms);
+    if (out->chunk < 1) return TCQ_E_WORKSPACE;
+    out->part = kT;
+    unsigned char* const base = static_cast<unsigned char*>(ws);
     out->status = reinterpret_cast<unsigned int*>(base);
-    out->chunk = chunk;
+    if (cluster_available()) {
+        long long chunk = 0;
+        plan_rows(n, ws_bytes, K, num_sms, &chunk, &out->part);
+        if (chunk >= 1) {
+            out->clustered = true;
+            out->chunk = chunk;
+            out->keys = reinterpret_cast<unsigned long long*>(base + 64);
+            out->overlap = reinterpret_cast<int*>(out->keys + chunk * kMaxKeys);
+            out->edge = out->overlap + chunk;
+            out->rows = reinterpret_cast<float*>(base + align_up(kSmallBytes * size_t(chunk) + 64));
+            return TCQ_OK;
+        }
+    }
+    const size_t ints = align_up(size_t(out->chunk) * sizeof(int));
+    out->overlap = reinterpret_cast<int*>(base + kAlign);
+    out->e_final = reinterpret_cast<int*>(base + kAlign + ints);
+    out->bp = base + kAlign + 2 * ints;
     return TCQ_OK;
 }
 
-cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& wk, int num_sms, cudaStream_t s, int* nkeys) {
+// One sweep of the step kernel over a chunk: a.steps steps, of whose path the last a.bp_steps will be walked.
+// Fills in what the traceback needs to know of it.
+cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& wk, int num_sms, cudaStream_t s, TracebackArgs* t) {
+    t->n = a.n;
+    t->bp_steps = a.bp_steps;
+    t->t_end = a.steps;
+    t->codebook = codebook;
+    t->w = a.w;
+    t->w_add = a.w_add;
+    t->ld = a.ld;
+    t->roll = a.roll;
+    t->overlap = a.overlap;
+    t->e_start = a.overlap != nullptr ? a.overlap : wk.e_final;
+    t->keys = nullptr;
+    if (wk.clustered) {
+        const ClusterShape shape = pick_cluster(a.n, K, nullptr);
+        ClusterArgs ca{a, wk.rows, rows_for(K, a.bp_steps), a.overlap == nullptr && a.steps == kT ? wk.keys : nullptr, nullptr};
+        t->rows = wk.rows;
+        t->nrows = ca.nrows;
+        t->keys = ca.keys;
+        t->nkeys = shape.C;
+        switch (K) {
+            case 2: return launch_forward_cluster<2>(codebook, ca, shape.C, shape.G, s);
+            case 3: return launch_forward_cluster<3>(codebook, ca, shape.C, shape.G, s);
+            case 4: return launch_forward_cluster<4>(codebook, ca, shape.C, shape.G, s);
+            default: return cudaErrorInvalidValue;
+        }
+    }
+    t->bp = wk.bp;
     switch (K) {
-        case 2: return launch_forward<2>(codebook, a, wk.keys, num_sms, s, nkeys);
-        case 3: return launch_forward<3>(codebook, a, wk.keys, num_sms, s, nkeys);
-        case 4: return launch_forward<4>(codebook, a, wk.keys, num_sms, s, nkeys);
+        case 2: return launch_forward_cta<2>(codebook, a, num_sms, s);
+        case 3: return launch_forward_cta<3>(codebook, a, num_sms, s);
+        case 4: return launch_forward_cta<4>(codebook, a, num_sms, s);
         default: return cudaErrorInvalidValue;
     }
 }
+
+// One pass over a chunk and the walk back over its last `walk` steps (256 or 128), in parts if the workspace holds the rows of
+// a part only.  `out`: the walk's outputs; its e_out gets the edge before the first walked step.
+int pass(int K, int codebook, ForwardArgs f, int walk, TracebackArgs out, const Workspace& wk, int num_sms, cudaStream_t s, const char* what) {
+    int* const e_out = out.e_out;
+    const int first = kT - walk;
+    for (int end = kT; end > first;) {
+        const int begin = end - wk.part > first ? end - wk.part : first;
+        f.steps = end;
+        f.bp_steps = end - begin;
+        cudaError_t err = forward(K, codebook, f, wk, num_sms, s, &out);
+        if (err != cudaSuccess) return cuda_fail(err, what);
+        if (end < kT) out.e_start = wk.edge;       // where the later part's walk arrived
+        out.e_out = begin == first ? e_out : wk.edge;
+        if ((err = launch_traceback(K, out, s)) != cudaSuccess) return cuda_fail(err, what);
+        f.final_cost = nullptr;                    // the first sweep is the whole pass: it reported
+        f.e_final = nullptr;
+        f.flags = 0;
+        end = begin;
+    }
+    return TCQ_OK;
+}
+
+// Launches of an encode per chunk: a sweep and a walk for each part of the two passes.
+int launches_per_chunk(int part) { return 2 * ((part >= 128 ? 1 : 2) + 256 / part); }
 
 int check_common(int K, int codebook, long long n) {
     if (K < 2 || K > 4) return TCQ_E_BAD_K;
@@ -135,47 +318,32 @@ int encode_core(const EncodeIO& io, int K, int codebook, void* ws, size_t ws_byt
         const long long cn = io.n - c0 < wk.chunk ? io.n - c0 : wk.chunk;
         const float* w = io.w + c0 * tile_step;
         const float* w_add = io.w_add ? io.w_add + c0 * tile_step : nullptr;
-        cudaError_t err;
-        // pass 1: tile rotated by half its length, free start; only the second half of the
-        // backpointers is needed to reach the state at rotated position 128 (qtip.py:138-141)
-        ForwardArgs f1{w, w_add, io.ld, cn, nullptr, kT / 2, kT / 2, wk.bp, wk.e_final, nullptr, 1.0f, 0, wk.status,
+        // pass 1: tile rotated by half its length, free start; only the second half of the path is needed, to
+        // reach the state at rotated position 128 (qtip.py:138-141)
+        ForwardArgs f1{w, w_add, io.ld, cn, nullptr, kT / 2, 0, 0, wk.bp, wk.e_final, nullptr, 1.0f, 0, wk.status,
                        c0 == 0 ? kFwdResetStatus : 0};
-        int nkeys = 0;
-        if ((err = forward(K, codebook, f1, wk, num_sms, s, &nkeys)) != cudaSuccess) return cuda_fail(err, "forward pass 1");
         TracebackArgs t1{};
-        t1.bp = wk.bp;
-        t1.n = cn;
-        t1.bp_steps = kT / 2;
-        t1.codebook = codebook;
-        t1.e_start = wk.e_final;
-        t1.keys = nkeys ? wk.keys : nullptr;
-        t1.nkeys = nkeys;
         t1.e_out = wk.overlap;
-        if ((err = launch_traceback(K, t1, s)) != cudaSuccess) return cuda_fail(err, "traceback pass 1");
+        if ((rc = pass(K, codebook, f1, kT / 2, t1, wk, num_sms, s, "pass 1")) != TCQ_OK) return rc;
         // pass 2: true order, start and end tied to the overlap (qtip.py:142)
-        ForwardArgs f2{w, w_add, io.ld, cn, wk.overlap, 0, kT, wk.bp, nullptr, io.sse ? io.sse + c0 : nullptr, 1.0f, 0,
+        ForwardArgs f2{w, w_add, io.ld, cn, wk.overlap, 0, 0, 0, wk.bp, nullptr, io.sse ? io.sse + c0 : nullptr, 1.0f, 0,
                        wk.status, kFwdCheckFinite};
-        if ((err = forward(K, codebook, f2, wk, num_sms, s, &nkeys)) != cudaSuccess) return cuda_fail(err, "forward pass 2");
-        TracebackArgs t2{};
-        t2.bp = wk.bp;
-        t2.n = cn;
-        t2.bp_steps = kT;
-        t2.codebook = codebook;
-        t2.e_start = wk.overlap;
-        t2.bits = io.bits ? reinterpret_cast<long long*>(io.bits) + c0 * kT : nullptr;
-        t2.dq = io.dq ? io.dq + c0 * kT : nullptr;
-        t2.packed = io.packed ? io.packed + c0 * io.packed_stride : nullptr;
-        t2.packed_stride = io.packed_stride;
-        t2.wq = io.wq ? io.wq + c0 * tile_step : nullptr;
-        t2.err = io.err ? io.err + c0 * tile_step : nullptr;
-        t2.src = io.w + c0 * tile_step;
-        t2.ld = io.ld;
-        if ((err = launch_traceback(K, t2, s)) != cudaSuccess) return cuda_fail(err, "traceback pass 2");
+        TracebackArgs t{};
+        t.bits = io.bits ? reinterpret_cast<long long*>(io.bits) + c0 * kT : nullptr;
+        t.dq = io.dq ? io.dq + c0 * kT : nullptr;
+        t.packed = io.packed ? io.packed + c0 * io.packed_stride : nullptr;
+        t.packed_stride = io.packed_stride;
+        t.wq = io.wq ? io.wq + c0 * tile_step : nullptr;
+        t.err = io.err ? io.err + c0 * tile_step : nullptr;
+        t.src = w;
+        if ((rc = pass(K, codebook, f2, kT, t, wk, num_sms, s, "pass 2")) != TCQ_OK) return rc;
     }
     return TCQ_OK;
 }
 
 }  // namespace
+
+size_t tcq::backpointer_workspace_bytes(long long n, int K) { return bp_ws_bytes(n, K); }
 
 extern "C" {
 
@@ -203,7 +371,7 @@ const char* tcq_last_cuda_error(void) { return g_last_cuda_error; }
 
 size_t tcq_workspace_min_bytes(int K) {
     if (K < 2 || K > 4) return 0;
-    return ws_bytes_for_chunk(1, K);
+    return bp_ws_bytes(1, K);
 }
 
 size_t tcq_workspace_bytes(int64_t n_tiles, int K) {
@@ -216,9 +384,10 @@ size_t tcq_workspace_bytes(int64_t n_tiles, int K) {
     } else {
         (void)cudaGetLastError();
     }
-    long long chunk = n_tiles < default_chunk(num_sms) ? n_tiles : default_chunk(num_sms);
-    if (chunk < 1) chunk = 1;
-    return ws_bytes_for_chunk(chunk, K);
+    const long long n = n_tiles < 1 ? 1 : n_tiles;
+    const size_t bp = bp_ws_bytes(n < bp_chunk(num_sms) ? n : bp_chunk(num_sms), K);
+    const size_t rows = rows_ws_bytes(n < rows_chunk(num_sms) ? n : rows_chunk(num_sms), K, kT);
+    return rows > bp ? rows : bp;
 }
 
 int tcq_encode_tb(const float* w, int64_t n_tiles, int K, int codebook, uint32_t* packed, int64_t* bits, float* dq,
@@ -283,22 +452,11 @@ int tcq_viterbi_pass(const float* w, int64_t n_tiles, int K, int codebook, const
 
     for (long long c0 = 0; c0 < n_tiles; c0 += wk.chunk) {
         const long long cn = n_tiles - c0 < wk.chunk ? n_tiles - c0 : wk.chunk;
-        cudaError_t err;
-        ForwardArgs f{w + c0 * kT, nullptr, 0, cn, overlap ? overlap + c0 : nullptr, roll, kT, wk.bp,
+        ForwardArgs f{w + c0 * kT, nullptr, 0, cn, overlap ? overlap + c0 : nullptr, roll, 0, 0, wk.bp,
                       overlap ? nullptr : wk.e_final, nullptr, 1.0f, 0, wk.status, kFwdCheckFinite};
-        int nkeys = 0;
-        if ((err = forward(K, codebook, f, wk, num_sms, s, &nkeys)) != cudaSuccess) return cuda_fail(err, "forward");
-        const bool use_keys = overlap == nullptr && nkeys > 0;
         TracebackArgs t{};
-        t.bp = wk.bp;
-        t.n = cn;
-        t.bp_steps = kT;
-        t.codebook = codebook;
-        t.e_start = overlap ? overlap + c0 : wk.e_final;
-        t.keys = use_keys ? wk.keys : nullptr;
-        t.nkeys = nkeys;
         t.states = reinterpret_cast<long long*>(states) + c0 * kT;
-        if ((err = launch_traceback(K, t, s)) != cudaSuccess) return cuda_fail(err, "traceback");
+        if ((rc = pass(K, codebook, f, kT, t, wk, num_sms, s, "viterbi pass")) != TCQ_OK) return rc;
     }
     return TCQ_OK;
 }
@@ -315,14 +473,19 @@ int tcq_forward_pass(const float* w, int64_t n_tiles, int K, int codebook, const
     if ((rc = current_num_sms(&num_sms)) != TCQ_OK) return rc;
     Workspace wk;
     if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
-    if (wk.chunk < n_tiles) return TCQ_E_WORKSPACE;
-    if (cudaMemsetAsync(wk.status, 0, sizeof(unsigned int), static_cast<cudaStream_t>(stream)) != cudaSuccess)
-        return cuda_fail(cudaGetLastError(), "status reset");
-    ForwardArgs f{w, nullptr, 0, n_tiles, overlap, roll, bp_steps, wk.bp, overlap ? nullptr : wk.e_final, nullptr, 1.0f, 0,
-                  wk.status, kFwdCheckFinite};
-    int nkeys = 0;
-    cudaError_t err = forward(K, codebook, f, wk, num_sms, static_cast<cudaStream_t>(stream), &nkeys);
-    return err == cudaSuccess ? TCQ_OK : cuda_fail(err, "forward");
+    if (bp_chunk_for(n_tiles, ws_bytes, K, num_sms) < n_tiles) return TCQ_E_WORKSPACE;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (cudaMemsetAsync(wk.status, 0, sizeof(unsigned int), s) != cudaSuccess) return cuda_fail(cudaGetLastError(), "status reset");
+    for (long long c0 = 0; c0 < n_tiles; c0 += wk.chunk) {
+        const long long cn = n_tiles - c0 < wk.chunk ? n_tiles - c0 : wk.chunk;
+        ForwardArgs f{w + c0 * kT, nullptr, 0, cn, overlap ? overlap + c0 : nullptr, roll, bp_steps < wk.part ? bp_steps : wk.part, kT,
+                      wk.bp, overlap ? nullptr : wk.e_final, nullptr, 1.0f, 0, wk.status, kFwdCheckFinite};
+        if (!wk.clustered) f.bp_steps = bp_steps;
+        TracebackArgs t{};
+        const cudaError_t err = forward(K, codebook, f, wk, num_sms, s, &t);
+        if (err != cudaSuccess) return cuda_fail(err, "forward");
+    }
+    return TCQ_OK;
 }
 
 int tcq_workspace_status(const void* ws, size_t ws_bytes, int64_t n_tiles, int K, void* stream) {
@@ -351,15 +514,17 @@ int tcq_selftest_wait_timeout(const float* w, int64_t n_tiles, int K, void* ws, 
     if ((rc = current_num_sms(&num_sms)) != TCQ_OK) return rc;
     Workspace wk;
     if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
-    if (wk.chunk < n_tiles) return TCQ_E_WORKSPACE;
+    if (bp_ws_bytes(n_tiles, K) > ws_bytes) return TCQ_E_WORKSPACE;
+    if (!cluster_available()) return TCQ_E_BAD_ARGUMENT;   // the single-CTA kernel has no bounded waits to test
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(wk.status, 0, sizeof(unsigned int), s) != cudaSuccess) return cuda_fail(cudaGetLastError(), "status reset");
     // the buffers of the final metrics are told to expect 16 bytes more than the cluster will ever send
-    ForwardArgs f{w, nullptr, 0, n_tiles, nullptr, 0, kT, wk.bp, wk.e_final, nullptr, 1.0f, 16, wk.status, 0};
-    int nkeys = 0;
-    cudaError_t err = forward(K, kCbMcg, f, wk, num_sms, s, &nkeys);
-    if (err != cudaSuccess) return cuda_fail(err, "forward (self-test)");
-    return nkeys > 0 ? TCQ_OK : TCQ_E_BAD_ARGUMENT;   // the single-CTA kernel has no bounded waits to test
+    ForwardArgs f{w, nullptr, 0, n_tiles, nullptr, 0, 0, kT, nullptr, nullptr, nullptr, 1.0f, 16, wk.status, 0};
+    ClusterArgs ca{f, nullptr, 0, nullptr, nullptr};
+    cudaError_t err = K == 2   ? launch_forward_cluster<2>(kCbMcg, ca, 2, 2, s)
+                      : K == 3 ? launch_forward_cluster<3>(kCbMcg, ca, 2, 2, s)
+                               : launch_forward_cluster<4>(kCbMcg, ca, 2, 2, s);
+    return err == cudaSuccess ? TCQ_OK : cuda_fail(err, "forward (self-test)");
 }
 
 int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes) {
@@ -372,7 +537,7 @@ int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes) {
     Workspace wk;
     alignas(256) static unsigned char dummy[256];          // carve() only does pointer arithmetic on it
     if ((rc = carve(dummy, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
-    return 4 * ((n_tiles + wk.chunk - 1) / wk.chunk);
+    return launches_per_chunk(wk.clustered ? wk.part : kT) * ((n_tiles + wk.chunk - 1) / wk.chunk);
 }
 
 int tcq_decode_packed(const uint32_t* packed, int64_t n_tiles, int K, int codebook, float* dq, void* stream) {

@@ -33,6 +33,30 @@ struct Geo {
     static constexpr int NWORDS = kT * K / 32;    // packed code words per tile
 };
 
+// Metric rows: what the cluster step kernel leaves in HBM for the traceback.  The metrics before step t = T - D*(j+1)
+// of a sweep over T steps are row j of their tile (the last row is row 0).  From an edge after step t + D - 1, the walk over the D steps
+// between two rows can have come from Q^D = NA edges only: those that share its bits above K*D, which are its LB = 4 lowest
+// bits D steps earlier.  A row is stored with these NA metrics contiguous.  Row j's steps are taken from HBM at one
+// dependent access per D steps (D = 5 / 3 / 2), of 4 / 2 / 1 KiB, and a pass writes E * 4 / D bytes per step and tile:
+// 13.1 / 10.9 / 8.2 KB against 4 / 3 / 2 KB of packed argmins, at most a quarter of the HBM bandwidth.
+template <int K>
+struct MetricRows {
+    static constexpr int D = K == 2 ? 5 : K == 3 ? 3 : 2;
+    static constexpr int LB = kL - K - K * D;
+    static constexpr int NA = 1 << (K * D);
+    static_assert(LB == 4, "the position arithmetic and the kernels' sector coverage are written for four group bits");
+    // rows that a walk over the last `steps` steps needs (metrics before step 0 are known)
+    static constexpr int rows_for(int steps) {
+        return (steps + D - 1) / D < (kT - 1) / D ? (steps + D - 1) / D : (kT - 1) / D;
+    }
+    __host__ __device__ static constexpr uint32_t pos(uint32_t e) { return ((e & ((1u << LB) - 1)) << (K * D)) | (e >> LB); }
+    // row that the results of step t of a sweep over `steps` steps are, or -1
+    __device__ static __forceinline__ int row_after(int t, int steps, int nrows) {
+        const int back = steps - 1 - t, j = back / D - 1;
+        return (back % D == 0 && j < nrows) ? j : -1;
+    }
+};
+
 // x(state) = state * MUL + ADD (mod 2^32) is the linear-congruential scramble that
 // each codebook starts with; it is affine in the state, so kernels form it once
 // per butterfly and add compile-time multiples of MUL for the other states.
@@ -149,6 +173,15 @@ template <> __device__ __forceinline__ float min_of<16>(const float (&c)[16]) {
     const float a = min3(min3(c[0], c[1], c[2]), min3(c[3], c[4], c[5]), min3(c[6], c[7], c[8]));
     const float b = min3(min3(c[9], c[10], c[11]), min3(c[12], c[13], c[14]), c[15]);
     return fminf(a, b);
+}
+// The same minimum as a tree of pairs, which the compiler makes three-input instructions of by itself and in an order that
+// suits it: 2 % faster than min_of in the cluster step kernel at K = 3 with two or three tiles per set, no difference at K = 4.
+template <int N> __device__ __forceinline__ float min_tree(const float (&c)[N]) {
+    float m[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) m[i] = fminf(c[2 * i], c[2 * i + 1]);
+    if constexpr (N == 2) return m[0];
+    else return min_tree<N / 2>(m);
 }
 
 // Conditional move "if (c == best) tag = value", the argmin scan's inner operation.

@@ -50,7 +50,8 @@ struct ForwardArgs {
     long long n;             // tiles in this launch
     const int* overlap;      // [n] forced first/last edge, or nullptr (unconstrained, metrics start at 0)
     int roll;                // step t consumes w[(t + roll) & 255]   (roll = 128: torch.roll(w,128))
-    int bp_steps;            // backpointer rows kept per tile: the LAST bp_steps steps (256 or 128)
+    int bp_steps;            // steps the traceback will walk: the LAST bp_steps ones (single-CTA kernel: 256 or 128 backpointer rows per tile)
+    int steps;               // cluster kernel: steps of the sweep, a multiple of 4 (256, or fewer to leave the rows of an earlier part)
     unsigned char* bp;       // [n][bp_steps][E*K/8] packed backpointers
     int* e_final;            // [n] out: argmin edge of the final metrics (lowest index on ties), or nullptr
     float* final_cost;       // [n] out: final metric at overlap[tile] (constrained) / its minimum, or nullptr
@@ -280,12 +281,22 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_kernel(const ForwardArgs a)
     }
 }
 
-// Host-side launcher for one (K, codebook): picks the tiles-per-CTA variant.
-// Implemented once per K in tcq_forward_k{2,3,4}.cu.
-// `keys` ([n][4] 64-bit scratch) enables the cluster kernel; *nkeys is then the number of
-// per-CTA partial minima written per tile (0: the single-CTA kernel ran and wrote e_final).
+// Cluster kernel (tcq_forward_cluster.cuh): the pass, and where its metric rows and final minima go.
+struct ClusterArgs {
+    ForwardArgs f;              // bp, bp_steps and e_final are not used
+    float* rows;                // [n][nrows][E] out: metric rows (MetricRows), the last nrows of the pass
+    int nrows;
+    unsigned long long* keys;   // [n][C] out: per-CTA (metric bits << 32 | edge) minima of the final metrics, or nullptr
+    int* at_once;               // host, with f.n == 0: receives how many such clusters the device runs at once
+};
+
+// Host-side launchers, implemented once per K in tcq_forward_k{2,3,4}.cu.
+// Cluster form: clusters of C CTAs that advance G tiles.  cudaErrorNotSupported (and nothing launched) if the
+// device cannot schedule such a cluster; with f.n == 0 nothing is launched: it only finds that out.
 template <int K>
-cudaError_t launch_forward(int codebook, const ForwardArgs& args, unsigned long long* keys, int num_sms,
-                           cudaStream_t stream, int* nkeys);
+cudaError_t launch_forward_cluster(int codebook, const ClusterArgs& args, int C, int G, cudaStream_t stream);
+// Single-CTA form (packed argmins to args.bp): picks the tiles-per-CTA variant.
+template <int K>
+cudaError_t launch_forward_cta(int codebook, const ForwardArgs& args, int num_sms, cudaStream_t stream);
 
 }  // namespace tcq

@@ -1,10 +1,15 @@
-// Viterbi step kernel, thread-block-cluster form: the whole codebook lives in registers.
+// Viterbi step kernel, thread-block-cluster form: the whole codebook lives in registers, and the
+// step keeps only the minima.
 //
 // The plain step kernel (tcq_forward.cuh) re-evaluates each of the 65536 codebook values on
-// every step and shares it between the few tiles one SM's shared memory can hold; that
-// evaluation is a quarter of its instructions.  Here a cluster of C CTAs (C SMs) owns a group
+// every step and records the argmin of every edge.  Here a cluster of C CTAs (C SMs) owns a group
 // of tiles together and the 65536 states are divided among its C * NT threads, so each thread
-// keeps its 65536 / (C * NT) codebook values in registers for the whole launch:
+// keeps its 65536 / (C * NT) codebook values in registers for the whole launch, and no argmin is
+// formed at all: one edge of 2^(16-K) per step lies on the path that the traceback walks, so the
+// argmin is worth having for that one only.  Every D-th step's path metrics go to HBM instead of every
+// step's argmins, and the traceback re-derives the D argmins between two such rows from the
+// Q^D metrics its edge can have come from (tcq_traceback.cu), with the same operations in the same
+// order, so that the codes are those of the recorded argmins bit for bit.
 //
 //   * CTA r owns the butterflies h in [r * HN/C, (r+1) * HN/C): it needs the path metrics
 //     old[q * HN + h] for all q (E/C values per tile, in ITS shared memory, layout [Q][HN/C])
@@ -13,38 +18,33 @@
 //     (the owner of h' = (h * Q + l) mod HN), so each result is stored once, straight into the
 //     consumer's shared memory: a local store or a distributed-shared-memory store
 //     (cluster.map_shared_rank), never both;
-//   * the stores are asynchronous (st.async) and each one reports its 16 bytes to an mbarrier
+//   * the stores are asynchronous (st.async) and each one reports its bytes to an mbarrier
 //     in the consumer CTA; a CTA starts a step when the mbarrier of its input buffer has
 //     counted the whole buffer.  No thread ever executes a memory fence, which matters because
 //     a release fence on this chip waits for every outstanding store of the SM, including the
-//     backpointer rows on their way to HBM;
+//     metric rows on their way to HBM;
 //   * the only other synchronisation is write-after-read: nobody may store into a buffer that
 //     a neighbour is still reading.  The hardware cluster barrier handles that with relaxed
 //     arrives at the end of every step and a wait just before the next step's first store;
 //   * the group's tiles form two sets that alternate, so both kinds of wait normally find
-//     their condition already true: the other set's step has run in between;
-//   * backpointers: each CTA packs the argmins of its slice into shared memory and streams
-//     the previous step's row slice to HBM with 128-bit stores, as the plain kernel does.
+//     their condition already true: the other set's step has run in between.
 //
-// A work item is (butterfly, LU successors); with LU * K not a multiple of 8 (K = 3, LU = 4)
-// the two items of a butterfly sit in neighbouring lanes and merge their 12 argmin bits with
-// one shuffle.  Nothing in this kernel waits on memory written by another CTA except through
-// the cluster barrier, and every CTA of a cluster executes the same number of barrier phases.
+// A metric row goes to HBM straight from the registers that hold the step's results, in the order
+// that makes the ancestors of one edge contiguous (MetricRows::pos): a warp's store instruction
+// covers whole 32-byte sectors.  Nothing in this kernel waits on memory written by another CTA except
+// through the mbarriers and the cluster barrier, and every CTA of a cluster executes the same number of
+// barrier phases.
 #pragma once
 
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "tcq_forward.cuh"
 
 namespace tcq {
 
 namespace cg = cooperative_groups;
-
-template <int K, int C, int GS>
-constexpr size_t cluster_smem_bytes() {
-    // per CTA: metrics [2 sets][GS][2 buffers][E/C] fp32, staging [2][2*GS][ROWB/C], weights [2*GS][256], reduction scratch
-    return size_t(2) * GS * 2 * (Geo<K>::E / C) * 4 + size_t(2) * 2 * GS * (Geo<K>::ROWB / C) + size_t(2) * GS * kT * 4 + 64 * 8;
-}
 
 // Hardware cluster barrier, split phase, no memory ordering: used only to keep stores away from
 // buffers that are still being read.
@@ -99,38 +99,93 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, volati
     *gave_up = 1u;
     return false;
 }
-__device__ __forceinline__ void st_async_v4(uint32_t dst, float x, float y, float z, float w, uint32_t mbar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];"
-                 ::"r"(dst), "f"(x), "f"(y), "f"(z), "f"(w), "r"(mbar) : "memory");
+__device__ __forceinline__ void mbar_arrive(uint32_t mbar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(mbar) : "memory");
 }
-__device__ __forceinline__ void st_async_v2(uint32_t dst, float x, float y, uint32_t mbar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];"
-                 ::"r"(dst), "f"(x), "f"(y), "r"(mbar) : "memory");
+// Stores of N = 1, 2 or 4 results, with the buffer's offset OFF as an immediate: to this CTA's shared memory, or
+// asynchronously to another CTA's, reporting to its mbarrier at bar + BOFF.
+template <int OFF, int N>
+__device__ __forceinline__ void st_local(uint32_t dst, const float* v) {
+    if constexpr (N == 4)
+        asm volatile("st.shared.v4.f32 [%0+%5], {%1, %2, %3, %4};" ::"r"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "n"(OFF) : "memory");
+    else if constexpr (N == 2)
+        asm volatile("st.shared.v2.f32 [%0+%3], {%1, %2};" ::"r"(dst), "f"(v[0]), "f"(v[1]), "n"(OFF) : "memory");
+    else
+        asm volatile("st.shared.f32 [%0+%2], %1;" ::"r"(dst), "f"(v[0]), "n"(OFF) : "memory");
+}
+template <int OFF, int BOFF, int N>
+__device__ __forceinline__ void st_remote(uint32_t dst, const float* v, uint32_t bar) {
+    if constexpr (N == 4)
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0+%6], {%1, %2, %3, %4}, [%5+%7];"
+                     ::"r"(dst), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"(bar), "n"(OFF), "n"(BOFF) : "memory");
+    else if constexpr (N == 2)
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0+%4], {%1, %2}, [%3+%5];"
+                     ::"r"(dst), "f"(v[0]), "f"(v[1]), "r"(bar), "n"(OFF), "n"(BOFF) : "memory");
+    else
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.f32 [%0+%3], %1, [%2+%4];"
+                     ::"r"(dst), "f"(v[0]), "r"(bar), "n"(OFF), "n"(BOFF) : "memory");
+}
+// One predecessor's metrics of HB neighbouring butterflies, OFF bytes from src.
+template <int HB>
+__device__ __forceinline__ void ld_metrics(const float* src, float (&v)[HB]) {
+    if constexpr (HB == 4) {
+        const float4 x = *reinterpret_cast<const float4*>(src);
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+    } else if constexpr (HB == 2) {
+        const float2 x = *reinterpret_cast<const float2*>(src);
+        v[0] = x.x; v[1] = x.y;
+    } else {
+        v[0] = *src;
+    }
 }
 
-struct ClusterArgs {
-    ForwardArgs f;
-    unsigned long long* keys;   // [n][C] out: per-CTA (metric bits << 32 | edge) minima of the final metrics, or nullptr
+// f(0), ..., f(N-1), each with its number as a compile-time constant.
+template <int N, int I = 0, typename F>
+__device__ __forceinline__ void static_for(F&& f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        static_for<N, I + 1>(f);
+    }
+}
+
+// Work of one thread and step: NI items of HB neighbouring butterflies x LU of their successors, i.e. of runs of R = HB * LU
+// consecutive edges.  LU = Q unless that would be more than the thread's 65536 / (C * NT) states.
+template <int K, int C, int NT>
+struct ClusterItem {
+    static constexpr int STATES = kStates / (C * NT);
+    static constexpr int Q = Geo<K>::Q;
+    static constexpr int NB = STATES >= Q * Q ? STATES / (Q * Q) : 1;      // butterflies of a thread
+    static constexpr int HB = NB > 2 ? 2 : NB;
+    static constexpr int NI = NB / HB;
+    static constexpr int LU = STATES >= Q * Q ? Q : STATES / Q;
+    static constexpr int R = HB * LU;
+    static_assert(NI * HB * LU * Q == STATES, "a thread's states must form whole successors");
 };
 
-template <int K, int CB, int C, int GS, int NT, int LU>
+template <int K, int C, int GA, int GB>
+constexpr size_t cluster_smem_bytes() {
+    // per CTA: metrics [GA+GB tiles][2 buffers][E/C] fp32, weights [GA+GB][256] (twice each), reduction scratch and mbarriers
+    return size_t(GA + GB) * 2 * (Geo<K>::E / C) * 4 + size_t(GA + GB) * kT * 8 + 64 * 8;
+}
+
+// GA, GB: tiles of the two sets that alternate (GB = 0: one set, for the smallest batches).
+template <int K, int CB, int C, int GA, int GB, int NT>
 __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const ClusterArgs ca) {
     using GE = Geo<K>;
-    constexpr int Q = GE::Q, E = GE::E, HN = GE::HN, ROWB = GE::ROWB;
-    constexpr int G = 2 * GS;                      // tiles per cluster group (two alternating sets)
+    using MR = MetricRows<K>;
+    using IT = ClusterItem<K, C, NT>;
+    constexpr int Q = GE::Q, E = GE::E, HN = GE::HN;
+    constexpr int NI = IT::NI, HB = IT::HB, LU = IT::LU, R = IT::R;
+    constexpr int G = GA + GB;                     // tiles per cluster group
     constexpr int HNC = HN / C;                    // butterflies per CTA
     constexpr int EC = E / C;                      // metrics per tile held by a CTA
-    constexpr int ROWBC = ROWB / C;                // backpointer bytes per step produced by a CTA
     constexpr int NCHUNK = Q / LU;
-    constexpr int NITEMS = HNC * NCHUNK;           // items per CTA
-    constexpr int NI = NITEMS / NT;                // items per thread
-    constexpr int ITEM_BITS = LU * K;
-    constexpr bool PAIRED = (ITEM_BITS % 8) != 0;  // two neighbouring lanes merge their bits
-    static_assert(NITEMS % NT == 0 && NI >= 1, "items must divide evenly over the threads");
-    static_assert(LU == 2 || LU % 4 == 0, "successor chunk is a float2 or whole float4s");
-    static_assert(!PAIRED || (NCHUNK == 2 && 2 * ITEM_BITS % 8 == 0 && 2 * ITEM_BITS <= 24), "paired items must complete whole bytes");
-    static_assert(PAIRED || (ITEM_BITS % 8 == 0 && ITEM_BITS <= 24), "an item's backpointers must be whole bytes and exact in fp32");
-    static_assert(ROWBC % 16 == 0, "row slices are streamed as 128-bit words");
+    constexpr int SV = R < 4 ? R : 4;              // successors per store (one float, float2 or float4)
+    constexpr int NWD = R / SV;                    // stores per item, tile and step
+    constexpr int HI = HNC / NI;                   // item i's butterflies lie HI * i after item 0's ...
+    constexpr int DQ = HI * Q / HN;                // ... and its successors are the predecessors DQ * i later of the same butterflies
+    static_assert(HNC / HB * NCHUNK == NI * NT, "items must divide evenly over the threads");
+    static_assert(NI == 1 || (HI * Q % HN == 0 && HI % (32 * R) == 0 && HI * Q % 16 == 0), "items must differ by constants");
     constexpr uint32_t MUL = CbLcg<CB>::MUL, ADD = CbLcg<CB>::ADD;
     const ForwardArgs& a = ca.f;
 
@@ -139,203 +194,177 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float* const cost = reinterpret_cast<float*>(smem_raw);                          // [G][2][EC]
-    unsigned char* const stage = smem_raw + size_t(G) * 2 * EC * 4;                   // [2][G][ROWBC]
-    float* const wv = reinterpret_cast<float*>(stage + size_t(2) * G * ROWBC);        // [G][256]
+    float2* const wv = reinterpret_cast<float2*>(cost + size_t(G) * 2 * EC);         // [G][256], each weight twice (a packed operand)
     unsigned long long* const red = reinterpret_cast<unsigned long long*>(wv + G * kT);   // [32] reduction scratch
     unsigned long long* const mbar = red + 32;     // [2 sets][2 buffers] mbarriers counting the bytes of each metric buffer
     volatile unsigned int* const gave_up = reinterpret_cast<volatile unsigned int*>(red + 40);   // set by the first wait that runs out
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31;
     const bool constrained = a.overlap != nullptr;
-    const int t_store0 = kT - a.bp_steps;
     const float kInf = __uint_as_float(kInfBits);
     const f32x2 one2 = pack2(a.one, a.one);
-    const float zero = a.one - 1.0f;
+
+    // Slot of butterfly hl in a row of metrics.  A thread's run of 8 or 16 edges is stored as 16-byte words; the warp's words
+    // w of all lanes lie together, so that each store instruction writes contiguous memory (the network between SMs takes
+    // half as long for it as for words 32 bytes apart), and the lane bits are flipped per w so that the loads of the next
+    // step, which walk along the edges, still touch every bank once.
+    auto slot = [](int hl) {
+        if constexpr (R <= 4) {
+            return hl;
+        } else {
+            const int word = hl >> 2, w = word % NWD, ln = (word / NWD) & 31;
+            return (hl & ~(32 * R - 1)) | (w * 128 + ((ln ^ (w * (8 / NWD))) << 2)) | (hl & 3);
+        }
+    };
+    auto unslot = [](int sl) {
+        if constexpr (R <= 4) {
+            return sl;
+        } else {
+            const int word = (sl >> 2) & (32 * NWD - 1), w = word >> 5, ln = (word & 31) ^ (w * (8 / NWD));
+            return (sl & ~(32 * R - 1)) | ((ln * NWD + w) << 2) | (sl & 3);
+        }
+    };
 
     // ---- this thread's items: codebook values and destinations, fixed for the whole launch ----
-    int h_loc[NI];               // butterfly index inside this CTA
-    int e_out[NI];               // first successor edge (global numbering)
-    uint32_t dst[NI];            // where its LU results go: shared::cluster address in the consumer CTA (tile 0, buffer 0)
-    uint32_t dst_bar[NI];        // the consumer CTA's mbarrier array (shared::cluster address)
-    f32x2 cbv[NI][LU][Q / 2];    // codebook values of (q = 2j, 2j+1; successor lu)
+    const int hl0 = tid / NCHUNK * HB, h0 = rank * HNC + hl0;    // first butterfly (chunk index fastest: a butterfly's items are neighbours)
+    const int e0 = h0 * Q + tid % NCHUNK * LU;                   // first successor edge
+    const int qn = e0 / HN, hn = e0 % HN;                        // its role in the next step: predecessor qn of butterfly hn
+    const bool local = hn / HNC == rank;                         // which this CTA owns itself, or another
+    uint32_t dst[NWD];                                           // where each store goes (tile 0, buffer 0)
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        const int it = tid + i * NT;
-        const int hl = it / NCHUNK, lc = it % NCHUNK;     // chunk index fastest: a butterfly's items are neighbours
-        const int h = rank * HNC + hl;
-        const int e0 = h * Q + lc * LU;
-        h_loc[i] = hl;
-        e_out[i] = e0;
-        const int qn = e0 / HN, hn = e0 % HN;              // role of e0 in the next step: predecessor qn of butterfly hn
-        const int owner = hn / HNC;
-        dst[i] = map_to_rank(smem_u32(cost + qn * HNC + (hn % HNC)), owner);
-        dst_bar[i] = map_to_rank(smem_u32(mbar), owner);
-        const uint32_t xb = uint32_t(e0) * MUL + ADD;
+    for (int w = 0; w < NWD; ++w) {
+        dst[w] = smem_u32(cost + qn * HNC + slot(hn % HNC + w * SV));
+        if (!local) dst[w] = map_to_rank(dst[w], hn / HNC);
+    }
+    const uint32_t dst_bar = map_to_rank(smem_u32(mbar), hn / HNC);   // the consumer's mbarriers
+    const float* const src = cost + slot(hl0);
+    const uint32_t row_off = MR::pos(uint32_t(e0));              // in a metric row; a run's next edges follow NA apart
+    f32x2 cbv[NI * R][Q / 2];                                    // codebook values of (q = 2j, 2j+1) into each run's edges
 #pragma unroll
-        for (int lu = 0; lu < LU; ++lu)
+    for (int i = 0; i < NI * R; ++i) {
+        const uint32_t xb = uint32_t(e0 + i / R * (HI * Q) + i % R) * MUL + ADD;
 #pragma unroll
-            for (int j = 0; j < Q / 2; ++j)
-                cbv[i][lu][j] = pack2(cb_from_x<CB>(xb + uint32_t((2 * j) * E + lu) * MUL),
-                                      cb_from_x<CB>(xb + uint32_t((2 * j + 1) * E + lu) * MUL));
+        for (int j = 0; j < Q / 2; ++j)
+            cbv[i][j] = pack2(cb_from_x<CB>(xb + uint32_t((2 * j) * E) * MUL), cb_from_x<CB>(xb + uint32_t((2 * j + 1) * E) * MUL));
     }
 
     const long long ngroups = (a.n + G - 1) / G;
     const long long nclusters = gridDim.x / C;
     const long long cluster_id = blockIdx.x / C;
 
-    long long tile0 = 0;                           // first tile of the group being processed
+    float* row_tile0 = nullptr;                    // metric rows of the group's first tile
+    int live = 0;                                  // tiles of the group that exist
 
-    // stream one step's row slices of tile set `s` (written during step t into staging buffer `buf` = t & 1) to HBM
-    // (coalesced 128-bit stores).  A set's slices are GS * ROWBC / 16 <= NT words, one per thread; which word, which
-    // tile of the set and the byte offset from the set's first row are fixed for the launch.
-    constexpr int V = ROWBC / 16;
-    constexpr int FW = (GS * V + NT - 1) / NT;     // 128-bit words of a set's row slices per thread
-    int fl_src[FW];
-    size_t fl_off[FW];
-    int fl_gg[FW];
-#pragma unroll
-    for (int k = 0; k < FW; ++k) {
-        const int wd = tid + k * NT;
-        fl_src[k] = wd;
-        fl_gg[k] = wd < GS * V ? wd / V : -1;
-        fl_off[k] = size_t(wd / V) * a.bp_steps * ROWB + size_t(rank) * ROWBC + size_t(wd % V) * 16;
-    }
-    auto flush_set = [&](int s, int t, int buf, long long tile0) {
-        if (t < t_store0) return;
-        const uint4* src = reinterpret_cast<const uint4*>(stage + size_t(buf) * G * ROWBC + size_t(s) * GS * ROWBC);
-        unsigned char* row0 = a.bp + (size_t(tile0 + s * GS) * a.bp_steps + (t - t_store0)) * ROWB;     // uniform
-#pragma unroll
-        for (int k = 0; k < FW; ++k)
-            if (fl_gg[k] >= 0 && tile0 + s * GS + fl_gg[k] < a.n) *reinterpret_cast<uint4*>(row0 + fl_off[k]) = src[fl_src[k]];
-    };
-
-    constexpr uint32_t kBufBytes = uint32_t(GS) * EC * 4;     // bytes every (set, buffer) receives per step
-    uint32_t parity = 0;          // bit (2*s + b): parity of the phase the next wait on mbarrier (s, b) is for
+    // Bytes buffer b of a set of GS tiles receives from OTHER CTAs per step.  The owner of edge e = h*Q + l is bits of h that
+    // start K below the rank's own: with C <= Q they are all bits of hl, and each CTA keeps 1/C of what it produces.  A larger
+    // cluster's upper owner bits are the rank's lowest ones: a CTA keeps 1/Q if those agree with its uppermost bits, else nothing.
+    constexpr int kUp = C > Q ? C / Q : 1;
+    const uint32_t tile_bytes = uint32_t(EC) * 4 - (kUp == 1 || rank / (C / kUp) == rank % kUp ? uint32_t(EC) * 4 / (C / kUp) : 0u);
     bool timed_out = false;
-    bool wait_pending = false;    // the barrier phase entered during the PREVIOUS step_set has not been closed yet
-    auto war_wait = [&]() {
-        if (wait_pending) {
-            cluster_wait_relaxed();
-            wait_pending = false;
-        }
-    };
 
     // All bytes of buffer b of set s have landed; then re-arm its mbarrier for the next use.
     // A wait that runs out is recorded (the launch's results are then invalid) and the thread
-    // carries on; it never re-arms an mbarrier again, because an arrive on an mbarrier whose phase
+    // carries on; it never arrives at an mbarrier again, because an arrive on an mbarrier whose phase
     // cannot complete would underflow its arrival count, which is a hardware error.  The byte
     // counts do not depend on the data, so a wait can only run out through a programming error,
     // which the tests would show on every run; the limit exists so that even then nothing hangs.
     // (`last`: the re-arm for the phase that the end-of-group wait checks; the wait self-test
     // inflates exactly that one, so that its timeouts happen after the last store has landed.)
-    auto wait_buffer = [&](int s, int b, bool last) {
+    auto wait_buffer = [&](int s, int b, uint32_t parity, bool last) __attribute__((always_inline)) {
         const uint32_t m = smem_u32(mbar + (2 * s + b));
-        if (!mbar_wait(m, (parity >> (2 * s + b)) & 1u, gave_up)) timed_out = true;
-        parity ^= 1u << (2 * s + b);
-        if (tid == 0 && !timed_out) mbar_expect(m, kBufBytes + (last ? uint32_t(a.inject_extra_bytes) : 0u));
+        if (!mbar_wait(m, parity, gave_up)) timed_out = true;
+        if (tid == 0 && !timed_out) mbar_expect(m, tile_bytes * uint32_t(s == 0 ? GA : GB) + (last ? uint32_t(a.inject_extra_bytes) : 0u));
     };
 
-    // One add-compare-select step of tile set `s` (tiles s*GS .. s*GS+GS-1), reading buffer `cur`.
-    // Half way through, the set's previous backpointer rows are streamed to HBM.
-    auto step_set = [&](int s, int t, int cur) {
-        if (t > 0) wait_buffer(s, cur, t == kT - 2);
+    // One add-compare-select step of tile set S (tiles T0 .. T0+GS-1 of the group), reading buffer CUR.
+    // row >= 0: the results are that metric row.  first: nothing to wait for (the pass's first step).
+    auto step_set = [&](auto set_c, auto cur_c, int t, uint32_t parity, int row, bool first, bool open_phase) __attribute__((always_inline)) {
+        constexpr int S = decltype(set_c)::value, CUR = decltype(cur_c)::value;
+        constexpr int T0 = S == 0 ? 0 : GA, GS = S == 0 ? GA : GB;
+        if (!first) wait_buffer(S, CUR, parity, t == a.steps - 2);
         f32x2 w2[GS];
 #pragma unroll
-        for (int gg = 0; gg < GS; ++gg) {
-            const float wt = wv[(s * GS + gg) * kT + ((t + a.roll) & (kT - 1))];
-            w2[gg] = pack2(wt, wt);
-        }
-        unsigned char* const st = stage + size_t(cur) * G * ROWBC;        // cur == t & 1
+        for (int g = 0; g < GS; ++g) w2[g] = *reinterpret_cast<const f32x2*>(wv + (T0 + g) * kT + ((t + a.roll) & (kT - 1)));
+        bool pending = open_phase;        // the barrier phase entered during the PREVIOUS step_set has not been closed yet
+        // The codebook is in registers, so tiles need not share anything: they go one at a time.  The next one's metrics are
+        // loaded ahead of this one's last store (which the compiler cannot move a load across): 3 % faster than at the
+        // tile's own beginning.  How far ahead is a matter of registers: from the start where the item is a part of a
+        // butterfly (K = 4), in the tile's second half with two tiles a set at K = 3 (558 us for 256 tiles, 577 from the
+        // end), at the end otherwise (804 us for 444 tiles with three a set; 847 and spills in the second half).
+        constexpr int kAhead = LU < Q ? 0 : GS == 2 && K == 3 ? R * 5 / 8 : R - 1;
+        float cin[2][Q][HB];
 #pragma unroll
-        for (int i = 0; i < NI; ++i) {
+        for (int q = 0; q < Q; ++q) ld_metrics<HB>(src + (T0 * 2 + CUR) * EC + q * HNC, cin[0][q]);
+        static_for<GS * NI>([&](auto gc) __attribute__((always_inline)) {
+            constexpr int gi = decltype(gc)::value, g = gi / NI, it = gi % NI, NX = gi + 1;
+            constexpr int OUT = (((T0 + g) * 2 + (CUR ^ 1)) * EC + it * DQ * HNC) * 4;
+            float outv[R];
+            static_for<R>([&](auto ic) __attribute__((always_inline)) {
+                constexpr int i = decltype(ic)::value;
+                float c[Q];
 #pragma unroll
-            for (int gg = 0; gg < GS; ++gg) {
-                // The codebook is in registers, so tiles need not share anything: one tile at a time
-                // keeps only Q predecessor metrics live and lets the next tile's loads fly under
-                // this tile's arithmetic.
-                f32x2 cin2[Q / 2];
-                const float* cin = cost + (size_t(s * GS + gg) * 2 + cur) * EC + h_loc[i];
+                for (int j = 0; j < Q / 2; ++j)
+                    unpack2(cand_cost2(w2[g], cbv[it * R + i][j], pack2(cin[gi & 1][2 * j][i / LU], cin[gi & 1][2 * j + 1][i / LU]), one2), c[2 * j], c[2 * j + 1]);
+                if constexpr (i == kAhead && NX < GS * NI) {
 #pragma unroll
-                for (int j = 0; j < Q / 2; ++j) cin2[j] = pack2(cin[(2 * j) * HNC], cin[(2 * j + 1) * HNC]);
-                constexpr int SV = LU < 4 ? LU : 4;            // successors per store (float2 or float4)
-                float outv[SV];
-                float tags = 0.0f;
-                const uint32_t d0 = dst[i] + uint32_t((size_t(s * GS + gg) * 2 + (cur ^ 1)) * EC * 4);
-                const uint32_t m = dst_bar[i] + uint32_t(2 * s + (cur ^ 1)) * 8u;
-#pragma unroll
-                for (int lu = 0; lu < LU; ++lu) {
-                    if (i == NI / 2 && gg == GS / 2 && lu == ((NI > 1 || GS > 1) ? 0 : LU / 2) && t > 0) flush_set(s, t - 1, cur ^ 1, tile0);
-                    float c[Q];
-#pragma unroll
-                    for (int j = 0; j < Q / 2; ++j)
-                        unpack2(cand_cost2(w2[gg], cbv[i][lu][j], cin2[j], one2), c[2 * j], c[2 * j + 1]);
-                    const float best = min_of<Q>(c);
-                    float tag = float((Q - 1) << (lu * K));
-#pragma unroll
-                    for (int q = Q - 2; q >= 0; --q) take_if_equal_balanced<Q>(q, tag, c[q], best, zero, float(q << (lu * K)));
-                    outv[lu % SV] = best;
-                    tags = __fadd_rn(tags, tag);
-                    if (i == NI - 1 && gg == GS - 1 && lu == 0) {
-                        // Every input of this step has been loaded AND used (the first successor of the
-                        // last tile of the last item consumed all of its predecessors' metrics), so this
-                        // thread no longer reads the input buffers: tell the cluster, well before anyone
-                        // needs to know.  (The barrier's phases are sequential: close the previous one first.)
-                        war_wait();
-                        cluster_arrive_relaxed();
-                    }
-                    if (lu % SV == SV - 1) {
-                        // Results leave as soon as a store's worth is ready (fewer live registers).
-                        // Write-after-read: the buffer written now was read by every CTA one step of this
-                        // set ago; the barrier phase that every thread entered during the previous
-                        // step_set (of the other set) proves it, and it is closed before the first store.
-                        war_wait();
-                        const uint32_t d = d0 + uint32_t(lu + 1 - SV) * 4u;
-                        if constexpr (SV == 2) st_async_v2(d, outv[0], outv[1], m);
-                        else st_async_v4(d, outv[0], outv[1], outv[2], outv[3], m);
-                    }
+                    for (int q = 0; q < Q; ++q) ld_metrics<HB>(src + ((T0 + NX / NI) * 2 + CUR) * EC + NX % NI * HI + q * HNC, cin[NX & 1][q]);
                 }
-                unsigned char* sb = st + (s * GS + gg) * ROWBC + ((e_out[i] - rank * EC) * K) / 8;
-                if constexpr (PAIRED) {
-                    // lanes 2m (chunk 0) and 2m+1 (chunk 1) hold the two halves of one butterfly's bits
-                    const float other = __shfl_xor_sync(0xffffffffu, tags, 1);
-                    if ((tid & 1) == 0) {
-                        const uint32_t bits = __float2uint_rz(tags) | (__float2uint_rz(other) << ITEM_BITS);
-#pragma unroll
-                        for (int b = 0; b < 2 * ITEM_BITS / 8; ++b) sb[b] = (unsigned char)(bits >> (8 * b));
-                    }
-                } else {
-                    const uint32_t bits = __float2uint_rz(tags);
-#pragma unroll
-                    for (int b = 0; b < ITEM_BITS / 8; ++b) sb[b] = (unsigned char)(bits >> (8 * b));
+                outv[i] = min_tree<Q>(c);
+                if constexpr (gi == GS * NI - 1 && i == R - LU) {
+                    // Every input of this step has been loaded AND used (the first successor of the
+                    // last tile's last butterfly consumed all of its predecessors' metrics), so this
+                    // thread no longer reads the input buffers: tell the cluster, well before anyone
+                    // needs to know.  (The barrier's phases are sequential: close the previous one first.)
+                    if (pending) cluster_wait_relaxed();
+                    pending = false;
+                    cluster_arrive_relaxed();
                 }
+                if constexpr (i % SV == SV - 1) {
+                    // Results leave as soon as a store's worth is ready.
+                    // Write-after-read: the buffer written now was read by every CTA one step of this
+                    // set ago; the barrier phase that every thread entered during the previous
+                    // step_set proves it, and it is closed before the first store.
+                    if (pending) cluster_wait_relaxed();
+                    pending = false;
+                    if (local) st_local<OUT, SV>(dst[i / SV], outv + (i + 1 - SV));
+                    else st_remote<OUT, (2 * S + (CUR ^ 1)) * 8, SV>(dst[i / SV], outv + (i + 1 - SV), dst_bar);
+                }
+            });
+            if (row >= 0 && T0 + g < live) {
+                float* const rp = row_tile0 + (size_t(T0 + g) * ca.nrows + row) * E + row_off + it * (HI * Q >> MR::LB);
+#pragma unroll
+                for (int i = 0; i < R; ++i) rp[i * MR::NA] = outv[i];
             }
-        }
-        wait_pending = true;          // the phase entered above is closed during the next step_set
+        });
+        __syncwarp();                 // this warp's local stores, then its arrival (which releases them to the CTA)
+        if (lane == 0 && !timed_out) mbar_arrive(smem_u32(mbar + 2 * S + (CUR ^ 1)));
     };
 
     if ((a.flags & kFwdResetStatus) && blockIdx.x == 0 && tid == 0 && a.status != nullptr) atomicExch(a.status, 0u);
 
-    // ---- mbarriers: one arrival (the re-arming thread) plus kBufBytes of stores per phase ----
+    // ---- mbarriers: the arrivals of the re-arming thread and of every warp (its local stores) plus the bytes of the remote
+    //      stores, per phase ----
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mbar_init(smem_u32(mbar + i), 1);
+        for (int i = 0; i < 4; ++i) mbar_init(smem_u32(mbar + i), 1 + NT / 32);
         mbar_fence_init();
         *gave_up = 0u;
     }
     cluster.sync();                      // every CTA's mbarriers exist before anyone can signal them
     if (tid == 0) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) mbar_expect(smem_u32(mbar + i), kBufBytes);
+        for (int i = 0; i < (GB > 0 ? 4 : 2); ++i) mbar_expect(smem_u32(mbar + i), tile_bytes * uint32_t(i < 2 ? GA : GB));
     }
 
     for (long long grp = cluster_id; grp < ngroups; grp += nclusters) {
-        tile0 = grp * G;
+        const long long tile0 = grp * G;
+        live = int(a.n - tile0 < G ? a.n - tile0 : G);
+        row_tile0 = ca.rows + size_t(tile0) * ca.nrows * E;
         // ---- weights and initial metrics (src/trellis/qtip.py:161-165) ----
         for (int i = tid; i < G * kT; i += NT) {
-            const long long tile = tile0 + (i >> 8);
             int t = i & 255;
-            const float x = tile < a.n ? load_weight(a, tile, i & 255, t) : 0.0f;
-            wv[(i & ~255) | t] = x;
+            const float x = (i >> 8) < live ? load_weight(a, tile0 + (i >> 8), i & 255, t) : 0.0f;
+            wv[(i & ~255) | t] = make_float2(x, x);
             if ((a.flags & kFwdCheckFinite) && !isfinite(x) && rank == 0 && a.status != nullptr) atomicOr(a.status, 2u);   // reported, never trapped on
         }
         {
@@ -344,41 +373,42 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
         }
         __syncthreads();
         if (constrained && tid < G) {
-            const long long tile = tile0 + tid;
-            const int ov = (tile < a.n ? a.overlap[tile] : 0) & (E - 1);
-            const int qn = ov / HN, hn = ov % HN;                 // metric of edge ov is predecessor qn of butterfly hn
-            if (hn / HNC == rank) cost[(size_t(tid) * 2) * EC + qn * HNC + (hn % HNC)] = 0.0f;
+            const int ov = (tid < live ? a.overlap[tile0 + tid] : 0) & (E - 1);
+            const int qo = ov / HN, ho = ov % HN;                 // metric of edge ov is predecessor qo of butterfly ho
+            if (ho / HNC == rank) cost[(size_t(tid) * 2) * EC + qo * HNC + slot(ho % HNC)] = 0.0f;
         }
         cluster.sync();   // every CTA's buffers are initialised before anyone stores into them
 
         // The two tile sets alternate; every step_set waits for its input buffer's bytes, computes,
         // waits for the previous step_set's barrier phase before its first store, stores, arrives.
         // (two steps per trip, so that the buffer index is a constant in every instance of step_set)
-        step_set(0, 0, 0);
-        for (int t = 0; t < kT; t += 2) {
-            step_set(1, t, 0);
-            step_set(0, t + 1, 1);
-            step_set(1, t + 1, 1);
-            if (t + 2 < kT) step_set(0, t + 2, 0);
+        // A group's waits on each buffer are an even number (steps / 2), so the phase parities start every group at 0 and
+        // alternate from trip to trip.
+        using C0 = std::integral_constant<int, 0>;
+        using C1 = std::integral_constant<int, 1>;
+        step_set(C0{}, C0{}, 0, 0u, MR::row_after(0, a.steps, ca.nrows), true, false);
+        uint32_t ph = 0;                                  // parity of the waits on buffer 1 of this trip
+#pragma unroll 1
+        for (int t = 0; t < a.steps; t += 2) {
+            const int row1 = MR::row_after(t + 1, a.steps, ca.nrows);
+            if constexpr (GB > 0) step_set(C1{}, C0{}, t, ph ^ 1u, MR::row_after(t, a.steps, ca.nrows), t == 0, true);
+            step_set(C0{}, C1{}, t + 1, ph, row1, false, true);
+            if constexpr (GB > 0) step_set(C1{}, C1{}, t + 1, ph, row1, false, true);
+            if (t + 2 < a.steps) step_set(C0{}, C0{}, t + 2, ph, MR::row_after(t + 2, a.steps, ca.nrows), false, true);
+            ph ^= 1u;
         }
-        cluster_wait_relaxed();          // closes the phase opened by the last step_set
-        wait_pending = false;
-        wait_buffer(0, 0, false);        // step 255 wrote the final metrics into buffer 0
-        wait_buffer(1, 0, false);
-        // The barrier phase above was entered at the START of the last step_set, so it says nothing
-        // about that step's backpointer bytes; the rows are CTA-local, a CTA barrier orders them.
+        cluster_wait_relaxed();             // closes the phase opened by the last step_set
+        wait_buffer(0, 0, 1u, false);       // the last step wrote the final metrics into buffer 0
+        if constexpr (GB > 0) wait_buffer(1, 0, 1u, false);
         __syncthreads();
-        flush_set(0, kT - 1, (kT - 1) & 1, tile0);
-        flush_set(1, kT - 1, (kT - 1) & 1, tile0);
 
-        // ---- final metrics live in buffer 0 (256 steps), layout [Q][HNC] = edges q*HN + rank*HNC + hl ----
-        const int fin = 0;
+        // ---- final metrics live in buffer 0 (an even number of steps), layout [Q][HNC] = edges q*HN + rank*HNC + hl ----
         if (ca.keys != nullptr) {
             for (int g = 0; g < G; ++g) {
-                const float* fv = cost + (size_t(g) * 2 + fin) * EC;
+                const float* fv = cost + (size_t(g) * 2) * EC;
                 unsigned long long key = ~0ull;
                 for (int i = tid; i < EC; i += NT) {
-                    const unsigned edge = unsigned(i / HNC) * HN + rank * HNC + (i % HNC);
+                    const unsigned edge = unsigned(i / HNC) * HN + rank * HNC + unslot(i % HNC);
                     const unsigned long long k2 = (static_cast<unsigned long long>(__float_as_uint(fv[i])) << 32) | edge;
                     key = k2 < key ? k2 : key;
                 }
@@ -387,7 +417,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                     const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, off);
                     key = o < key ? o : key;
                 }
-                if ((tid & 31) == 0) red[tid >> 5] = key;
+                if (lane == 0) red[tid >> 5] = key;
                 __syncthreads();
                 if (tid < 32) {
                     unsigned long long k2 = tid < NT / 32 ? red[tid] : ~0ull;
@@ -396,19 +426,15 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                         const unsigned long long o = __shfl_xor_sync(0xffffffffu, k2, off);
                         k2 = o < k2 ? o : k2;
                     }
-                    const long long tile = tile0 + g;
-                    if (tid == 0 && tile < a.n) ca.keys[tile * C + rank] = k2;
+                    if (tid == 0 && g < live) ca.keys[(tile0 + g) * C + rank] = k2;
                 }
                 __syncthreads();
             }
         }
-        if (a.final_cost != nullptr && constrained && tid < G) {
-            const long long tile = tile0 + tid;
-            if (tile < a.n) {
-                const int ov = a.overlap[tile] & (E - 1);
-                const int qn = ov / HN, hn = ov % HN;
-                if (hn / HNC == rank) a.final_cost[tile] = cost[(size_t(tid) * 2 + fin) * EC + qn * HNC + (hn % HNC)];
-            }
+        if (a.final_cost != nullptr && constrained && tid < live) {
+            const int ov = a.overlap[tile0 + tid] & (E - 1);
+            const int qo = ov / HN, ho = ov % HN;
+            if (ho / HNC == rank) a.final_cost[tile0 + tid] = cost[(size_t(tid) * 2) * EC + qo * HNC + slot(ho % HNC)];
         }
         cluster.sync();   // nobody may start re-initialising while a neighbour still reads or is written to
     }

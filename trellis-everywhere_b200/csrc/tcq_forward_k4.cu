@@ -4,49 +4,51 @@
 namespace tcq {
 
 namespace {
-constexpr int kNT = 512;     // threads per CTA
-constexpr int kLU = 4;       // successors per work item, single-CTA kernel
-constexpr int kGMax = 3;     // most tiles one CTA advances together (shared-memory bound)
-constexpr int kCLU4 = 2;     // successors per work item with 4 CTAs per cluster (32 codebook values per thread)
-constexpr int kCLU2 = 4;     // ... with 2 CTAs per cluster (64 codebook values per thread)
+template <int CB>
+cudaError_t launch_cluster_cb(const ClusterArgs& ca, int C, int G, cudaStream_t stream) {
+    switch (100 * C + G) {                       // the shapes of pick_cluster
+        case 801: return launch_cluster_variant<4, CB, 8, 1, 0, 256>(ca, stream);
+        case 802: return launch_cluster_variant<4, CB, 8, 1, 1, 256>(ca, stream);
+        case 401: return launch_cluster_variant<4, CB, 4, 1, 0, 512>(ca, stream);
+        case 402: return launch_cluster_variant<4, CB, 4, 1, 1, 512>(ca, stream);
+        case 201: return launch_cluster_variant<4, CB, 2, 1, 0, 512>(ca, stream);
+        case 202: return launch_cluster_variant<4, CB, 2, 1, 1, 512>(ca, stream);
+        case 203: return launch_cluster_variant<4, CB, 2, 2, 1, 512>(ca, stream);
+        case 204: return launch_cluster_variant<4, CB, 2, 2, 2, 512>(ca, stream);
+        case 205: return launch_cluster_variant<4, CB, 2, 3, 2, 512>(ca, stream);
+        case 206: return launch_cluster_variant<4, CB, 2, 3, 3, 512>(ca, stream);
+        default: return cudaErrorInvalidValue;
+    }
+}
 
 template <int CB>
-cudaError_t launch_cb(const ForwardArgs& a, unsigned long long* keys, int num_sms, cudaStream_t stream, int* nkeys) {
-    *nkeys = 0;
-    const int csize = cluster_size_choice();
-    if (keys != nullptr && csize != 0) {
-        cudaError_t err;
-        if (csize == 2) {
-            switch (pick_cluster_set(a.n, num_sms, 2, 3)) {
-                case 1: err = launch_cluster_variant<4, CB, 2, 1, kNT, kCLU2>(a, keys, stream); break;
-                case 2: err = launch_cluster_variant<4, CB, 2, 2, kNT, kCLU2>(a, keys, stream); break;
-                default: err = launch_cluster_variant<4, CB, 2, 3, kNT, kCLU2>(a, keys, stream); break;
-            }
-        } else {
-            err = pick_cluster_set(a.n, num_sms, 4, 2) == 2 ? launch_cluster_variant<4, CB, 4, 2, kNT, kCLU4>(a, keys, stream)
-                                                           : launch_cluster_variant<4, CB, 4, 1, kNT, kCLU4>(a, keys, stream);
-        }
-        if (err != cudaErrorNotSupported) {
-            *nkeys = csize;
-            return err;
-        }
-    }
-    switch (pick_group<kGMax>(a.n, num_sms)) {
-        case 1: return launch_variant<4, CB, 1, kNT, kLU>(a, num_sms, stream);
-        case 2: return launch_variant<4, CB, 2, kNT, kLU>(a, num_sms, stream);
-        case 3: return launch_variant<4, CB, 3, kNT, kLU>(a, num_sms, stream);
+cudaError_t launch_cta_cb(const ForwardArgs& a, int num_sms, cudaStream_t stream) {
+    constexpr int NT = 512, LU = 4;
+    switch (pick_group<3>(a.n, num_sms)) {
+        case 1: return launch_variant<4, CB, 1, NT, LU>(a, num_sms, stream);
+        case 2: return launch_variant<4, CB, 2, NT, LU>(a, num_sms, stream);
+        case 3: return launch_variant<4, CB, 3, NT, LU>(a, num_sms, stream);
         default: return cudaErrorInvalidValue;
     }
 }
 }  // namespace
 
 template <>
-cudaError_t launch_forward<4>(int codebook, const ForwardArgs& a, unsigned long long* keys, int num_sms,
-                               cudaStream_t stream, int* nkeys) {
+cudaError_t launch_forward_cluster<4>(int codebook, const ClusterArgs& ca, int C, int G, cudaStream_t stream) {
     switch (codebook) {
-        case kCb1Mad:  return launch_cb<kCb1Mad>(a, keys, num_sms, stream, nkeys);
-        case kCb3Inst: return launch_cb<kCb3Inst>(a, keys, num_sms, stream, nkeys);
-        case kCbMcg:   return launch_cb<kCbMcg>(a, keys, num_sms, stream, nkeys);
+        case kCb1Mad:  return launch_cluster_cb<kCb1Mad>(ca, C, G, stream);
+        case kCb3Inst: return launch_cluster_cb<kCb3Inst>(ca, C, G, stream);
+        case kCbMcg:   return launch_cluster_cb<kCbMcg>(ca, C, G, stream);
+        default:       return cudaErrorInvalidValue;
+    }
+}
+
+template <>
+cudaError_t launch_forward_cta<4>(int codebook, const ForwardArgs& a, int num_sms, cudaStream_t stream) {
+    switch (codebook) {
+        case kCb1Mad:  return launch_cta_cb<kCb1Mad>(a, num_sms, stream);
+        case kCb3Inst: return launch_cta_cb<kCb3Inst>(a, num_sms, stream);
+        case kCbMcg:   return launch_cta_cb<kCbMcg>(a, num_sms, stream);
         default:       return cudaErrorInvalidValue;
     }
 }

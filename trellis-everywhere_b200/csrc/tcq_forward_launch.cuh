@@ -46,16 +46,23 @@ static cudaError_t launch_variant(const ForwardArgs& a, int num_sms, cudaStream_
     return cudaGetLastError();
 }
 
-// Cluster form.  Returns cudaErrorNotSupported (and launches nothing) if this device cannot
-// co-schedule a cluster of C CTAs with the kernel's shared-memory footprint.
-template <int K, int CB, int C, int GS, int NT, int LU>
-static cudaError_t launch_cluster_variant(const ForwardArgs& a, unsigned long long* keys, cudaStream_t stream) {
-    auto kern = tcq_forward_cluster_kernel<K, CB, C, GS, NT, LU>;
-    constexpr size_t smem = cluster_smem_bytes<K, C, GS>();
+constexpr size_t kOneCtaPerSm = 116 * 1024;        // dynamic shared memory of which an SM (228 KiB) holds one
+
+// Cluster form with clusters of C CTAs, tile sets of GS and LU successors per work item.  How many clusters of this
+// shape the device runs at once is asked once per device; a launch uses at most that many.
+template <int K, int CB, int C, int GA, int GB, int NT>
+static cudaError_t launch_cluster_variant(const ClusterArgs& ca, cudaStream_t stream) {
+    auto kern = tcq_forward_cluster_kernel<K, CB, C, GA, GB, NT>;
+    // Never less than half of what an SM has: two small CTAs on one SM leave another SM idle, and a step takes as long as
+    // the slowest CTA of its cluster.
+    constexpr size_t need = cluster_smem_bytes<K, C, GA, GB>(), smem = need < kOneCtaPerSm ? kOneCtaPerSm : need;
     static bool optin[kMaxDeviceOrdinals] = {false};
     int dev = -1;
     cudaError_t err = device_slot(&dev);
     if (err != cudaSuccess) return err;
+    if (C > 8 && (dev < 0 || !optin[dev])) {
+        if ((err = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return err;
+    }
     if ((err = ensure_smem_optin(kern, smem, optin, dev)) != cudaSuccess) return err;
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeClusterDimension;
@@ -82,42 +89,15 @@ static cudaError_t launch_cluster_variant(const ForwardArgs& a, unsigned long lo
         if (dev >= 0) max_clusters[dev] = maxc;    // cached only when the query itself succeeded
     }
     if (maxc < 0) return cudaErrorNotSupported;
-    constexpr int G = 2 * GS;
-    const long long ngroups = (a.n + G - 1) / G;
+    if (ca.f.n <= 0) {                             // a query only
+        if (ca.at_once != nullptr) *ca.at_once = maxc;
+        return cudaSuccess;
+    }
+    constexpr int G = GA + GB;
+    const long long ngroups = (ca.f.n + G - 1) / G;
     const long long ncl = ngroups < maxc ? ngroups : maxc;
     cfg.gridDim = dim3(unsigned(ncl * C));
-    ClusterArgs ca{a, keys};
     return cudaLaunchKernelEx(&cfg, kern, ca);
-}
-
-// Tiles per set (a cluster advances two sets): the size that finishes n tiles soonest on the
-// device's clusters, counting whole rounds of groups and a fixed cost per round.  Measured on a
-// B200 at K = 3, one round of 2 / 4 / 6 tiles per cluster takes 1.12 / 1.91 / 2.74 ms, i.e.
-// 0.406 ms x (tiles + 0.75).
-static inline int pick_cluster_set(long long n, int num_sms, int C, int gs_max) {
-    const long long clusters = num_sms / C > 0 ? num_sms / C : 1;
-    int best = 1;
-    double best_t = 1e300;
-    for (int gs = 1; gs <= gs_max; ++gs) {
-        const long long groups = (n + 2 * gs - 1) / (2 * gs);
-        const long long rounds = (groups + clusters - 1) / clusters;
-        const double t = double(rounds) * (2.0 * gs + 0.75);
-        if (t < best_t - 1e-9) { best_t = t; best = gs; }
-    }
-    return best;
-}
-
-// Which step kernel runs.  Returns the cluster size (2 or 4) or 0 for the single-CTA kernel.
-// Default: 2-CTA clusters (all 148 SMs of a B200 pair up; clusters of 4 leave 16 SMs idle).
-// TCQ_FORWARD_KERNEL = cta | cluster2 | cluster4 overrides it for comparison runs; the single-CTA
-// kernel is also the fallback on a device that cannot co-schedule clusters.
-static inline int cluster_size_choice() {
-    const char* v = std::getenv("TCQ_FORWARD_KERNEL");
-    if (v != nullptr) {
-        if (std::strcmp(v, "cta") == 0) return 0;
-        if (std::strcmp(v, "cluster4") == 0) return 4;
-    }
-    return 2;
 }
 
 // Relative time of one group of G tiles: G tiles of add-compare-select work plus

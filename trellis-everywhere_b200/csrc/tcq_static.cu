@@ -3,7 +3,7 @@
 // Some hosts of this library may not call cudaMalloc at the point where they need the encoder:
 // a plugin running inside another framework's memory budget, a service that fixed its device
 // footprint at start-up.  tcq_encode_tb asks such a
-// caller for a workspace it has no way to obtain.  This entry point needs none: the backpointer
+// caller for a workspace it has no way to obtain.  This entry point needs none: the
 // scratch is a fixed array in the library's own device image.
 //
 //   * The array is TCQ_STATIC_SCRATCH_BYTES (32 MiB) and is part of every GPU context that loads
@@ -13,10 +13,10 @@
 //   * The first call on each device looks up the array's device address (with that device
 //     current) and remembers it.  Make that first call outside any stream capture.
 //   * All calls share the one array and it keeps whatever the previous call left in it.  The
-//     encoder never reads a byte it has not written earlier in the same call (every backpointer
+//     encoder never reads a byte it has not written earlier in the same call (every metric
 //     row, argmin edge and overlap word is produced before it is consumed), so nothing has to be
 //     cleared; but two calls whose kernels overlap on the GPU (different streams, no dependency)
-//     overwrite each other's backpointers.  Serialise them.
+//     overwrite each other's rows.  Serialise them.
 //   * tcq_encode_tb_static_status(stream) is tcq_workspace_status for this path: the status word
 //     (a bounded in-kernel wait gave up / a weight was NaN or infinite) lives inside the array, where a
 //     caller without the array's address could not otherwise read it.  It reports on the LAST call made
@@ -27,7 +27,7 @@
 // unrelated memory.  The address comes from cudaGetSymbolAddress below.
 #include "../../include/tcq_b200.h"
 
-#include <cuda_runtime.h>
+#include "tcq_traceback.cuh"
 
 namespace {
 
@@ -73,7 +73,7 @@ int64_t tcq_encode_tb_static_max_tiles(int K) {
     static int64_t cached[5] = {0, 0, 0, 0, 0};
     if (cached[K] == 0) {
         int64_t n = 0;
-        while (tcq_workspace_bytes(n + 1, K) <= size_t(TCQ_STATIC_SCRATCH_BYTES)) ++n;
+        while (tcq::backpointer_workspace_bytes(n + 1, K) <= size_t(TCQ_STATIC_SCRATCH_BYTES)) ++n;
         cached[K] = n;
     }
     return cached[K];

@@ -69,7 +69,7 @@ _workspaces_lock = threading.Lock()
 
 
 def _workspace(dev: torch.device, n_tiles: int, K: int) -> torch.Tensor:
-    """Grow-only scratch per (device, stream): backpointers and per-tile hand-off words.
+    """Grow-only scratch per (device, stream): path metrics for the traceback and per-tile hand-off words.
 
     Kernels of one stream run one after another, so a stream's calls can share one block; calls on
     different streams may overlap and get different blocks.  Code that creates streams of its own
