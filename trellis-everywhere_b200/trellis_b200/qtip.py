@@ -43,10 +43,10 @@ CodebookLike = Union[str, int, torch.Tensor]
 
 # --------------------------------------------------------------------------- plumbing
 def _cuda_device(t: Optional[torch.Tensor] = None) -> torch.device:
-    if not torch.cuda.is_available():
-        raise RuntimeError("trellis_b200 needs a CUDA device (sm_100a); there is no CPU fallback")
     if t is not None and t.is_cuda:
         return t.device
+    if not torch.cuda.is_available():
+        raise RuntimeError("trellis_b200 needs a CUDA device (sm_100a); there is no CPU fallback")
     return torch.device("cuda", torch.cuda.current_device())
 
 
@@ -54,8 +54,26 @@ def _stream(dev: torch.device) -> int:
     return torch.cuda.current_stream(dev).cuda_stream
 
 
+def _call(dev: torch.device, name: str, *args) -> None:
+    """One C-ABI call on ``dev`` and its current stream (the call's last argument); raises on a negative status.
+
+    The small calls (unpacking a few tiles, one product in token generation) last a few microseconds on the GPU, less than what
+    leads up to them here; so the device is switched only when it is not the current one.
+    """
+    fn = getattr(_lib.lib(), name)
+    if torch.cuda.current_device() == dev.index:
+        rc = fn(*args, _stream(dev))
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(*args, _stream(dev))
+    if rc != 0:
+        _lib.check(rc, name)
+
+
 def _to_dev(t: torch.Tensor, dev: torch.device, dtype: torch.dtype) -> torch.Tensor:
     """Contiguous tensor of `dtype` on `dev`; host tensors go through pinned memory."""
+    if t.dtype == dtype and t.device == dev and t.is_contiguous():
+        return t
     if t.is_cuda:
         return t.to(device=dev, dtype=dtype).contiguous()
     t = t.to(dtype).contiguous()
@@ -191,13 +209,11 @@ def _encode_device(wd: torch.Tensor, K: int, cid: int, packed, dq, sse, bits) ->
         return
     dev = wd.device
     ws = _workspace(dev, n, K)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().tcq_encode_tb(wd.data_ptr(), n, K, cid, packed.data_ptr(),
-                                      bits.data_ptr() if bits is not None else None,
-                                      dq.data_ptr() if dq is not None else None,
-                                      sse.data_ptr() if sse is not None else None,
-                                      ws.data_ptr(), ws.numel(), _stream(dev))
-    _lib.check(rc, "tcq_encode_tb")
+    _call(dev, "tcq_encode_tb", wd.data_ptr(), n, K, cid, packed.data_ptr(),
+          bits.data_ptr() if bits is not None else None,
+          dq.data_ptr() if dq is not None else None,
+          sse.data_ptr() if sse is not None else None,
+          ws.data_ptr(), ws.numel())
 
 
 @torch.no_grad()
@@ -239,12 +255,10 @@ def encode_rows(src: torch.Tensor, comp: Optional[torch.Tensor], K: int, codeboo
     if n_out == 0:
         return
     ws = _workspace(dev, n_out // 16, K)
-    with torch.cuda.device(dev):
-        rc = _lib.lib().tcq_encode_tb_rows(src.data_ptr(), comp.data_ptr() if comp is not None else None, ld, n_out, K, cid,
-                                           packed.data_ptr() if packed is not None else None, pstride, wq.data_ptr(),
-                                           err.data_ptr() if err is not None else None,
-                                           sse.data_ptr() if sse is not None else None, ws.data_ptr(), ws.numel(), _stream(dev))
-    _lib.check(rc, "tcq_encode_tb_rows")
+    _call(dev, "tcq_encode_tb_rows", src.data_ptr(), comp.data_ptr() if comp is not None else None, ld, n_out, K, cid,
+          packed.data_ptr() if packed is not None else None, pstride, wq.data_ptr(),
+          err.data_ptr() if err is not None else None,
+          sse.data_ptr() if sse is not None else None, ws.data_ptr(), ws.numel())
 
 
 _HOST_CHUNK = 2 * 3552          # tiles per pipelined chunk of a host-tensor encode (two workspace chunks)
@@ -414,13 +428,11 @@ def decode_packed(packed: torch.Tensor, K: int, codebook: CodebookLike) -> torch
     dev = _cuda_device(packed)
     if packed.dtype not in (torch.int32, torch.uint32):
         raise ValueError("packed words must be int32 or uint32")
-    pd = _to_dev(packed.view(torch.int32), dev, torch.int32)
+    pd = _to_dev(packed if packed.dtype == torch.int32 else packed.view(torch.int32), dev, torch.int32)
     n = pd.shape[0]
     dq = torch.empty((n, T_SEQ), dtype=torch.float32, device=dev)
     if n:
-        with torch.cuda.device(dev):
-            rc = _lib.lib().tcq_decode_packed(pd.data_ptr(), n, K, cid, dq.data_ptr(), _stream(dev))
-        _lib.check(rc, "tcq_decode_packed")
+        _call(dev, "tcq_decode_packed", pd.data_ptr(), n, K, cid, dq.data_ptr())
     return dq if packed.is_cuda else dq.cpu()
 
 
@@ -445,18 +457,16 @@ def decode_matvec(packed: torch.Tensor, n_out: int, k_in: int, K: int, codebook:
         raise ValueError(f"x must be [{k_in}] or [m, {k_in}], got {tuple(x.shape)}")
     cid = codebook_id(codebook)
     dev = _cuda_device(packed if packed.is_cuda else (x if x.is_cuda else None))
-    pd = _to_dev(packed.view(torch.int32), dev, torch.int32)
-    xd = _to_dev(x.reshape(-1, k_in), dev, torch.float32)
+    pd = _to_dev(packed if packed.dtype == torch.int32 else packed.view(torch.int32), dev, torch.int32)
+    xd = _to_dev(x if x.dim() == 2 and k_in else x.reshape(-1, k_in), dev, torch.float32)
     m = xd.shape[0]
     y = torch.empty((m, n_out), dtype=torch.float32, device=dev)
     if k_in == 0:
         y.zero_()
     elif m and n_out:
-        with torch.cuda.device(dev):
-            rc = _lib.lib().tcq_decode_matvec(pd.data_ptr(), n_out, k_in, K, cid, xd.data_ptr(), k_in, m, y.data_ptr(), n_out,
-                                              _stream(dev))
-        _lib.check(rc, "tcq_decode_matvec")
-    y = y.reshape(*x.shape[:-1], n_out)
+        _call(dev, "tcq_decode_matvec", pd.data_ptr(), n_out, k_in, K, cid, xd.data_ptr(), k_in, m, y.data_ptr(), n_out)
+    if x.dim() == 1:
+        y = y.reshape(n_out)
     return y if (packed.is_cuda or x.is_cuda) else y.cpu()
 
 
@@ -550,8 +560,9 @@ class IPContext:
         n, k = w.shape
         self.block = block
         self.shape = (n, k)
-        self.sv = (torch.randint(0, 2, (n,), generator=gen).float() * 2 - 1).to(w.device)
-        self.su = (torch.randint(0, 2, (k,), generator=gen).float() * 2 - 1).to(w.device)
+        # the reference's two randint draws, in one go: the generator gives one number per sign whatever the type and the count
+        signs = torch.empty(n + k, dtype=torch.float32).random_(0, 2, generator=gen).mul_(2).sub_(1).to(w.device)
+        self.sv, self.su = signs[:n], signs[n:]
         self._z = self._tiles = self._scale = self._scale_t = None
         self.on_device = bool(w.is_cuda and block == 128 and n % 16 == 0 and k % 16 == 0 and 0 < n <= 16 * 65535 and k > 0)
         if self.on_device:
@@ -562,11 +573,8 @@ class IPContext:
             self.in_s = torch.empty(k, dtype=torch.float32, device=dev)
             self._scale_t = torch.empty(1, dtype=torch.float32, device=dev)
             ws = self._ip_workspace(dev)
-            with torch.cuda.device(dev):
-                rc = _lib.lib().tcq_ip_forward(wd.data_ptr(), n, k, self.sv.data_ptr(), self.su.data_ptr(), float(cb_rms), 1,
-                                               self._tiles.data_ptr(), self.out_s.data_ptr(), self.in_s.data_ptr(),
-                                               self._scale_t.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev))
-            _lib.check(rc, "tcq_ip_forward")
+            _call(dev, "tcq_ip_forward", wd.data_ptr(), n, k, self.sv.data_ptr(), self.su.data_ptr(), float(cb_rms), 1,
+                  self._tiles.data_ptr(), self.out_s.data_ptr(), self.in_s.data_ptr(), self._scale_t.data_ptr(), ws.data_ptr(), ws.numel())
             return
         z = w * self.sv[:, None] * self.su[None, :]
         out_s = z.square().mean(dim=1).sqrt().clamp_min(1e-8)
@@ -608,11 +616,8 @@ class IPContext:
         zd = zq.to(device=dev, dtype=torch.float32).contiguous()
         out = torch.empty((n, k), dtype=torch.float32, device=dev)
         ws = self._ip_workspace(dev)
-        with torch.cuda.device(dev):
-            rc = _lib.lib().tcq_ip_restore(zd.data_ptr(), int(tiled), n, k, self.sv.data_ptr(), self.su.data_ptr(),
-                                           self.out_s.data_ptr(), self.in_s.data_ptr(), self._scale_t.data_ptr(),
-                                           out.data_ptr(), ws.data_ptr(), ws.numel(), _stream(dev))
-        _lib.check(rc, "tcq_ip_restore")
+        _call(dev, "tcq_ip_restore", zd.data_ptr(), int(tiled), n, k, self.sv.data_ptr(), self.su.data_ptr(), self.out_s.data_ptr(),
+              self.in_s.data_ptr(), self._scale_t.data_ptr(), out.data_ptr(), ws.data_ptr(), ws.numel())
         return out
 
     def restore(self, zq: torch.Tensor) -> torch.Tensor:
