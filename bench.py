@@ -286,7 +286,7 @@ def check_parity(torch, qtip, lib, _lib, tiles, last, dev, cid) -> dict:
     ok_sse = np.array_equal(last.sse[idx].cpu().numpy().view(np.uint32), sse.view(np.uint32))
     # the launches the roofline leg times: one full chunk through the pass-level entry point (same launch code and
     # tile-group shape as tcq_forward_pass), states of 64 spread tiles against the oracle's passes
-    chunk = min(n, 24 * torch.cuda.get_device_properties(dev).multi_processor_count)
+    chunk = min(n, 6 * torch.cuda.get_device_properties(dev).multi_processor_count)
     s1 = qtip.viterbi_pass_b200(tiles[:chunk], K_BITS, None, cid, roll=128)
     jdx = torch.linspace(0, chunk - 1, min(64, chunk), device=dev).round().long()
     w2 = tiles[:chunk][jdx].cpu().numpy()
@@ -456,7 +456,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
         raise SystemExit("end-to-end leg produced different codes than the device-resident leg")
 
     # ---- the step kernel alone (roofline), one chunk per launch exactly as encode uses it ----
-    chunk = min(n, 24 * torch.cuda.get_device_properties(dev).multi_processor_count)
+    chunk = min(n, 6 * torch.cuda.get_device_properties(dev).multi_processor_count)
     ws = qtip._workspace(dev, chunk, K_BITS)
     ov = torch.randint(0, 1 << (16 - K_BITS), (chunk,), dtype=torch.int32, device=dev)
     stream = torch.cuda.current_stream(dev).cuda_stream
@@ -504,7 +504,8 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
         avg_kernel_ms = sum(kern_ms) / 2
         evals_per_launch = chunk * T_SEQ * 65536
         achieved = evals_per_launch * LANE_OPS_PER_EVAL / (avg_kernel_ms * 1e-3)
-        bp_bytes = chunk * (128 + 256) / 2 * (1 << (16 - K_BITS)) * K_BITS / 8      # mean of the two passes
+        # metric rows of every 5th / 3rd / 2nd step, 4 bytes an edge: mean of the two passes
+        row_bytes = chunk * {2: (26 + 51) / 2, 3: (43 + 85) / 2, 4: (64 + 127) / 2}[K_BITS] * (1 << (16 - K_BITS)) * 4
         ck = clocks.summary()
         roofline = {
             "bound": "alu", "kernel": f"Viterbi step kernel (tcq_forward_cluster_kernel, K={K_BITS}, {CODEBOOK}, 2 CTAs per cluster)",
@@ -515,11 +516,11 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
             "algorithmic": "4 lane-ops (fsub, fmul, fadd, compare-select) x 65536 state evaluations per tile-step",
             "launch_ms": {"pass1": kern_ms[0], "pass2": kern_ms[1]}, "tiles_per_launch": chunk,
             "frac_at_sampled_clock": (achieved / (sms * 128 * ck["sm_mhz"] * 1e6)) if ck.get("sm_mhz") else None,
-            # ncu dram__bytes_read+write of an 888-tile launch pair = 0.89 of its algorithmic backpointer bytes
-            # (profiles/step_kernel_k3_3inst_888tiles_ncu_full.md), scaled here by the tiles per launch
-            "traffic": 0.89 * bp_bytes,
-            "hbm": {"algorithmic_bytes_per_launch": bp_bytes, "achieved_GBps": bp_bytes / (avg_kernel_ms * 1e-3) / 1e9,
-                    "peak_GBps": peaks.get("hbm_gbs"), "note": "packed backpointer stream, K bits per edge per step"},
+            # ncu dram__bytes_read+write of a 444-tile launch pair against its metric rows
+            # (profiles/step_kernel_k3_3inst_444tiles_ncu_counters.md), scaled here by the tiles per launch
+            "traffic": 0.94 * row_bytes,
+            "hbm": {"algorithmic_bytes_per_launch": row_bytes, "achieved_GBps": row_bytes / (avg_kernel_ms * 1e-3) / 1e9,
+                    "peak_GBps": peaks.get("hbm_gbs"), "note": "path metrics of every third step (K = 3)"},
         }
         cpu = None
         if world == 1 and not args.no_cpu_baseline:
@@ -537,7 +538,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
                        + ("" if (K_BITS, CODEBOOK) == (3, "3inst") else f" -- SIDE MEASUREMENT at K={K_BITS}, {CODEBOOK}"),
                        "K": K_BITS, "codebook": CODEBOOK, "tiles_per_gpu": n,
                        "parallelism": f"{world} x whole matrices, NCCL all-gather of packed codes" if world > 1 else "1 GPU",
-                       "l2": "each step streams 2.7 GiB of backpointer scratch, far more than the 126 MB L2, so nothing "
+                       "l2": "each step streams 2.5 GB of metric-row scratch many times over, far more than the 126 MB L2, so nothing "
                              "survives between steps; the 64 MiB of tiles are re-read from HBM"},
             "e2e": {"value": total_weights / (e2e_ms * 1e-3), "unit": "weights/s", "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms / args.steps},
@@ -825,7 +826,7 @@ def run_ip(args) -> None:
         torch.cuda.synchronize()
     err = float((out - w).norm() / w.norm())
     hbm = measured_peaks().get("hbm_gbs") or 6650.0
-    gbs_f, gbs_i = n * k * 20 / (ms_f * 1e-3) / 1e9, n * k * 16 / (ms_i * 1e-3) / 1e9
+    gbs_f, gbs_i = n * k * 16 / (ms_f * 1e-3) / 1e9, n * k * 8 / (ms_i * 1e-3) / 1e9
     print(json.dumps({
         "metric": "weights incoherence-processed/sec (forward)", "value": n * k / (ms_f * 1e-3), "unit": "weights/s", "n_gpus": 1,
         "steps": args.steps, "warmup": max(args.warmup, 3), "ms_per_step": ms_f, "higher_is_better": True, "scaling": "weak",
@@ -833,8 +834,8 @@ def run_ip(args) -> None:
         "config": {"workload": f"SIDE MEASUREMENT: incoherence processing of a [{n}, {k}] fp32 matrix ({n * k * 4 / 2 ** 20:.0f} MiB, larger "
                                "than L2) through tcq_ip_forward / tcq_ip_restore, buffers preallocated", "n": n, "k": k},
         "restore": {"ms_per_step": ms_i, "weights_per_s": n * k / (ms_i * 1e-3), "round_trip_rel_err": err},
-        "gpu_launches": 5 * args.steps,
-        "roofline": {"bound": "hbm", "kernel": "ip_row_sumsq + ip_had_rows + ip_had_cols (forward, 5 launches)", "achieved": gbs_f,
+        "gpu_launches": 4 * args.steps,
+        "roofline": {"bound": "hbm", "kernel": "ip_row_rms + ip_col_sumsq + ip_finish_cols + ip_block (forward, 4 launches: 3 reads, 1 write)", "achieved": gbs_f,
                      "peak": hbm, "unit": "GB/s", "frac": gbs_f / hbm, "traffic": None,
                      "restore": {"achieved": gbs_i, "frac": gbs_i / hbm}},
         "clocks": clocks.summary()}), flush=True)
