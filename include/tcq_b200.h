@@ -192,7 +192,8 @@ TCQ_API int tcq_selftest_wait_timeout(const float *w, int64_t n_tiles, int K, vo
 /*
  * Number of kernel launches tcq_encode_tb issues for n_tiles with a workspace of
  * ws_bytes (four per chunk: step kernel and traceback for each of the two passes;
- * six or twelve where the workspace holds a half or a quarter of a path only),
+ * six or twelve where the workspace holds a half or a quarter of a path only, and
+ * half as many again where a sweep is two launches of different shape),
  * or a negative TCQ_E_* code.  No reference counterpart; used for accounting.
  */
 TCQ_API int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes);

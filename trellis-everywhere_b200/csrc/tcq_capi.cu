@@ -70,28 +70,47 @@ constexpr ClusterShape kShapes2[] = {{16, 1, 100}, {8, 1, 124}, {8, 2, 175}, {4,
 constexpr ClusterShape kShapes3[] = {{8, 1, 107}, {8, 2, 150}, {4, 1, 152}, {4, 2, 205}, {2, 1, 223}, {2, 2, 337}, {2, 3, 460}, {2, 4, 558}, {2, 5, 690}, {2, 6, 804}};
 constexpr ClusterShape kShapes4[] = {{8, 1, 105}, {8, 2, 150}, {4, 1, 142}, {4, 2, 213}, {2, 1, 205}, {2, 2, 338}, {2, 3, 447}, {2, 4, 548}, {2, 5, 680}, {2, 6, 804}};
 
-// The shape that finishes n tiles soonest, counting whole rounds; *us its time for one pass.  (Clusters of 4, 8 and 16 leave SMs of
-// some GPCs over: 33, 15 and 7 of them run at once on a B200's 148 SMs.)
-// TCQ_FORWARD_KERNEL = cluster2 | cluster4 | cluster8 | cluster16 fixes the cluster size, for comparison runs.
-ClusterShape pick_cluster(long long n, int K, double* us) {
+// The shape that finishes n tiles soonest, counting whole rounds.  (Clusters of 4, 8 and 16 leave SMs of
+// some GPCs over: 33, 15 and 7 of them run at once on a B200's 148 SMs.)  only: this cluster size (0: any).
+struct Sweep { ClusterShape shape; double us; };
+Sweep pick_cluster(long long n, int K, int only) {
     const ClusterShape* s = K == 2 ? kShapes2 : K == 3 ? kShapes3 : kShapes4;
     const int ns = int(K == 2 ? std::size(kShapes2) : K == 3 ? std::size(kShapes3) : std::size(kShapes4));
-    const char* v = std::getenv("TCQ_FORWARD_KERNEL");
-    const int only = v != nullptr && std::strncmp(v, "cluster", 7) == 0 ? std::atoi(v + 7) : 0;
-    ClusterShape best{2, 2, 0};
-    double best_t = 1e300;
+    Sweep best{{2, 2, 0}, 1e300};
     for (int i = 0; i < ns; ++i) {
-        if (only != 0 && s[i].C != only) continue;
-        const long long at_once = clusters_at_once(s[i].C);
+        const long long at_once = only != 0 && s[i].C != only ? 0 : clusters_at_once(s[i].C);
         if (at_once < 1) continue;
         const long long groups = (n + s[i].G - 1) / s[i].G, rounds = (groups + at_once - 1) / at_once;
-        if (double(rounds) * s[i].us < best_t) {
-            best_t = double(rounds) * s[i].us;
-            best = s[i];
-        }
+        if (double(rounds) * s[i].us < best.us) best = Sweep{s[i], double(rounds) * s[i].us};
     }
-    if (us != nullptr) *us = best_t;
     return best;
+}
+
+// A sweep as one launch, or as two: whole rounds of one shape and what is left in another, both with two SMs per cluster (the
+// walk reads as many partial minima for every tile).  One shape for all of 768 tiles takes two rounds of six tiles, the second
+// three quarters empty: 3394 us a call at K = 3, 3203 with a round of six and one of five; 500 tiles 2466 -> 2222 us, 300 at K = 2
+// 2282 -> 1991.  5 us: a launch.  Only where it promises 4 %: the table is not better than that (256 tiles at K = 2, where it
+// promises 2 %, took 3 % longer).
+// TCQ_FORWARD_KERNEL = cluster2 | cluster4 | cluster8 | cluster16 fixes the cluster size, for comparison runs.
+struct SweepPlan { ClusterShape first, second; long long n_first; double us; };
+SweepPlan plan_sweep(long long n, int K) {
+    const char* v = std::getenv("TCQ_FORWARD_KERNEL");
+    const int only = v != nullptr && std::strncmp(v, "cluster", 7) == 0 ? std::atoi(v + 7) : 0;
+    const Sweep one = pick_cluster(n, K, only);
+    const SweepPlan whole{one.shape, one.shape, n, one.us};
+    if (only != 0 && only != 2) return whole;
+    SweepPlan best = whole;
+    best.us *= 0.96;
+    const ClusterShape* s = K == 2 ? kShapes2 : K == 3 ? kShapes3 : kShapes4;
+    const int ns = int(K == 2 ? std::size(kShapes2) : K == 3 ? std::size(kShapes3) : std::size(kShapes4));
+    for (int i = 0; i < ns; ++i) {
+        const long long round = s[i].C == 2 ? (long long)clusters_at_once(2) * s[i].G : 0;
+        if (round < 1 || n <= round || n % round == 0) continue;
+        const Sweep rest = pick_cluster(n % round, K, 2);
+        const double us = double(n / round) * s[i].us + rest.us + 5.0;
+        if (us < best.us) best = SweepPlan{s[i], rest.shape, n / round * round, us};
+    }
+    return best.n_first < n ? best : whole;
 }
 
 size_t rowb(int K) { return (size_t(1) << (kL - K)) * size_t(K) / 8; }
@@ -176,9 +195,7 @@ void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chun
         if (c < 1) continue;
         const bool all = c >= want;
         if (!all) c = (n + (n + c - 1) / c - 1) / ((n + c - 1) / c);        // as many chunks, of equal size
-        double us = 0.0, rest = 0.0;
-        pick_cluster(c, K, &us);
-        if (n % c != 0) pick_cluster(n % c, K, &rest);
+        const double us = plan_sweep(c, K).us, rest = n % c != 0 ? plan_sweep(n % c, K).us : 0.0;
         const double total = (double(n / c) * us + rest) * swept_steps(p) / 256.0 + double((n + c - 1) / c) * (80.0 + 40.0 * (256 / p - 1));
         if (total < best) {
             best = total;
@@ -233,18 +250,33 @@ cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& 
     t->e_start = a.overlap != nullptr ? a.overlap : wk.e_final;
     t->keys = nullptr;
     if (wk.clustered) {
-        const ClusterShape shape = pick_cluster(a.n, K, nullptr);
+        const SweepPlan plan = plan_sweep(a.n, K);
         ClusterArgs ca{a, wk.rows, rows_for(K, a.bp_steps), a.overlap == nullptr && a.steps == kT ? wk.keys : nullptr, nullptr};
         t->rows = wk.rows;
         t->nrows = ca.nrows;
         t->keys = ca.keys;
-        t->nkeys = shape.C;
-        switch (K) {
-            case 2: return launch_forward_cluster<2>(codebook, ca, shape.C, shape.G, s);
-            case 3: return launch_forward_cluster<3>(codebook, ca, shape.C, shape.G, s);
-            case 4: return launch_forward_cluster<4>(codebook, ca, shape.C, shape.G, s);
-            default: return cudaErrorInvalidValue;
-        }
+        t->nkeys = plan.first.C;
+        auto launch = [&](const ClusterShape& shape) -> cudaError_t {
+            switch (K) {
+                case 2: return launch_forward_cluster<2>(codebook, ca, shape.C, shape.G, s);
+                case 3: return launch_forward_cluster<3>(codebook, ca, shape.C, shape.G, s);
+                case 4: return launch_forward_cluster<4>(codebook, ca, shape.C, shape.G, s);
+                default: return cudaErrorInvalidValue;
+            }
+        };
+        ca.f.n = plan.n_first;
+        cudaError_t err = launch(plan.first);
+        if (err != cudaSuccess || plan.n_first == a.n) return err;
+        const long long at = plan.n_first, tile_step = a.ld > 0 ? 16 : kT;
+        ca.f.n = a.n - at;
+        ca.f.w += at * tile_step;
+        if (ca.f.w_add != nullptr) ca.f.w_add += at * tile_step;
+        if (ca.f.overlap != nullptr) ca.f.overlap += at;
+        if (ca.f.final_cost != nullptr) ca.f.final_cost += at;
+        ca.f.flags &= ~kFwdResetStatus;            // the first launch has cleared the status word
+        ca.rows += size_t(at) * ca.nrows * (size_t(1) << (kL - K));
+        if (ca.keys != nullptr) ca.keys += at * plan.first.C;
+        return launch(plan.second);
     }
     t->bp = wk.bp;
     switch (K) {
@@ -277,8 +309,11 @@ int pass(int K, int codebook, ForwardArgs f, int walk, TracebackArgs out, const 
     return TCQ_OK;
 }
 
-// Launches of an encode per chunk: a sweep and a walk for each part of the two passes.
-int launches_per_chunk(int part) { return 2 * ((part >= 128 ? 1 : 2) + 256 / part); }
+// Launches of an encode for a chunk of n tiles: a sweep (of one or two launches) and a walk for each part of the two passes.
+int launches_of_chunk(long long n, int K, const Workspace& wk) {
+    const int parts = (wk.part >= 128 ? 1 : 2) + 256 / wk.part;
+    return parts * (wk.clustered && plan_sweep(n, K).n_first < n ? 3 : 2);
+}
 
 int check_common(int K, int codebook, long long n) {
     if (K < 2 || K > 4) return TCQ_E_BAD_K;
@@ -537,7 +572,8 @@ int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes) {
     Workspace wk;
     alignas(256) static unsigned char dummy[256];          // carve() only does pointer arithmetic on it
     if ((rc = carve(dummy, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
-    return launches_per_chunk(wk.clustered ? wk.part : kT) * ((n_tiles + wk.chunk - 1) / wk.chunk);
+    const int64_t whole = n_tiles / wk.chunk, rest = n_tiles % wk.chunk;
+    return whole * launches_of_chunk(wk.chunk, K, wk) + (rest > 0 ? launches_of_chunk(rest, K, wk) : 0);
 }
 
 int tcq_decode_packed(const uint32_t* packed, int64_t n_tiles, int K, int codebook, float* dq, void* stream) {

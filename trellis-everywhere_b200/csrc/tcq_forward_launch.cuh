@@ -3,8 +3,6 @@
 // so that the large kernels compile in parallel.
 #pragma once
 
-#include <cstdlib>
-#include <cstring>
 
 #include "tcq_forward_cluster.cuh"
 
