@@ -1,0 +1,67 @@
+// The encoder's host side on a made-up CUDA runtime, so that what it launches can be looked at without a GPU: the real argument
+// checks, scratch plans and cluster queries (tcq_capi.cu, tcq_forward_launch.cuh) over the entry points of
+// launch_plan_runtime.cpp.  Built and run by test_launch_plan.py.  Arguments, in order:
+//   fail N             the next N occupancy queries fail
+//   encode K N BYTES   tcq_encode_tb of N tiles with BYTES of scratch (0: what tcq_workspace_bytes says)
+// Each launch and each call's status is printed on a line.
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+
+#include "../trellis-everywhere_b200/csrc/tcq_forward_launch.cuh"
+#include "../trellis-everywhere_b200/csrc/tcq_traceback.cuh"
+
+extern int g_failing_queries;
+
+namespace tcq {
+
+static cudaError_t cluster(int K, const ClusterArgs& ca, int C, int G) {
+    // queries go through the real launcher (of the size with the smallest kernel for all but one)
+    if (ca.f.n <= 0) return C == 16 ? launch_cluster_variant<2, kCbMcg, 16, 1, 0, 256>(ca, nullptr) : C == 8 ? launch_cluster_variant<2, kCbMcg, 8, 1, 0, 512>(ca, nullptr)
+                          : C == 4 ? launch_cluster_variant<2, kCbMcg, 4, 1, 0, 512>(ca, nullptr) : launch_cluster_variant<2, kCbMcg, 2, 1, 0, 512>(ca, nullptr);
+    std::printf("cluster K=%d C=%d G=%d n=%lld\n", K, C, G, ca.f.n);
+    return cudaSuccess;
+}
+static cudaError_t cta(int K, const ForwardArgs& a) {
+    std::printf("cta K=%d n=%lld\n", K, a.n);
+    return cudaSuccess;
+}
+template <> cudaError_t launch_forward_cluster<2>(int, const ClusterArgs& ca, int C, int G, cudaStream_t) { return cluster(2, ca, C, G); }
+template <> cudaError_t launch_forward_cluster<3>(int, const ClusterArgs& ca, int C, int G, cudaStream_t) { return cluster(3, ca, C, G); }
+template <> cudaError_t launch_forward_cluster<4>(int, const ClusterArgs& ca, int C, int G, cudaStream_t) { return cluster(4, ca, C, G); }
+template <> cudaError_t launch_forward_cta<2>(int, const ForwardArgs& a, int, cudaStream_t) { return cta(2, a); }
+template <> cudaError_t launch_forward_cta<3>(int, const ForwardArgs& a, int, cudaStream_t) { return cta(3, a); }
+template <> cudaError_t launch_forward_cta<4>(int, const ForwardArgs& a, int, cudaStream_t) { return cta(4, a); }
+cudaError_t launch_traceback(int, const TracebackArgs& a, cudaStream_t) {
+    std::printf("walk %s n=%lld keys=%d\n", a.rows != nullptr ? "rows" : "backpointers", a.n, a.keys != nullptr ? a.nkeys : 0);
+    return cudaSuccess;
+}
+cudaError_t launch_decode_packed(const uint32_t*, long long, int, int, float*, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t launch_decode_matvec(const uint32_t*, long long, long long, int, int, const float*, long long, int, float*, long long, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t launch_decode_symbols(const long long*, long long, long long, int, int, const long long*, float*, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t launch_pack_symbols(const long long*, long long, int, uint32_t*, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t launch_codebook_lut(int, float*, cudaStream_t) { return cudaErrorUnknown; }
+size_t ip_workspace_bytes(long long, long long) { return 0; }
+cudaError_t launch_ip_forward(const float*, long long, long long, const float*, const float*, float, int, float*, float*, float*, float*, void*, cudaStream_t) { return cudaErrorUnknown; }
+cudaError_t launch_ip_restore(const float*, int, long long, long long, const float*, const float*, const float*, const float*, const float*, float*, void*, cudaStream_t) { return cudaErrorUnknown; }
+
+}  // namespace tcq
+
+#include "../trellis-everywhere_b200/csrc/tcq_capi.cu"
+
+int main(int argc, char** argv) {
+    auto address = [](uintptr_t a) { return reinterpret_cast<void*>(a); };          // aligned and never read
+    for (int i = 1; i < argc;) {
+        if (!std::strcmp(argv[i], "fail")) {
+            g_failing_queries = std::atoi(argv[i + 1]);
+            i += 2;
+        } else {
+            const int K = std::atoi(argv[i + 1]);
+            const long long n = std::atoll(argv[i + 2]), bytes = std::atoll(argv[i + 3]);
+            std::printf("status %d\n", tcq_encode_tb(static_cast<float*>(address(1 << 20)), n, K, 2, static_cast<uint32_t*>(address(1 << 21)), nullptr, nullptr,
+                                                     nullptr, address(1 << 22), bytes > 0 ? size_t(bytes) : tcq_workspace_bytes(n, K), nullptr));
+            i += 4;
+        }
+    }
+    return 0;
+}

@@ -46,11 +46,13 @@ int clusters_at_once(int C) {
     int n = cached ? cache[dev][C] : 0;
     if (n == 0) {
         ClusterArgs ca{};                          // no tiles: a query.  One CTA fits an SM whatever K and the tiles per group are.
-        ca.at_once = &n;
-        const cudaError_t err = launch_forward_cluster<2>(kCbMcg, ca, C, 1, nullptr);
-        if (err != cudaSuccess) (void)cudaGetLastError();
-        if (err == cudaErrorNotSupported) n = -1;
-        if (cached) cache[dev][C] = n;             // a failed query leaves 0: it says nothing about the device
+        ca.query = &n;
+        if (launch_forward_cluster<2>(kCbMcg, ca, C, 1, nullptr) != cudaSuccess) {
+            (void)cudaGetLastError();              // a failed query says nothing about the device: the next call asks again
+            return 0;
+        }
+        if (n < 1) n = -1;
+        if (cached) cache[dev][C] = n;
     }
     return n > 0 ? n : 0;
 }
@@ -251,12 +253,14 @@ cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& 
     t->keys = nullptr;
     if (wk.clustered) {
         const SweepPlan plan = plan_sweep(a.n, K);
-        ClusterArgs ca{a, wk.rows, rows_for(K, a.bp_steps), a.overlap == nullptr && a.steps == kT ? wk.keys : nullptr, nullptr};
+        ClusterArgs ca{a, wk.rows, rows_for(K, a.bp_steps), a.overlap == nullptr && a.steps == kT ? wk.keys : nullptr, 0, nullptr};
         t->rows = wk.rows;
         t->nrows = ca.nrows;
         t->keys = ca.keys;
         t->nkeys = plan.first.C;
         auto launch = [&](const ClusterShape& shape) -> cudaError_t {
+            ca.at_once = clusters_at_once(shape.C);
+            if (ca.at_once < 1) return cudaErrorNotSupported;
             switch (K) {
                 case 2: return launch_forward_cluster<2>(codebook, ca, shape.C, shape.G, s);
                 case 3: return launch_forward_cluster<3>(codebook, ca, shape.C, shape.G, s);
@@ -555,7 +559,7 @@ int tcq_selftest_wait_timeout(const float* w, int64_t n_tiles, int K, void* ws, 
     if (cudaMemsetAsync(wk.status, 0, sizeof(unsigned int), s) != cudaSuccess) return cuda_fail(cudaGetLastError(), "status reset");
     // the buffers of the final metrics are told to expect 16 bytes more than the cluster will ever send
     ForwardArgs f{w, nullptr, 0, n_tiles, nullptr, 0, 0, kT, nullptr, nullptr, nullptr, 1.0f, 16, wk.status, 0};
-    ClusterArgs ca{f, nullptr, 0, nullptr, nullptr};
+    ClusterArgs ca{f, nullptr, 0, nullptr, clusters_at_once(2), nullptr};
     cudaError_t err = K == 2   ? launch_forward_cluster<2>(kCbMcg, ca, 2, 2, s)
                       : K == 3 ? launch_forward_cluster<3>(kCbMcg, ca, 2, 2, s)
                                : launch_forward_cluster<4>(kCbMcg, ca, 2, 2, s);

@@ -287,12 +287,13 @@ struct ClusterArgs {
     float* rows;                // [n][nrows][E] out: metric rows (MetricRows), the last nrows of the pass
     int nrows;
     unsigned long long* keys;   // [n][C] out: per-CTA (metric bits << 32 | edge) minima of the final metrics, or nullptr
-    int* at_once;               // host, with f.n == 0: receives how many such clusters the device runs at once
+    int at_once;                // launches: how many such clusters the device runs at once (the grid is no larger)
+    int* query;                 // host, with f.n == 0: receives that number, 0 if the device cannot schedule such a cluster
 };
 
 // Host-side launchers, implemented once per K in tcq_forward_k{2,3,4}.cu.
-// Cluster form: clusters of C CTAs that advance G tiles.  cudaErrorNotSupported (and nothing launched) if the
-// device cannot schedule such a cluster; with f.n == 0 nothing is launched: it only finds that out.
+// Cluster form: clusters of C CTAs that advance G tiles.  With f.n == 0 nothing is launched: it asks how many the device
+// runs at once, and any error is that of the question.
 template <int K>
 cudaError_t launch_forward_cluster(int codebook, const ClusterArgs& args, int C, int G, cudaStream_t stream);
 // Single-CTA form (packed argmins to args.bp): picks the tiles-per-CTA variant.

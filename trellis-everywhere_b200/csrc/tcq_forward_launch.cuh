@@ -46,8 +46,8 @@ static cudaError_t launch_variant(const ForwardArgs& a, int num_sms, cudaStream_
 
 constexpr size_t kOneCtaPerSm = 116 * 1024;        // dynamic shared memory of which an SM (228 KiB) holds one
 
-// Cluster form with clusters of C CTAs, tile sets of GS and LU successors per work item.  How many clusters of this
-// shape the device runs at once is asked once per device; a launch uses at most that many.
+// Cluster form with clusters of C CTAs and tile sets of GA and GB.  A launch uses at most as many clusters as the device runs at
+// once, which depends on C only (one CTA fills an SM in every instantiation) and is asked for in a call of its own.
 template <int K, int CB, int C, int GA, int GB, int NT>
 static cudaError_t launch_cluster_variant(const ClusterArgs& ca, cudaStream_t stream) {
     auto kern = tcq_forward_cluster_kernel<K, CB, C, GA, GB, NT>;
@@ -74,26 +74,10 @@ static cudaError_t launch_cluster_variant(const ClusterArgs& ca, cudaStream_t st
     cfg.stream = stream;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    static int max_clusters[kMaxDeviceOrdinals] = {0};   // per device ordinal; 0 = not known yet, -1 = cannot schedule this cluster
-    int maxc = dev >= 0 ? max_clusters[dev] : 0;
-    if (maxc == 0) {
-        int q = 0;
-        err = cudaOccupancyMaxActiveClusters(&q, kern, &cfg);
-        if (err != cudaSuccess) {
-            (void)cudaGetLastError();              // a failed query says nothing about the device: ask again next time
-            return cudaErrorNotSupported;
-        }
-        maxc = q > 0 ? q : -1;
-        if (dev >= 0) max_clusters[dev] = maxc;    // cached only when the query itself succeeded
-    }
-    if (maxc < 0) return cudaErrorNotSupported;
-    if (ca.f.n <= 0) {                             // a query only
-        if (ca.at_once != nullptr) *ca.at_once = maxc;
-        return cudaSuccess;
-    }
+    if (ca.f.n <= 0) return cudaOccupancyMaxActiveClusters(ca.query, kern, &cfg);
     constexpr int G = GA + GB;
     const long long ngroups = (ca.f.n + G - 1) / G;
-    const long long ncl = ngroups < maxc ? ngroups : maxc;
+    const long long ncl = ngroups < ca.at_once ? ngroups : ca.at_once;
     cfg.gridDim = dim3(unsigned(ncl * C));
     return cudaLaunchKernelEx(&cfg, kern, ca);
 }
