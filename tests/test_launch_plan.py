@@ -28,3 +28,16 @@ def test_a_failed_query_is_asked_again(plan):
         calls = " ".join(lines).split("status 0")
         assert len(calls) == fails + 2
         assert "cluster" in calls[fails] and "cta" not in calls[fails]
+
+
+def test_a_cluster_size_that_a_rate_has_not_is_refused(plan):
+    """TCQ_FORWARD_KERNEL fixes the cluster size for comparison runs: what it names runs or the call is refused, and text that
+    names nothing is no request."""
+    for K, C in ((2, 2), (2, 8), (2, 16), (3, 2), (3, 4), (3, 8), (4, 2), (4, 4), (4, 8)):
+        lines = plan("encode", K, 5, 0, TCQ_FORWARD_KERNEL=f"cluster{C}")
+        assert lines[-1] == "status 0" and all(f" C={C} " in x for x in lines if x.startswith("c"))
+    for K in (3, 4):
+        assert plan("encode", K, 5, 0, TCQ_FORWARD_KERNEL="cluster16") == ["status -8"]
+    for text in ("cluster3", "cluster", "warp"):
+        assert plan("encode", 3, 5, 0, TCQ_FORWARD_KERNEL=text) == plan("encode", 3, 5, 0)
+    assert any(x.startswith("cta") for x in plan("encode", 3, 5, 0, TCQ_FORWARD_KERNEL="cta"))

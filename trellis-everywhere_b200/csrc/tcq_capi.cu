@@ -3,6 +3,7 @@
 // memory is allocated or freed here and nothing synchronises with the host.
 #include "../../include/tcq_b200.h"
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -57,11 +58,19 @@ int clusters_at_once(int C) {
     return n > 0 ? n : 0;
 }
 
-// Whether the cluster step kernel runs on the current device (TCQ_FORWARD_KERNEL=cta: the single-CTA form is asked for).
-bool cluster_available() {
+// TCQ_FORWARD_KERNEL = cta | cluster2 | cluster4 | cluster8 | cluster16, for comparison runs: the cluster size it asks for, 1 for the
+// single-CTA kernel, 0 if it is not set or names none of them.
+int kernel_asked_for() {
     const char* v = std::getenv("TCQ_FORWARD_KERNEL");
-    return !(v != nullptr && std::strcmp(v, "cta") == 0) && clusters_at_once(2) > 0;
+    if (v == nullptr) return 0;
+    if (std::strcmp(v, "cta") == 0) return 1;
+    for (const char* name : {"cluster2", "cluster4", "cluster8", "cluster16"})
+        if (std::strcmp(v, name) == 0) return std::atoi(name + 7);
+    return 0;
 }
+
+// Whether the cluster step kernel runs on the current device.
+bool cluster_available() { return kernel_asked_for() != 1 && clusters_at_once(2) > 0; }
 
 // How a batch is spread over the chip: clusters of C CTAs, G tiles each, and the time of one round of a 256-step sweep with
 // all SMs of a B200 at work, measured.  A larger cluster divides a tile's step over more SMs, which shortens the step for
@@ -72,12 +81,20 @@ constexpr ClusterShape kShapes2[] = {{16, 1, 100}, {8, 1, 120}, {8, 2, 156}, {4,
 constexpr ClusterShape kShapes3[] = {{8, 1, 107}, {8, 2, 150}, {4, 1, 152}, {4, 2, 205}, {2, 1, 223}, {2, 2, 337}, {2, 3, 460}, {2, 4, 558}, {2, 5, 690}, {2, 6, 804}};
 constexpr ClusterShape kShapes4[] = {{8, 1, 105}, {8, 2, 150}, {4, 1, 142}, {4, 2, 213}, {2, 1, 205}, {2, 2, 338}, {2, 3, 447}, {2, 4, 548}, {2, 5, 680}, {2, 6, 804}};
 
+struct ShapeList { const ClusterShape* s; int n; };
+ShapeList shapes(int K) {
+    return K == 2 ? ShapeList{kShapes2, int(std::size(kShapes2))} : K == 3 ? ShapeList{kShapes3, int(std::size(kShapes3))} : ShapeList{kShapes4, int(std::size(kShapes4))};
+}
+bool has_cluster_size(int K, int C) {
+    const ShapeList l = shapes(K);
+    return std::any_of(l.s, l.s + l.n, [C](const ClusterShape& x) { return x.C == C; });
+}
+
 // The shape that finishes n tiles soonest, counting whole rounds.  (Clusters of 4, 8 and 16 leave SMs of
 // some GPCs over: 33, 15 and 7 of them run at once on a B200's 148 SMs.)  only: this cluster size (0: any).
 struct Sweep { ClusterShape shape; double us; };
 Sweep pick_cluster(long long n, int K, int only) {
-    const ClusterShape* s = K == 2 ? kShapes2 : K == 3 ? kShapes3 : kShapes4;
-    const int ns = int(K == 2 ? std::size(kShapes2) : K == 3 ? std::size(kShapes3) : std::size(kShapes4));
+    const auto [s, ns] = shapes(K);
     Sweep best{{2, 2, 0}, 1e300};
     for (int i = 0; i < ns; ++i) {
         const long long at_once = only != 0 && s[i].C != only ? 0 : clusters_at_once(s[i].C);
@@ -93,18 +110,15 @@ Sweep pick_cluster(long long n, int K, int only) {
 // three quarters empty: 3394 us a call at K = 3, 3203 with a round of six and one of five; 500 tiles 2466 -> 2222 us, 300 at K = 2
 // 2282 -> 1991.  5 us: a launch.  Only where it promises 4 %: the table is not better than that (256 tiles at K = 2, where it
 // promises 2 %, took 3 % longer).
-// TCQ_FORWARD_KERNEL = cluster2 | cluster4 | cluster8 | cluster16 fixes the cluster size, for comparison runs.
 struct SweepPlan { ClusterShape first, second; long long n_first; double us; };
 SweepPlan plan_sweep(long long n, int K) {
-    const char* v = std::getenv("TCQ_FORWARD_KERNEL");
-    const int only = v != nullptr && std::strncmp(v, "cluster", 7) == 0 ? std::atoi(v + 7) : 0;
+    const int asked = kernel_asked_for(), only = asked > 1 ? asked : 0;
     const Sweep one = pick_cluster(n, K, only);
     const SweepPlan whole{one.shape, one.shape, n, one.us};
     if (only != 0 && only != 2) return whole;
     SweepPlan best = whole;
     best.us *= 0.96;
-    const ClusterShape* s = K == 2 ? kShapes2 : K == 3 ? kShapes3 : kShapes4;
-    const int ns = int(K == 2 ? std::size(kShapes2) : K == 3 ? std::size(kShapes3) : std::size(kShapes4));
+    const auto [s, ns] = shapes(K);
     for (int i = 0; i < ns; ++i) {
         const long long round = s[i].C == 2 ? (long long)clusters_at_once(2) * s[i].G : 0;
         if (round < 1 || n <= round || n % round == 0) continue;
@@ -211,6 +225,7 @@ void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chun
 int carve(void* ws, size_t ws_bytes, long long n, int K, int num_sms, Workspace* out) {
     if (ws == nullptr) return TCQ_E_NULL_POINTER;
     if (reinterpret_cast<uintptr_t>(ws) % kAlign) return TCQ_E_MISALIGNED;
+    if (kernel_asked_for() > 1 && !has_cluster_size(K, kernel_asked_for())) return TCQ_E_BAD_ARGUMENT;
     *out = Workspace{};
     out->chunk = bp_chunk_for(n, ws_bytes, K, num_sms);
     if (out->chunk < 1) return TCQ_E_WORKSPACE;
