@@ -3,7 +3,8 @@
 // launch_plan_runtime.cpp.  Built and run by test_launch_plan.py.  Arguments, in order:
 //   fail N             the next N occupancy queries fail
 //   encode K N BYTES   tcq_encode_tb of N tiles with BYTES of scratch (0: what tcq_workspace_bytes says)
-// Each launch and each call's status is printed on a line.
+//   shapes K           the shapes that a launch may have
+// Each launch, each call's status and each shape is printed on a line.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -54,6 +55,10 @@ int main(int argc, char** argv) {
     for (int i = 1; i < argc;) {
         if (!std::strcmp(argv[i], "fail")) {
             g_failing_queries = std::atoi(argv[i + 1]);
+            i += 2;
+        } else if (!std::strcmp(argv[i], "shapes")) {
+            const auto [s, n] = shapes(std::atoi(argv[i + 1]));
+            for (int j = 0; j < n; ++j) std::printf("C=%d G=%d\n", s[j].C, s[j].G);
             i += 2;
         } else {
             const int K = std::atoi(argv[i + 1]);

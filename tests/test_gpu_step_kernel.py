@@ -21,10 +21,12 @@ def _np(t):
     return t.detach().cpu().numpy()
 
 
-# one tile, and both sides of every batch size at which another shape (SMs per cluster x tiles per cluster) takes over; the last of
-# each K go as two launches: whole rounds of one shape and the rest in another
-SIZES = {2: (1, 7, 9, 16, 17, 33, 67, 74, 75, 149, 223, 299, 671), 3: (1, 16, 17, 32, 33, 66, 67, 75, 149, 223, 297, 371, 443, 445, 768),
-         4: (1, 15, 17, 33, 67, 75, 149, 223, 297, 371, 445, 521)}
+# one tile, and both sides of every batch size up to two rounds of the largest shape at which another shape (SMs per cluster x tiles
+# per cluster) takes over (test_launch_plan.py holds them against the plan); some go as two launches, whole rounds of one shape and the
+# rest in another
+_ROUNDS = tuple(m for k in range(1, 12) for m in (74 * k, 74 * k + 1))
+SIZES = {2: (1, 7, 8, 9, 15, 16, 17, 30, 31, 33, 34, 67, 299, 671, 888) + _ROUNDS, 3: (1, 15, 16, 17, 30, 31, 32, 33, 34, 66, 67, 443, 768, 888) + _ROUNDS,
+         4: (1, 15, 16, 17, 33, 34, 67, 521, 888) + _ROUNDS}
 
 
 @pytest.mark.parametrize("K,n", [(K, n) for K in KS for n in SIZES[K]])

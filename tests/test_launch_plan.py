@@ -1,10 +1,12 @@
 """What the encoder launches, and for which batch: its host code on a made-up CUDA runtime (launch_plan.cu), no GPU needed."""
 import os
+import re
 import subprocess
 
 import pytest
 
-from conftest import ROOT
+from conftest import KS, ROOT
+from test_gpu_step_kernel import SIZES
 
 
 @pytest.fixture(scope="module")
@@ -41,3 +43,15 @@ def test_a_cluster_size_that_a_rate_has_not_is_refused(plan):
     for text in ("cluster3", "cluster", "warp"):
         assert plan("encode", 3, 5, 0, TCQ_FORWARD_KERNEL=text) == plan("encode", 3, 5, 0)
     assert any(x.startswith("cta") for x in plan("encode", 3, 5, 0, TCQ_FORWARD_KERNEL="cta"))
+
+
+@pytest.mark.parametrize("K", KS)
+def test_every_shape_is_some_batch_s_and_every_switch_is_tested(plan, K):
+    """No shape is compiled that no batch takes, and the sizes of the GPU test hold both sides of every size at which another
+    shape, or another pair of shapes, takes over (up to two rounds of the largest, the tiles of one chunk)."""
+    lines = plan(*(x for n in range(1, 889) for x in ("encode", K, n, 0)))
+    calls = "\n".join(lines).split("status 0")[:-1]
+    taken = [tuple(re.findall(r"C=\d+ G=\d+", c)) for c in calls]
+    assert {s for t in taken for s in t} == set(plan("shapes", K))
+    switches = [n for n in range(2, 889) if taken[n - 1] != taken[n - 2]]
+    assert len(switches) >= 10 and {n - 1 for n in switches} | set(switches) <= set(SIZES[K])
