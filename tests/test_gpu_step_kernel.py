@@ -79,6 +79,29 @@ def test_workspaces_of_every_size_give_the_same_codes(q, K):
     assert lib.tcq_encode_tb(w.data_ptr(), n, K, 1, packed.data_ptr(), None, None, None, small.data_ptr(), per_tile - 1, stream) == -6
 
 
+def test_a_nearly_full_device_encodes_with_less_scratch(q):
+    """768 tiles at K = 3 ask for 2.1 GB of scratch; where 1.2 GB are left the call runs on less, with the same results and status."""
+    n, K = 768, 3
+    w = torch.randn(n, 256, generator=torch.Generator().manual_seed(3)).cuda()
+    want = q.encode(w, K, "mcg")
+    q.release_workspaces()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 1.2e9) / total)
+    try:
+        got = q.encode(w, K, "mcg")
+        q.workspace_status(n, K)
+        w[5, 5] = float("nan")
+        q.encode(w, K, "mcg")
+        with pytest.raises(q._lib.TcqError, match="NaN"):
+            q.workspace_status(n, K)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        q.release_workspaces()
+    assert all(torch.equal(a, b) for a, b in zip(got[:3], want[:3]))
+
+
 @pytest.mark.parametrize("K", KS)
 @pytest.mark.parametrize("name", ("1mad", "3inst", "mcg"))
 def test_ties_and_numbers_that_are_none(q, K, name, monkeypatch):

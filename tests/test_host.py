@@ -77,6 +77,30 @@ def test_encode_rejects_bad_shapes_before_touching_the_device():
         qtip.pack_bits(torch.zeros(2, 100, dtype=torch.long), 3)
 
 
+def test_scratch_of_a_device_that_is_nearly_full(monkeypatch):
+    """Where the full-speed scratch does not fit, a call takes the smaller one that the library accepts, and keeps it."""
+    L, dev, asked, empty = _lib.lib(), torch.device("cpu"), [], torch.empty
+    full, small = L.tcq_workspace_bytes(768, 3), 768 * L.tcq_workspace_min_bytes(3)
+    limit = 10 ** 9
+
+    def scarce(size, **kw):
+        asked.append(size)
+        if size > limit:
+            raise torch.OutOfMemoryError("made up")
+        return empty(1, **kw).expand(size)
+
+    monkeypatch.setattr(torch, "empty", scarce)
+    monkeypatch.setattr(qtip, "_stream", lambda dev: 0)
+    monkeypatch.setattr(qtip, "_workspaces", {})
+    ws = qtip._workspace(dev, 768, 3)
+    assert asked == [full, small] and ws.numel() == small < full
+    assert qtip._workspace(dev, 768, 3) is ws and qtip._workspace(dev, 256, 3) is ws and len(asked) == 2
+    assert qtip._workspace(dev, 700, 2).numel() == 700 * L.tcq_workspace_min_bytes(2)       # more than that block is good for
+    limit = 10 ** 5
+    with pytest.raises(torch.OutOfMemoryError):
+        qtip._workspace(dev, 900, 3)
+
+
 def test_tiling_matches_reference_index_map():
     # qtip.py:288 / :303: tile = (row/16)*(k/16) + col/16, t = (row%16)*16 + col%16
     n, k = 32, 48

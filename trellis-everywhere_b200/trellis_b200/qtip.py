@@ -82,7 +82,7 @@ def _to_dev(t: torch.Tensor, dev: torch.device, dtype: torch.dtype) -> torch.Ten
     return t.to(dev, non_blocking=True)
 
 
-_workspaces: dict = {}
+_workspaces: dict = {}          # (device, stream) -> (bytes asked for, block)
 _workspaces_lock = threading.Lock()
 
 
@@ -94,15 +94,24 @@ def _workspace(dev: torch.device, n_tiles: int, K: int) -> torch.Tensor:
     (``ldlq.ldlq_row_groups``, ``model.encode_model``) hands the block back with
     ``release_workspace`` when its stream is done, otherwise every short-lived stream would keep
     gigabytes alive.
+
+    The full-speed size is up to 4 times what the smallest plans for as many tiles need (768 tiles at K = 3: 2.1 GB, 0.6 GB).  On
+    a device too full for it a call takes the smaller size, which the library accepts with the same results, and the
+    stream's calls keep it until one needs more or it is released.
     """
     need = int(_lib.lib().tcq_workspace_bytes(n_tiles, K))
+    least = min(need, max(n_tiles, 1) * int(_lib.lib().tcq_workspace_min_bytes(K)))
     key = (dev.index, _stream(dev))
     with _workspaces_lock:
-        ws = _workspaces.get(key)
-        if ws is None or ws.numel() < need:
-            _workspaces[key] = None          # drop the old block before asking for a larger one
-            ws = torch.empty(need, dtype=torch.uint8, device=dev)
-            _workspaces[key] = ws
+        asked, ws = _workspaces.get(key, (0, None))
+        if ws is None or asked < need or ws.numel() < least:
+            _workspaces.pop(key, None)
+            ws = None                        # drop the old block before asking for a larger one
+            try:
+                ws = torch.empty(need, dtype=torch.uint8, device=dev)
+            except torch.OutOfMemoryError:
+                ws = torch.empty(least, dtype=torch.uint8, device=dev)
+            _workspaces[key] = (need, ws)
     return ws
 
 
@@ -123,7 +132,7 @@ def workspace_status(n_tiles: int, K: int, device=None) -> None:
     that call was NaN or infinite (its tile's codes are meaningless); returns None otherwise.
     """
     dev = torch.device(device) if device is not None else _cuda_device()
-    ws = _workspace(dev, n_tiles, K)
+    ws = _workspace(dev, n_tiles, K)            # the block of that call: it asked for as much
     with torch.cuda.device(dev):
         rc = _lib.lib().tcq_workspace_status(ws.data_ptr(), ws.numel(), n_tiles, K, _stream(dev))
     _lib.check(rc, "tcq_workspace_status")
