@@ -13,12 +13,10 @@
 // multiply-adds.  Partial sums (of even and odd columns) stay in registers; the two half-warps meet in one shuffle and the eight
 // warps in shared memory, in a fixed order, so results are reproducible run to run.
 //
-// Bound: instruction issue (83 % of the slots at one right-hand side), not HBM.  A weight costs about seven instructions to decode
-// (window, multiply, and/xor, two conversions, addition) and half a packed multiply-add per
-// right-hand side.  151936 x 4096, before -> now: one right-hand side K = 2 191 -> 177 us, K = 3 203 -> 193, K = 4 192 -> 170; two
-// 217 -> 205, 233 -> 221, 225 -> 205; four 322 -> 291, 318 -> 314, 327 -> 320.  Largest relative error against fp64 on a 4096 x 4096
-// matrix 2.9e-7 -> 2.1e-7 (two partial sums).  Fetching the next trip's words ahead and x in shared memory gave nothing (four right-hand sides,
-// K = 4: 342 and 314 us).
+// Bound: with many tile rows instruction issue (83 % of the slots at one right-hand side), not HBM; a weight costs about seven
+// instructions to decode (window, multiply, and/xor, two conversions, addition) and half a packed multiply-add per right-hand side.  With
+// few, the latency of a trip: words, x, products.  How the two are held is a matter of registers, which launch_m chooses by size.
+// Largest relative error against fp64 on a 4096 x 4096 matrix 2.1e-7.
 #include "tcq_traceback.cuh"
 
 namespace tcq {
@@ -27,37 +25,25 @@ namespace {
 
 constexpr int kMvWarps = 8;
 
-// The 16 weights of a tile row from its 15K+16 stream bits (v, normalised to start at bit 0), as pairs of neighbouring columns.
-// A window is cut out of a word as two bytes, in one instruction, where its offset is a whole number of bytes; words are shifted to make it
-// so, one shift for the (at most three) windows of a word that are a byte apart.  At K = 3 no two windows of a word are.
-template <int K, int CB, int WN>
-__device__ __forceinline__ void decode_row(const uint32_t (&v)[WN], f32x2 (&val)[8]) {
+// The 16-bit window of column col, out of a tile row's 15K+16 stream bits (v, normalised to start at bit 0).  Where windows of a word
+// are whole bytes apart (K = 2, 4), three of them are cut out of one shifted word, as two bytes each in one instruction.
+template <int K, int WN>
+__device__ __forceinline__ uint32_t window(const uint32_t (&v)[WN], int col) {
     auto word_at = [&](int s) { return (s & 31) == 0 ? v[s >> 5] : __funnelshift_r(v[s >> 5], (s >> 5) + 1 < WN ? v[(s >> 5) + 1] : 0u, s & 31); };
-    uint32_t win[16];
     if constexpr (K == 3) {
-#pragma unroll
-        for (int col = 0; col < 16; ++col) {
-            const int off = (15 - col) * K, s = off & 31;
-            win[col] = (s + 16 <= 32 ? v[off >> 5] >> s : word_at(off)) & 0xFFFFu;
-        }
+        const int off = (15 - col) * K, s = off & 31;
+        return (s + 16 <= 32 ? v[off >> 5] >> s : word_at(off)) & 0xFFFFu;
     } else {
-#pragma unroll
-        for (int ph = 0; ph < 8 / K; ++ph)                     // windows ph, ph + 8/K, ...: eight bits apart
-#pragma unroll
-            for (int a = 0; a < 2 * K; a += 3) {
-                const uint32_t u = word_at(K * ph + 8 * a);
-#pragma unroll
-                for (int b = 0; b < 3; ++b)
-                    if (a + b < 2 * K) win[15 - (ph + (a + b) * (8 / K))] = __byte_perm(u, 0u, 0x4400 | (b + 1) << 4 | b);
-            }
+        const int ph = (15 - col) % (8 / K), byte = (15 - col) / (8 / K), b = byte % 3;
+        return __byte_perm(word_at(K * ph + 8 * (byte - b)), 0u, 0x4400 | (b + 1) << 4 | b);
     }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) val[c] = pack2(cb_value<CB>(win[2 * c]), cb_value<CB>(win[2 * c + 1]));
 }
 
-// RT: tile rows per CTA.  Two share the loads of x, which for several right-hand sides are as many instructions as the products.
-template <int K, int CB, int M, int RT>
-__global__ void __launch_bounds__(kMvWarps * 32)
+// RT: tile rows per CTA; two share the loads of x, which for several right-hand sides are as many instructions as the products.
+// MB: CTAs that an SM must hold, i.e. the registers; x is then loaded ahead and a pair of weights lives from its decode to its products.
+// MB = 0: the compiler's choice, weights decoded first.
+template <int K, int CB, int M, int RT, int MB>
+__global__ void __launch_bounds__(kMvWarps * 32, MB)
 tcq_decode_matvec_kernel(const uint32_t* __restrict__ packed, int tiles_out, int tiles_in, const float* __restrict__ x, long long ldx,
                          int m, float* __restrict__ y, long long ldy) {
     constexpr int NW = Geo<K>::NWORDS;
@@ -90,28 +76,61 @@ tcq_decode_matvec_kernel(const uint32_t* __restrict__ packed, int tiles_out, int
                 v[t][j] = __ldg(p + (wi >= uint32_t(NW) ? wi - NW : wi));       // the first row's window wraps to word 0
             }
         }
-        f32x2 val[RT][8];
+        auto x4 = [&](int j, int q) { return __ldg(reinterpret_cast<const ulonglong2*>(x + (long long)(j < m ? j : 0) * ldx + 16 * c) + q); };
+        ulonglong2 xr[MB > 0 ? M : 1][4];
+        if constexpr (MB > 0) {
 #pragma unroll
-        for (int t = 0; t < RT; ++t) {
-            if constexpr (K == 3) {
+            for (int j = 0; j < M; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) xr[j][q] = x4(j, q);
+        }
+        if constexpr (K == 3) {
+#pragma unroll
+            for (int t = 0; t < RT; ++t) {
 #pragma unroll
                 for (int j = 0; j + 1 < WN; ++j) v[t][j] = __funnelshift_r(v[t][j], v[t][j + 1], sh);
                 v[t][WN - 1] >>= sh;
             }
-            decode_row<K, CB>(v[t], val[t]);
         }
-#pragma unroll
-        for (int j = 0; j < M; ++j) {
-            const ulonglong2* const xp = reinterpret_cast<const ulonglong2*>(x + (long long)(j < m ? j : 0) * ldx + 16 * c);
+        auto pair = [&](int t, int p) {                      // columns 2p and 2p + 1 of tile row t
+            return pack2(cb_value<CB>(window<K, WN>(v[t], 2 * p)), cb_value<CB>(window<K, WN>(v[t], 2 * p + 1)));
+        };
+        auto products = [&](int t, int j, f32x2 lo, f32x2 hi, const ulonglong2& xq) {
+            acc[t][j] = fma2(lo, xq.x, acc[t][j]);
+            acc[t][j] = fma2(hi, xq.y, acc[t][j]);
+        };
+        if constexpr (MB > 0) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const ulonglong2 x4 = __ldg(xp + q);
+                f32x2 val[RT][2];
 #pragma unroll
-                for (int t = 0; t < RT; ++t) {
-                    acc[t][j] = fma2(val[t][2 * q], x4.x, acc[t][j]);
-                    acc[t][j] = fma2(val[t][2 * q + 1], x4.y, acc[t][j]);
-                }
+                for (int t = 0; t < RT; ++t) { val[t][0] = pair(t, 2 * q); val[t][1] = pair(t, 2 * q + 1); }
+#pragma unroll
+                for (int j = 0; j < M; ++j)
+#pragma unroll
+                    for (int t = 0; t < RT; ++t) products(t, j, val[t][0], val[t][1], xr[j][q]);
             }
+        } else {
+            f32x2 val[RT][8];
+#pragma unroll
+            for (int t = 0; t < RT; ++t) {
+                uint32_t win[16];                            // in stream order, word by word
+#pragma unroll
+                for (int p = 0; p < 16; ++p) {
+                    const int col = K == 3 ? p : 15 - (p / (2 * K) + p % (2 * K) * (8 / K));
+                    win[col] = window<K, WN>(v[t], col);
+                }
+#pragma unroll
+                for (int p = 0; p < 8; ++p) val[t][p] = pack2(cb_value<CB>(win[2 * p]), cb_value<CB>(win[2 * p + 1]));
+            }
+#pragma unroll
+            for (int j = 0; j < M; ++j)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const ulonglong2 xq = x4(j, q);
+#pragma unroll
+                    for (int t = 0; t < RT; ++t) products(t, j, val[t][2 * q], val[t][2 * q + 1], xq);
+                }
         }
     }
 #pragma unroll
@@ -134,24 +153,41 @@ tcq_decode_matvec_kernel(const uint32_t* __restrict__ packed, int tiles_out, int
     }
 }
 
-template <int K, int CB, int M, int RT>
+template <int K, int CB, int M, int RT, int MB>
 void launch_mv(const uint32_t* packed, int tiles_out, int tiles_in, const float* x, long long ldx, int m, float* y, long long ldy,
                cudaStream_t stream) {
-    tcq_decode_matvec_kernel<K, CB, M, RT><<<(tiles_out + RT - 1) / RT, kMvWarps * 32, 0, stream>>>(packed, tiles_out, tiles_in, x, ldx, m, y, ldy);
+    tcq_decode_matvec_kernel<K, CB, M, RT, MB><<<(tiles_out + RT - 1) / RT, kMvWarps * 32, 0, stream>>>(packed, tiles_out, tiles_in, x, ldx, m, y, ldy);
 }
 
-// Two tile rows per CTA for four right-hand sides, where the loads of x (16 of 128 bits a tile, four passes through L1 each)
-// were the bound: from two CTAs per SM on, and at K = 2, whose decode is shortest, always.  151936 x 4096, one row -> two:
-// K = 2 318 -> 291 us, K = 3 345 -> 314, K = 4 339 -> 320; 12288 x 4096: 43 -> 27, 34 -> 39, 33 -> 36 (768 tile rows: one row there
-// at K = 3 and 4); 4096 x 4096: 18.6 -> 12.5, 16.5 -> 20.4, 16.5 -> 17.6.
-// One and two right-hand sides are bound by instruction issue and gain nothing (K = 3: 193 -> 194, 221 -> 232 us).
+// Which form, by tile rows per SM, column tiles and rate; measured at 4 to 9496 tile rows of 4 to 768 tiles, MCG.  us for rows of 256 tiles,
+// the compiler's choice of registers -> this one:
+//   one right-hand side: loads ahead (47 registers) up to two rows an SM, where the latency of a trip is the bound (K = 3, 64 rows 10.3 -> 8.3), and
+//     at K = 2, whose decode is shortest, always (9496 rows 174 -> 171).  With more rows other warps hide it, and need the registers (31; K = 4, 9496
+//     rows 168, with loads ahead 178), and so do rows too narrow to give every warp a tile (K = 2, 9496 rows of 4 tiles 10.4, 12.4).
+//   two: the compiler's choice (48), within 4 % of the best; narrow rows, which are one trip or less, want more CTAs (K = 3, 9496 rows of 4 tiles 14.4 -> 12.3).
+//   three and four: one row per CTA while all run at once, three CTAs per SM (K = 3, 64 rows 14.4 -> 10.3, 256 rows 16.4 -> 14.4), two rows from
+//     there on (K = 4, 592 rows 32.8 -> 19.2; 9496 rows K = 2 / 3 / 4 294 / 318 / 331 -> 263 / 290 / 267).  At K = 2 between one and two rows
+//     an SM two rows in one CTA, decoded first, are faster (256 rows 12.3, 13.1 with one).
 template <int K, int CB>
 cudaError_t launch_m(const uint32_t* packed, int tiles_out, int tiles_in, const float* x, long long ldx, int m, float* y,
                      long long ldy, cudaStream_t stream) {
-    if (m == 1)                            launch_mv<K, CB, 1, 1>(packed, tiles_out, tiles_in, x, ldx, m, y, ldy, stream);
-    else if (m == 2)                       launch_mv<K, CB, 2, 1>(packed, tiles_out, tiles_in, x, ldx, m, y, ldy, stream);
-    else if (K == 2 || tiles_out >= 2048)  launch_mv<K, CB, 4, 2>(packed, tiles_out, tiles_in, x, ldx, m, y, ldy, stream);
-    else                                   launch_mv<K, CB, 4, 1>(packed, tiles_out, tiles_in, x, ldx, m, y, ldy, stream);
+    constexpr int kSms = 148;
+    const bool narrow = tiles_in <= 2 * kMvWarps;
+#define TCQ_MV(M, RT, MB) launch_mv<K, CB, M, RT, MB>(packed, tiles_out, tiles_in, x, ldx, m, y, ldy, stream)
+    if (m == 1) {
+        if ((K == 2 || tiles_out <= 2 * kSms) && !narrow) TCQ_MV(1, 1, 5);
+        else TCQ_MV(1, 1, 0);
+    } else if (m == 2) {
+        if (narrow) TCQ_MV(2, 1, 6);
+        else TCQ_MV(2, 1, 0);
+    } else if (tiles_out > 3 * kSms) {
+        TCQ_MV(4, 2, 3);
+    } else if (K == 2 && tiles_out > kSms && tiles_out <= 2 * kSms) {
+        if constexpr (K == 2) TCQ_MV(4, 2, 0);
+    } else {
+        TCQ_MV(4, 1, 3);
+    }
+#undef TCQ_MV
     return cudaGetLastError();
 }
 
