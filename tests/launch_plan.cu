@@ -8,11 +8,27 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <string>
+#include <vector>
 
 #include "../trellis-everywhere_b200/csrc/tcq_forward_launch.cuh"
 #include "../trellis-everywhere_b200/csrc/tcq_traceback.cuh"
 
 extern int g_failing_queries;
+
+// What a call puts where in its scratch: complaints about bytes outside, and about bytes that another buffer holds.
+constexpr uintptr_t kScratch = 1 << 22;
+static size_t g_scratch_bytes = 0;
+struct Use { std::string what; uintptr_t begin, end; };
+static std::vector<Use> g_uses;
+static void use(const std::string& what, const void* p, size_t bytes) {
+    const Use u{what, reinterpret_cast<uintptr_t>(p), reinterpret_cast<uintptr_t>(p) + bytes};
+    if (u.begin < kScratch + 4 || u.end > kScratch + g_scratch_bytes) std::printf("outside: %s\n", what.c_str());     // (the status word comes first)
+    for (const Use& o : g_uses)
+        if (o.what != what && !(o.what == "edges" && what == "overlap") && !(o.what == "overlap" && what == "edges") && u.begin < o.end && o.begin < u.end)
+            std::printf("shared: %s, %s\n", what.c_str(), o.what.c_str());
+    g_uses.push_back(u);
+}
 
 namespace tcq {
 
@@ -20,7 +36,10 @@ static cudaError_t cluster(int K, const ClusterArgs& ca, int C, int G) {
     // queries go through the real launcher (of the size with the smallest kernel for all but one)
     if (ca.f.n <= 0) return C == 16 ? launch_cluster_variant<2, kCbMcg, 16, 1, 0, 256>(ca, nullptr) : C == 8 ? launch_cluster_variant<2, kCbMcg, 8, 1, 0, 512>(ca, nullptr)
                           : C == 4 ? launch_cluster_variant<2, kCbMcg, 4, 1, 0, 512>(ca, nullptr) : launch_cluster_variant<2, kCbMcg, 2, 1, 0, 512>(ca, nullptr);
-    std::printf("cluster K=%d C=%d G=%d n=%lld\n", K, C, G, ca.f.n);
+    std::printf("cluster K=%d C=%d G=%d n=%lld steps=%d\n", K, C, G, ca.f.n, ca.f.steps);
+    use("rows", ca.rows, ca.f.n * ca.nrows * (size_t(4) << (16 - K)));
+    if (ca.keys != nullptr) use("keys", ca.keys, ca.f.n * C * 8);
+    if (ca.f.overlap != nullptr) use("overlap", ca.f.overlap, ca.f.n * 4);
     return cudaSuccess;
 }
 static cudaError_t cta(int K, const ForwardArgs& a) {
@@ -35,6 +54,7 @@ template <> cudaError_t launch_forward_cta<3>(int, const ForwardArgs& a, int, cu
 template <> cudaError_t launch_forward_cta<4>(int, const ForwardArgs& a, int, cudaStream_t) { return cta(4, a); }
 cudaError_t launch_traceback(int, const TracebackArgs& a, cudaStream_t) {
     std::printf("walk %s n=%lld keys=%d\n", a.rows != nullptr ? "rows" : "backpointers", a.n, a.keys != nullptr ? a.nkeys : 0);
+    if (a.e_out != nullptr) use("edges", a.e_out, a.n * 4);
     return cudaSuccess;
 }
 cudaError_t launch_decode_packed(const uint32_t*, long long, int, int, float*, cudaStream_t) { return cudaErrorUnknown; }
@@ -63,8 +83,10 @@ int main(int argc, char** argv) {
         } else {
             const int K = std::atoi(argv[i + 1]);
             const long long n = std::atoll(argv[i + 2]), bytes = std::atoll(argv[i + 3]);
+            g_scratch_bytes = bytes > 0 ? size_t(bytes) : tcq_workspace_bytes(n, K);
+            g_uses.clear();
             std::printf("status %d\n", tcq_encode_tb(static_cast<float*>(address(1 << 20)), n, K, 2, static_cast<uint32_t*>(address(1 << 21)), nullptr, nullptr,
-                                                     nullptr, address(1 << 22), bytes > 0 ? size_t(bytes) : tcq_workspace_bytes(n, K), nullptr));
+                                                     nullptr, address(kScratch), g_scratch_bytes, nullptr));
             i += 4;
         }
     }

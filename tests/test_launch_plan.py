@@ -55,3 +55,26 @@ def test_every_shape_is_some_batch_s_and_every_switch_is_tested(plan, K):
     assert {s for t in taken for s in t} == set(plan("shapes", K))
     switches = [n for n in range(2, 889) if taken[n - 1] != taken[n - 2]]
     assert len(switches) >= 10 and {n - 1 for n in switches} | set(switches) <= set(SIZES[K])
+
+
+def _earlier_size(n, K):
+    """Scratch that held the recorded argmins of n tiles: a quarter to a third of what their metric rows take."""
+    up = lambda b: -(-b // 256) * 256
+    return up(n * 256 * (1 << (16 - K)) * K // 8) + 2 * up(4 * n) + up(32 * n) + 256
+
+
+@pytest.mark.parametrize("K", KS)
+def test_every_plan_stays_inside_its_scratch(plan, K):
+    full = lambda n: 0
+    for size in (full, lambda n: _earlier_size(n, K), lambda n: _earlier_size(n, K) // 2 + 1024 * 1024, lambda n: _earlier_size(1, K)):
+        lines = plan(*(x for n in (1, 2, 7, 8, 15, 16, 17, 31, 64, 100, 101, 443, 888, 1000) for x in ("encode", K, n, size(n))))
+        assert lines.count("status 0") == 14 and not [x for x in lines if x.startswith(("outside", "shared"))]
+    assert not [x for x in plan("encode", 2, 100, 0, TCQ_FORWARD_KERNEL="cluster16") if x.startswith(("outside", "shared"))]
+
+
+@pytest.mark.parametrize("n,tiles", [(48, 24), (64, 32), (200, 67), (256, 128), (300, 150), (444, 222)])
+def test_half_paths_fit_half_the_tiles_of_the_earlier_size(plan, n, tiles):
+    """K = 4: the rows of half a path are twice the argmins of a whole one, so half the tiles fit: two chunks of three walks each, the
+    fastest plan for these sizes, or three where a third fits a round of a faster shape."""
+    walks = [x for x in plan("encode", 4, n, _earlier_size(n, 4)) if x.startswith("walk")]
+    assert len(walks) == 3 * -(-n // tiles) and f" n={tiles} " in walks[0]

@@ -93,12 +93,14 @@ bool has_cluster_size(int K, int C) {
 
 // The shape that finishes n tiles soonest, counting whole rounds.  (Clusters of 4, 8 and 16 leave SMs of
 // some GPCs over: 33, 15 and 7 of them run at once on a B200's 148 SMs.)  only: this cluster size (0: any).
+constexpr long long kTilesOf16 = 16;              // clusters of sixteen are for the smallest batches, no larger than this (key_words)
 struct Sweep { ClusterShape shape; double us; };
 Sweep pick_cluster(long long n, int K, int only) {
     const auto [s, ns] = shapes(K);
     Sweep best{{2, 2, 0}, 1e300};
     for (int i = 0; i < ns; ++i) {
-        const long long at_once = only != 0 && s[i].C != only ? 0 : clusters_at_once(s[i].C);
+        if (only != 0 ? s[i].C != only : s[i].C > 8 && n > kTilesOf16) continue;
+        const long long at_once = clusters_at_once(s[i].C);
         if (at_once < 1) continue;
         const long long groups = (n + s[i].G - 1) / s[i].G, rounds = (groups + at_once - 1) / at_once;
         if (double(rounds) * s[i].us < best.us) best = Sweep{s[i], double(rounds) * s[i].us};
@@ -135,8 +137,6 @@ size_t bp_bytes_per_tile(int K) { return size_t(kT) * rowb(K); }
 constexpr size_t kAlign = 256;
 size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
-constexpr int kMaxKeys = 16;   // partial minima per tile left by the cluster kernel (one per CTA of a cluster)
-
 // Scratch comes in two forms.  The cluster step kernel leaves metric rows (MetricRows), the single-CTA kernel packed
 // argmins of every step ("backpointers"), which are a quarter of the size.  The status word lies at the front in both.
 int rows_for(int K, int steps) {
@@ -144,7 +144,17 @@ int rows_for(int K, int steps) {
 }
 
 size_t rows_bytes_per_tile(int K, int part) { return size_t(rows_for(K, part)) * (size_t(1) << (kL - K)) * 4; }
-constexpr size_t kSmallBytes = kMaxKeys * sizeof(unsigned long long) + 2 * sizeof(int);     // per tile, beside the rows
+
+// Partial minima left by the cluster kernel, one per tile and CTA of its cluster: eight a tile, sixteen for the tiles that clusters of
+// sixteen may take.  (Sixteen for all took two thirds more beside the rows than there is beside the argmins, so that in the scratch of
+// the argmins of n tiles the rows of half a path fitted n/2 - 1 of them: 64 tiles at K = 4 went in three chunks, 1376 us instead of 934.)
+size_t key_words(long long chunk, int K) {
+    if (kernel_asked_for() == 16) return 16 * size_t(chunk);
+    return 8 * size_t(chunk) + (K == 2 ? 8 * size_t(chunk < kTilesOf16 ? chunk : kTilesOf16) : 0);
+}
+size_t beside_rows_bytes(long long chunk, int K) {             // status word, partial minima, overlaps, edges
+    return align_up(64 + key_words(chunk, K) * sizeof(unsigned long long) + 2 * sizeof(int) * size_t(chunk));
+}
 
 // Bytes for `chunk` tiles with backpointers: those of one whole pass and two int32 hand-off arrays (and a part that is no longer used:
 // what callers were told to bring stays the same).
@@ -155,7 +165,7 @@ size_t bp_ws_bytes(long long chunk, int K) {
 // ... with metric rows for walks over `part` steps at a time, the overlaps, the edges handed from part to part and the partial
 // minima of the final metrics.
 size_t rows_ws_bytes(long long chunk, int K, int part) {
-    return align_up(kSmallBytes * size_t(chunk) + 64) + size_t(chunk) * rows_bytes_per_tile(K, part);
+    return beside_rows_bytes(chunk, K) + size_t(chunk) * rows_bytes_per_tile(K, part);
 }
 
 // Tiles per chunk at full speed.  Backpointers: eight rounds of the largest tile group on every SM.  Metric rows: two
@@ -200,7 +210,7 @@ int swept_steps(int part) { return part == 256 ? 512 : part == 128 ? 256 + 256 +
 
 // Chunk and part for metric rows in ws_bytes: the whole path at once if that many tiles fit; a workspace too small for it holds
 // half or a quarter of a path for two or four times the tiles, which pays (and for one tile may be all that fits) although
-// the sweep is repeated for each part.  80 us: the walks and launches of a chunk.
+// the sweep is repeated for each part.  The walks and launches of a chunk: 86 us at 30 tiles, 160 from 110 on; about 120 in halves and 200 in quarters.
 void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chunk, int* part) {
     *chunk = 0;
     *part = 256;
@@ -211,13 +221,17 @@ void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chun
                                     [K, p](long long m) { return rows_ws_bytes(m, K, p); });
         if (c < 1) continue;
         const bool all = c >= want;
-        if (!all) c = (n + (n + c - 1) / c - 1) / ((n + c - 1) / c);        // as many chunks, of equal size
-        const double us = plan_sweep(c, K).us, rest = n % c != 0 ? plan_sweep(n % c, K).us : 0.0;
-        const double total = (double(n / c) * us + rest) * swept_steps(p) / 256.0 + double((n + c - 1) / c) * (80.0 + 40.0 * (256 / p - 1));
-        if (total < best) {
-            best = total;
-            *chunk = c;
-            *part = p;
+        const long long chunks = (n + c - 1) / c;
+        // as many chunks as that takes, or one more, of equal size: a smaller one may fit a round of a faster shape
+        for (long long m = chunks; m <= chunks + (all ? 0 : 1); ++m) {
+            if (!all) c = (n + m - 1) / m;
+            const double us = plan_sweep(c, K).us, rest = n % c != 0 ? plan_sweep(n % c, K).us : 0.0;
+            const double total = (double(n / c) * us + rest) * swept_steps(p) / 256.0 + double((n + c - 1) / c) * (p == 256 ? 60.0 + (c < 110 ? 0.9 * double(c) : 100.0) : p == 128 ? 120.0 : 200.0);
+            if (total < best) {
+                best = total;
+                *chunk = c;
+                *part = p;
+            }
         }
         if (all) break;                            // smaller parts gain nothing
     }
@@ -240,9 +254,9 @@ int carve(void* ws, size_t ws_bytes, long long n, int K, int num_sms, Workspace*
             out->clustered = true;
             out->chunk = chunk;
             out->keys = reinterpret_cast<unsigned long long*>(base + 64);
-            out->overlap = reinterpret_cast<int*>(out->keys + chunk * kMaxKeys);
+            out->overlap = reinterpret_cast<int*>(out->keys + key_words(chunk, K));
             out->edge = out->overlap + chunk;
-            out->rows = reinterpret_cast<float*>(base + align_up(kSmallBytes * size_t(chunk) + 64));
+            out->rows = reinterpret_cast<float*>(base + beside_rows_bytes(chunk, K));
             return TCQ_OK;
         }
     }
