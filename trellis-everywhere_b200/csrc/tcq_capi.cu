@@ -210,7 +210,7 @@ int swept_steps(int part) { return part == 256 ? 512 : part == 128 ? 256 + 256 +
 
 // Chunk and part for metric rows in ws_bytes: the whole path at once if that many tiles fit; a workspace too small for it holds
 // half or a quarter of a path for two or four times the tiles, which pays (and for one tile may be all that fits) although
-// the sweep is repeated for each part.  The walks and launches of a chunk: 86 us at 30 tiles, 160 from 110 on; about 120 in halves and 200 in quarters.
+// the sweep is repeated for each part.  The walks and launches of a chunk: 86 us at 30 tiles, about 120 from 70 on and in halves, 200 in quarters.
 void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chunk, int* part) {
     *chunk = 0;
     *part = 256;
@@ -226,7 +226,7 @@ void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chun
         for (long long m = chunks; m <= chunks + (all ? 0 : 1); ++m) {
             if (!all) c = (n + m - 1) / m;
             const double us = plan_sweep(c, K).us, rest = n % c != 0 ? plan_sweep(n % c, K).us : 0.0;
-            const double total = (double(n / c) * us + rest) * swept_steps(p) / 256.0 + double((n + c - 1) / c) * (p == 256 ? 60.0 + (c < 110 ? 0.9 * double(c) : 100.0) : p == 128 ? 120.0 : 200.0);
+            const double total = (double(n / c) * us + rest) * swept_steps(p) / 256.0 + double((n + c - 1) / c) * (p == 256 ? 60.0 + (c < 67 ? 0.9 * double(c) : 60.0) : p == 128 ? 120.0 : 200.0);
             if (total < best) {
                 best = total;
                 *chunk = c;
