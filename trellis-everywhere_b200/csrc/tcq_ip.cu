@@ -15,14 +15,14 @@
 //
 // Forward is three reads and one write of 4 bytes per weight: row sums, column sums after the transform down the rows (which is done again
 // in the blocks rather than written and read back; the second read starts at the matrix' end, where the first left it in L2), blocks.  Restore is one
-// read and one write.  12288 x 4096 (201 MB): forward 220 us (rows 35, their mean 8, columns 53 + 4 + 8, blocks 101), restore 90 us; with a kernel
+// read and one write.  12288 x 4096 (201 MB): forward 220 us (rows 35, their mean 8, columns 53 + 4 + 8, blocks 102), restore 87 us; with a kernel
 // per transform and an intermediate matrix 240 and 167.
 //
 // Every product and sum is rounded where the recipe has it (but divisions by the scale vectors are multiplications by their reciprocals,
 // one rounding more than the reference's division), every stage of a transform in natural order, and every reduction runs in an order of
 // its own definition, whatever the launch, without atomics.  A weight that moves by an ulp may fall to another code, and the packed bytes
 // of a matrix with it, so all of that is part of the result (tests/test_gpu_ip_blocks.py states it bit for bit).  Column sums taken from w itself, which an orthonormal
-// transform allows, one factor for two and another order of stages would save 30 + 12 us, at the price of other codes in one matrix of three.
+// transform allows, one factor for two and another order of stages would save 29 + 10 us, at the price of other codes in one matrix of three.
 #include <cmath>
 
 #include <cooperative_groups.h>
@@ -132,6 +132,13 @@ __global__ void __launch_bounds__(1024) ip_finish_rows_kernel(const float* __res
     }
 }
 
+__device__ __forceinline__ void mul4(float* v, const float4& f) {
+    v[0] = __fmul_rn(v[0], f.x);
+    v[1] = __fmul_rn(v[1], f.y);
+    v[2] = __fmul_rn(v[2], f.z);
+    v[3] = __fmul_rn(v[3], f.w);
+}
+
 // One butterfly stage over the register bit H of v.
 template <int N, int H>
 __device__ __forceinline__ void had_stage(float (&v)[N]) {
@@ -158,8 +165,8 @@ __global__ void __launch_bounds__(kColThreads) ip_col_sumsq_kernel(const float* 
                                                                   const float* __restrict__ r, float* __restrict__ out_s,
                                                                   float* __restrict__ inv_out_s, float* __restrict__ part) {
     constexpr int V = B == 128 ? 64 : B;                       // rows of a thread
-    __shared__ float rowf[B + 1];                              // (the upper lanes' rows one bank further)
-    auto slot = [](int i) { return i + (i >> 6); };
+    __shared__ __align__(16) float rowf[B + 4];                // read four at a time (the upper lanes' rows four banks further)
+    auto slot = [](int i) { return i + (i >> 6) * 4; };
     __shared__ float red[kColThreads];
     const int lane = threadIdx.x & 31;
     const int col = B == 128 ? (threadIdx.x >> 5) * 16 + (lane & 15) : threadIdx.x, row = B == 128 ? (lane >> 4) * 64 : 0;
@@ -186,7 +193,7 @@ __global__ void __launch_bounds__(kColThreads) ip_col_sumsq_kernel(const float* 
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < V; ++i) v[i] = __fmul_rn(v[i], rowf[slot(row) + i]);
+    for (int i = 0; i < V; i += 4) mul4(v + i, *reinterpret_cast<const float4*>(rowf + slot(row) + i));
     had_stage<V, 1>(v);
     had_stage<V, 2>(v);
     had_stage<V, 4>(v);
@@ -398,11 +405,16 @@ __device__ __forceinline__ void ip_block(const float* __restrict__ in, int n_liv
 #pragma unroll
         for (int i = 0; i < 64; ++i) v[i] = blk[at(row_of(i), cc)];
         column_stages(v);
-        const float suc = c_live ? su[cc] : 0.0f;
+        const float f = __fmul_rn(norm0, c_live ? su[cc] : 0.0f);            // a sign makes no difference to a rounding
         float* p = out + rc * k + cc;
 #pragma unroll
-        for (int i = 0; i < 64; ++i)
-            if (FULL || (c_live && row_of(i) < n_live)) p[(i * RS) * k] = __fmul_rn(__fmul_rn(v[i], norm0), __fmul_rn(rowf[row_of(i)], suc));
+        for (int i = 0; i < 64; i += 4) {
+            mul4(v + i, make_float4(f, f, f, f));
+            mul4(v + i, *reinterpret_cast<const float4*>(rowf + (warp >> 2) * 64 + i));
+#pragma unroll
+            for (int j = i; j < i + 4; ++j)
+                if (FULL || (c_live && row_of(j) < n_live)) p[(j * RS) * k] = v[j];
+        }
     }
 }
 
@@ -413,10 +425,13 @@ ip_block_kernel(const float* __restrict__ in, long long n, long long k, int logB
                 const float* __restrict__ scale, float* __restrict__ out) {
     extern __shared__ __align__(16) float ip_smem[];
     float* const blk = ip_smem;                                // [128][128]
-    float* const rowf = ip_smem + 128 * 128;                   // [128] factors of the rows
+    float* const rowf = ip_smem + 128 * 128;                   // [128] factors of the rows, back in the order in which a thread of the column form has them
     const long long r0 = (long long)blockIdx.y * 128, c0 = (long long)blockIdx.x * 128;
     const int n_live = int(n - r0 < 128 ? n - r0 : 128), k_live = int(k - c0 < 128 ? k - c0 : 128);
-    if (threadIdx.x < 128) rowf[threadIdx.x] = int(threadIdx.x) < n_live ? __fmul_rn(sv[r0 + threadIdx.x], rs[r0 + threadIdx.x]) : 0.0f;
+    if (threadIdx.x < 128) {
+        const int row = INV ? (threadIdx.x & 63) * 2 + (threadIdx.x >> 6) : threadIdx.x;
+        rowf[threadIdx.x] = row < n_live ? __fmul_rn(sv[r0 + row], rs[r0 + row]) : 0.0f;
+    }
     const long long rowmajor = r0 * k + c0, tile = r0 * k + c0 * 16;          // the block's origin: tile (r0/16)*(k/16) + c0/16, 256 values each
     const float* const src = in + (INV && TILED ? tile : rowmajor);
     float* const dst = out + (!INV && TILED ? tile : rowmajor);
