@@ -60,7 +60,7 @@ CODEBOOK = "3inst"
 MATRIX = (4096, 4096)
 T_SEQ = 256
 STATE_EVALS_PER_WEIGHT = 2 * 65536            # two passes x 2^16 add-compare-select per step
-LANE_OPS_PER_EVAL = 4                         # fsub, fmul, fadd, compare-select: the algorithmic minimum
+LANE_OPS_PER_EVAL = 3                         # fsub, fmul, fadd; the minimum runs on another pipe beside them and does not bind
 WORKLOAD = ("config 2: 4096x4096 fp32 matrix, N(0,0.02^2) + 1% outliers x20, incoherence-processed, "
             "65536 tiles of 256, K=3, L=16, 3INST")
 
@@ -513,7 +513,8 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
             "peak_source": f"{sms} SMs x 128 fp32/int lanes x {sm_max_mhz:.0f} MHz (max SM clock of MEASURED_PEAKS.json"
                            f"{'' if peaks else '; file absent, nominal clock used'}); the path does no tensor-core or "
                            "HBM-bound work, so the measured HBM/bf16 peaks do not bound it",
-            "algorithmic": "4 lane-ops (fsub, fmul, fadd, compare-select) x 65536 state evaluations per tile-step",
+            "algorithmic": "3 fp32 lane-ops (fsub, fmul, fadd) x 65536 state evaluations per tile-step; the minimum runs on the "
+                           "compare/select pipe beside them",
             "launch_ms": {"pass1": kern_ms[0], "pass2": kern_ms[1]}, "tiles_per_launch": chunk,
             "frac_at_sampled_clock": (achieved / (sms * 128 * ck["sm_mhz"] * 1e6)) if ck.get("sm_mhz") else None,
             # ncu dram__bytes_read+write of a 444-tile launch pair against its metric rows
@@ -782,8 +783,8 @@ def run_ldlq(args) -> None:
 
 def run_ip(args) -> None:
     """Side measurement of the incoherence-processing kernels (the producer of the encoder's tiles and the consumer of
-    its reconstruction) through the C ABI with preallocated buffers: forward = 20 algorithmic bytes per weight (w read
-    twice, one intermediate written and read, tiles written), restore = 16."""
+    its reconstruction) through the C ABI with preallocated buffers: forward = 16 algorithmic bytes per weight (w read
+    three times, tiles written), restore = 8."""
     import torch
     from trellis_b200 import _lib, qtip
     torch.cuda.set_device(0)
@@ -834,8 +835,9 @@ def run_ip(args) -> None:
         "config": {"workload": f"SIDE MEASUREMENT: incoherence processing of a [{n}, {k}] fp32 matrix ({n * k * 4 / 2 ** 20:.0f} MiB, larger "
                                "than L2) through tcq_ip_forward / tcq_ip_restore, buffers preallocated", "n": n, "k": k},
         "restore": {"ms_per_step": ms_i, "weights_per_s": n * k / (ms_i * 1e-3), "round_trip_rel_err": err},
-        "gpu_launches": 4 * args.steps,
-        "roofline": {"bound": "hbm", "kernel": "ip_row_rms + ip_col_sumsq + ip_finish_cols + ip_block (forward, 4 launches: 3 reads, 1 write)", "achieved": gbs_f,
+        # forward: row sums, column sums, their scales, blocks; the row scales and the column sums' parts by size; restore one
+        "gpu_launches": (5 + (n > 1024) + (n // qtip._pow2_block(n, 128) > 16)) * args.steps,
+        "roofline": {"bound": "hbm", "kernel": "ip_row_rms + ip_col_sumsq + ip_finish_cols + ip_block (forward: 3 reads, 1 write)", "achieved": gbs_f,
                      "peak": hbm, "unit": "GB/s", "frac": gbs_f / hbm, "traffic": None,
                      "restore": {"achieved": gbs_i, "frac": gbs_i / hbm}},
         "clocks": clocks.summary()}), flush=True)

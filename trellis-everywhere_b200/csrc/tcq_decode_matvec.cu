@@ -164,7 +164,7 @@ void launch_mv(const uint32_t* packed, int tiles_out, int tiles_in, const float*
 //   one right-hand side: loads ahead (47 registers) up to two rows an SM, where the latency of a trip is the bound (K = 3, 64 rows 10.3 -> 8.3), and
 //     at K = 2, whose decode is shortest, always (9496 rows 174 -> 171).  With more rows other warps hide it, and need the registers (31; K = 4, 9496
 //     rows 168, with loads ahead 178), and so do rows too narrow to give every warp a tile (K = 2, 9496 rows of 4 tiles 10.4, 12.4).
-//   two: the compiler's choice (48), within 4 % of the best; narrow rows, which are one trip or less, want more CTAs (K = 3, 9496 rows of 4 tiles 14.4 -> 12.3).
+//   two: the compiler's choice (48; 64 are 10 to 19 % faster up to 148 rows and up to 7 % slower beyond); narrow rows, which are one trip or less, want more CTAs (K = 3, 9496 rows of 4 tiles 14.4 -> 12.3).
 //   three and four: one row per CTA while all run at once, three CTAs per SM (K = 3, 64 rows 14.4 -> 10.3, 256 rows 16.4 -> 14.4), two rows from
 //     there on (K = 4, 592 rows 32.8 -> 19.2; 9496 rows K = 2 / 3 / 4 294 / 318 / 331 -> 263 / 290 / 267).  At K = 2 between one and two rows
 //     an SM two rows in one CTA, decoded first, are faster (256 rows 12.3, 13.1 with one).

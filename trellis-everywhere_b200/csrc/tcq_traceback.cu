@@ -164,8 +164,8 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) tcq_traceback_kernel(const 
 // Per trip the walk takes D steps back.  It reads the NA = Q^D metrics, contiguous in the row, that the current edge can
 // have come from, forms the candidates of the first of the D steps for the Q^(D-1) nodes above them exactly as the step
 // kernel does (same operations, same order, lowest q among equals), and so on up the tree to the current edge; each node
-// carries the q's chosen below it, so the root holds the whole path.  Work per step and tile is at most 1/240 of the step
-// kernel's.
+// carries the q's chosen below it, so the root holds the whole path.  Candidates per step and tile, those that warps and lanes form
+// more than once included: 1/100, 1/180, 1/450 of the step kernel's (K = 2, 3, 4).
 //
 // What bounds it is the latency of one trip, whose address the trip before decides.  So the first level is spread over
 // the CTA (one barrier per trip, two buffers); the other levels are small and every warp does them for itself; and the

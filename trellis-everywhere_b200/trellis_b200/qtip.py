@@ -270,7 +270,7 @@ def encode_rows(src: torch.Tensor, comp: Optional[torch.Tensor], K: int, codeboo
           sse.data_ptr() if sse is not None else None, ws.data_ptr(), ws.numel())
 
 
-_HOST_CHUNK = 2 * 3552          # tiles per pipelined chunk of a host-tensor encode (two workspace chunks)
+_HOST_CHUNK = 2 * 3552          # tiles per pipelined chunk of a host-tensor encode (eight full chunks of the encoder)
 _copy_streams: dict = {}
 
 
