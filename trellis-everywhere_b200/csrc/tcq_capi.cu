@@ -76,10 +76,10 @@ bool cluster_available() { return kernel_asked_for() != 1 && clusters_at_once(2)
 // all SMs of a B200 at work, measured.  A larger cluster divides a tile's step over more SMs, which shortens the step for
 // the few tiles that then fit, no further than the exchange of metrics between SMs allows (0.4 us a step); more tiles per
 // cluster share the step's fixed cost (0.35 us with two SMs; 0.45 us a tile beyond that at K = 3).
-// (A shape that another beats in time and tiles at once is not listed: 4 x 2 at K = 2 and 4, 8 x 2 at K = 4.)
+// (A shape that another beats in time and tiles at once is not listed: 4 x 2 everywhere, 8 x 2 at K = 4.)
 struct ClusterShape { int C, G; double us; };
 constexpr ClusterShape kShapes2[] = {{16, 1, 100}, {8, 1, 120}, {8, 2, 156}, {4, 1, 181}, {2, 1, 240}, {2, 2, 398}, {2, 3, 532}};
-constexpr ClusterShape kShapes3[] = {{8, 1, 107}, {8, 2, 150}, {4, 1, 152}, {4, 2, 205}, {2, 1, 223}, {2, 2, 337}, {2, 3, 460}, {2, 4, 558}, {2, 5, 690}, {2, 6, 804}};
+constexpr ClusterShape kShapes3[] = {{8, 1, 107}, {8, 2, 150}, {4, 1, 152}, {2, 1, 203}, {2, 2, 325}, {2, 3, 440}, {2, 4, 540}, {2, 5, 665}, {2, 6, 786}};
 constexpr ClusterShape kShapes4[] = {{8, 1, 105}, {4, 1, 142}, {2, 1, 205}, {2, 2, 338}, {2, 3, 447}, {2, 4, 548}, {2, 5, 680}, {2, 6, 804}};
 
 struct ShapeList { const ClusterShape* s; int n; };
@@ -286,6 +286,7 @@ cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& 
         ClusterArgs ca{a, wk.rows, rows_for(K, a.bp_steps), a.overlap == nullptr && a.steps == kT ? wk.keys : nullptr, 0, nullptr};
         t->rows = wk.rows;
         t->nrows = ca.nrows;
+        t->other_order = K == 3 && plan.first.C == 2;      // (both launches of a sweep have as many CTAs per cluster)
         t->keys = ca.keys;
         t->nkeys = plan.first.C;
         auto launch = [&](const ClusterShape& shape) -> cudaError_t {

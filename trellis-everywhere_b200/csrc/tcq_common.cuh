@@ -50,6 +50,12 @@ struct MetricRows {
         return (steps + D - 1) / D < (kT - 1) / D ? (steps + D - 1) / D : (kT - 1) / D;
     }
     __host__ __device__ static constexpr uint32_t pos(uint32_t e) { return ((e & ((1u << LB) - 1)) << (K * D)) | (e >> LB); }
+    // The rows of the two-CTA kernel at K = 3 (ClusterPlace<3, 2, 512>) have the ancestors p of an edge (its bits from LB on) in another order: the
+    // bits in which the lanes of a warp of that kernel differ come lowest, so that its store instructions write whole sectors.
+    __host__ __device__ static constexpr uint32_t order(uint32_t p) {
+        return (p & 3) | (p >> 1 & 12) | (p >> 2 & 16) | (p << 3 & 32) | (p << 1 & 64) | (p & 384);
+    }
+    __host__ __device__ static constexpr uint32_t other_pos(uint32_t e) { return ((e & ((1u << LB) - 1)) << (K * D)) | order(e >> LB); }
     // row that the results of step t of a sweep over `steps` steps are, or -1
     __device__ static __forceinline__ int row_after(int t, int steps, int nrows) {
         const int back = steps - 1 - t, j = back / D - 1;

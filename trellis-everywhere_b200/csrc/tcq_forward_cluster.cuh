@@ -159,7 +159,101 @@ struct ClusterItem {
     static constexpr int NI = NB / HB;
     static constexpr int LU = STATES >= Q * Q ? Q : STATES / Q;
     static constexpr int R = HB * LU;
+    static constexpr int SV = R < 4 ? R : 4;               // successors per store (one float, float2 or float4)
+    static constexpr int NWD = R / SV;                     // stores ("words") per item, tile and step
     static_assert(NI * HB * LU * Q == STATES, "a thread's states must form whole successors");
+};
+
+// Which CTA owns a butterfly, where in its rows of metrics the butterfly lies, and which run of edges a thread takes.
+//
+// In general CTA r owns butterflies [r * HN/C, (r+1) * HN/C).  The successors h*Q + l of butterfly h become butterflies
+// (h*Q + l) mod HN, i.e. the bits of h move up by K, and the owner's bits are others every step: all but 1/C of the metrics cross
+// between SMs.
+template <int K, int C, int NT>
+struct ClusterPlace {
+    using IT = ClusterItem<K, C, NT>;
+    static constexpr int Q = Geo<K>::Q, HN = Geo<K>::HN, HNC = HN / C, R = IT::R, NWD = IT::NWD;
+    static constexpr int NCHUNK = Q / IT::LU;
+    // Item i's butterflies lie HI * i after item 0's, and its successors are the predecessors DQ * i later of the same butterflies.
+    static constexpr int HI = HNC / IT::NI, DQ = HI * Q / HN;
+    static_assert(IT::NI == 1 || (HI * Q % HN == 0 && HI % (32 * R) == 0 && HI * Q % 16 == 0), "items must differ by constants");
+    static constexpr int ITEM_EDGE = HI * Q, ITEM_SLOT = HI, ITEM_ROW = HI * Q >> MetricRows<K>::LB;
+    // Address of word w of item i: one of NBASE held in registers, and a constant number of floats.
+    static constexpr int NBASE = NWD, BASE_EDGE = IT::SV;  // base b is where edge b * BASE_EDGE after the thread's first goes
+    __host__ __device__ static constexpr int base(int, int w) { return w; }
+    __host__ __device__ static constexpr int offset(int i, int) { return i * DQ * HNC; }
+    __device__ static uint32_t row_pos(uint32_t e) { return MetricRows<K>::pos(e); }
+    static constexpr int kSwap = 0;                        // value k of an odd word lies at k ^ kSwap
+    // Bytes of a tile's metrics that a CTA receives from others.  The owner of edge e = h*Q + l is bits of h that
+    // start K below the rank's own: with C <= Q they are all bits of hl, and each CTA keeps 1/C of what it produces.  A larger
+    // cluster's upper owner bits are the rank's lowest ones: a CTA keeps 1/Q if those agree with its uppermost bits, else nothing.
+    __device__ static uint32_t remote_bytes(int rank) {
+        constexpr int kUp = C > Q ? C / Q : 1;
+        constexpr uint32_t all = uint32_t(Q * HNC) * 4;
+        return all - (kUp == 1 || rank / (C / kUp) == rank % kUp ? all / (C / kUp) : 0u);
+    }
+    __device__ static int owner(int h) { return h / HNC; }
+    // Slot of a butterfly in a row of metrics.  A thread's run of 8 or 16 edges is stored as 16-byte words; the warp's words
+    // w of all lanes lie together, so that each store instruction writes contiguous memory (the network between SMs takes
+    // half as long for it as for words 32 bytes apart), and the lane bits are flipped per w so that the loads of the next
+    // step, which walk along the edges, still touch every bank once.
+    __device__ static int slot(int h) {
+        const int hl = h % HNC;
+        if constexpr (R <= 4) {
+            return hl;
+        } else {
+            const int word = hl >> 2, w = word % NWD, ln = (word / NWD) & 31;
+            return (hl & ~(32 * R - 1)) | (w * 128 + ((ln ^ (w * (8 / NWD))) << 2)) | (hl & 3);
+        }
+    }
+    __device__ static int butterfly(int rank, int sl) {    // the butterfly of a slot
+        if constexpr (R <= 4) {
+            return rank * HNC + sl;
+        } else {
+            const int word = (sl >> 2) & (32 * NWD - 1), w = word >> 5, ln = (word & 31) ^ (w * (8 / NWD));
+            return rank * HNC + ((sl & ~(32 * R - 1)) | ((ln * NWD + w) << 2) | (sl & 3));
+        }
+    }
+    // first edge of a thread's first run (chunk index fastest: a butterfly's items are neighbours)
+    __device__ static int first_edge(int rank, int tid) { return (rank * HNC + tid / NCHUNK * IT::HB) * Q + tid % NCHUNK * IT::LU; }
+};
+
+// Two CTAs at K = 3: the owner is the majority of h9 h6 h3.  A step moves these bits up by one place and brings in one new one, so
+// most majorities stay: 1/4 of the metrics cross between the SMs, where 1/2 do with an owner that is a bit of its own (or any sum of
+// bits modulo two).  Sweep of 74 / 148 / 222 / 296 / 370 / 444 tiles: 230 / 363 / 469 / 596 / 727 / 828 -> 209 / 340 / 449 / 566 / 697 / 809 us;
+// with nothing sent at all 183 / 330 / 433 / 556 / 688 / 801.  (At K = 2, majority of h11 h9 h7: 564 -> 568 us for 222 tiles, 561 with
+// nothing sent: there the network does not bind.)
+//   slot, from the top: number of the pattern h9 h6 h3 among those with its majority, h2, h8 h7 h5 h4, h1, h0 flipped by h2.
+//   thread: the warp is the pattern's number, h8 and h0, so that a warp's stores all stay or all cross; the lanes are h7 h5 h4 h2 h1.
+//   Loads of a warp then touch every bank once; its store instructions write two runs of 256 bytes, and whole sectors of a metric row
+//   (MetricRows::other_pos).
+template <> struct ClusterPlace<3, 2, 512> {
+    using IT = ClusterItem<3, 2, 512>;
+    static constexpr int ITEM_EDGE = 0, ITEM_SLOT = 0, ITEM_ROW = 0;          // one item
+    static constexpr int NBASE = 1, BASE_EDGE = 0;
+    __host__ __device__ static constexpr int base(int, int) { return 0; }
+    __host__ __device__ static constexpr int offset(int, int w) { return w * 64; }
+    __device__ static uint32_t row_pos(uint32_t e) { return MetricRows<3>::other_pos(e); }
+    static constexpr int kSwap = 1;
+    __device__ static uint32_t remote_bytes(int) { return uint32_t(Geo<3>::E) / 2 * 4 / 4; }
+    __device__ static int pattern(int h) { return (h >> 3 & 1) | (h >> 5 & 2) | (h >> 7 & 4); }
+    // 0 1 2 4 have one set bit at most, 3 5 6 7 two at least
+    __device__ static int number(int p) { return 0x32130210 >> (4 * p) & 3; }
+    __device__ static int numbered(int rank, int n) {      // a pattern's bits at their places in h
+        const int p = (rank != 0 ? 0x7653 : 0x4210) >> (4 * n) & 7;
+        return (p & 1) << 3 | (p & 2) << 5 | (p & 4) << 7;
+    }
+    __device__ static int owner(int h) { return 0xe8 >> pattern(h) & 1; }
+    __device__ static int slot(int h) {
+        return number(pattern(h)) << 7 | (h >> 2 & 1) << 6 | (h >> 7 & 3) << 4 | (h >> 4 & 3) << 2 | ((h & 3) ^ (h >> 2 & 1));
+    }
+    __device__ static int butterfly(int rank, int sl) {
+        return numbered(rank, sl >> 7) | (sl >> 6 & 1) << 2 | (sl >> 4 & 3) << 7 | (sl >> 2 & 3) << 4 | ((sl & 3) ^ (sl >> 6 & 1));
+    }
+    __device__ static int first_edge(int rank, int tid) {
+        const int ln = tid & 31, wp = tid >> 5;
+        return (numbered(rank, wp >> 2) | (wp & 2) << 7 | (wp & 1) | (ln & 3) << 1 | (ln & 12) << 2 | (ln & 16) << 3) * 8;
+    }
 };
 
 template <int K, int C, int GA, int GB>
@@ -175,17 +269,12 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     using MR = MetricRows<K>;
     using IT = ClusterItem<K, C, NT>;
     constexpr int Q = GE::Q, E = GE::E, HN = GE::HN;
-    constexpr int NI = IT::NI, HB = IT::HB, LU = IT::LU, R = IT::R;
+    using PL = ClusterPlace<K, C, NT>;
+    constexpr int NI = IT::NI, HB = IT::HB, LU = IT::LU, R = IT::R, SV = IT::SV, NBASE = PL::NBASE;
     constexpr int G = GA + GB;                     // tiles per cluster group
     constexpr int HNC = HN / C;                    // butterflies per CTA
     constexpr int EC = E / C;                      // metrics per tile held by a CTA
-    constexpr int NCHUNK = Q / LU;
-    constexpr int SV = R < 4 ? R : 4;              // successors per store (one float, float2 or float4)
-    constexpr int NWD = R / SV;                    // stores per item, tile and step
-    constexpr int HI = HNC / NI;                   // item i's butterflies lie HI * i after item 0's ...
-    constexpr int DQ = HI * Q / HN;                // ... and its successors are the predecessors DQ * i later of the same butterflies
-    static_assert(HNC / HB * NCHUNK == NI * NT, "items must divide evenly over the threads");
-    static_assert(NI == 1 || (HI * Q % HN == 0 && HI % (32 * R) == 0 && HI * Q % 16 == 0), "items must differ by constants");
+    static_assert(HNC / HB * (Q / LU) == NI * NT, "items must divide evenly over the threads");
     constexpr uint32_t MUL = CbLcg<CB>::MUL, ADD = CbLcg<CB>::ADD;
     const ForwardArgs& a = ca.f;
 
@@ -204,45 +293,25 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     const float kInf = __uint_as_float(kInfBits);
     const f32x2 one2 = pack2(a.one, a.one);
 
-    // Slot of butterfly hl in a row of metrics.  A thread's run of 8 or 16 edges is stored as 16-byte words; the warp's words
-    // w of all lanes lie together, so that each store instruction writes contiguous memory (the network between SMs takes
-    // half as long for it as for words 32 bytes apart), and the lane bits are flipped per w so that the loads of the next
-    // step, which walk along the edges, still touch every bank once.
-    auto slot = [](int hl) {
-        if constexpr (R <= 4) {
-            return hl;
-        } else {
-            const int word = hl >> 2, w = word % NWD, ln = (word / NWD) & 31;
-            return (hl & ~(32 * R - 1)) | (w * 128 + ((ln ^ (w * (8 / NWD))) << 2)) | (hl & 3);
-        }
-    };
-    auto unslot = [](int sl) {
-        if constexpr (R <= 4) {
-            return sl;
-        } else {
-            const int word = (sl >> 2) & (32 * NWD - 1), w = word >> 5, ln = (word & 31) ^ (w * (8 / NWD));
-            return (sl & ~(32 * R - 1)) | ((ln * NWD + w) << 2) | (sl & 3);
-        }
-    };
-
     // ---- this thread's items: codebook values and destinations, fixed for the whole launch ----
-    const int hl0 = tid / NCHUNK * HB, h0 = rank * HNC + hl0;    // first butterfly (chunk index fastest: a butterfly's items are neighbours)
-    const int e0 = h0 * Q + tid % NCHUNK * LU;                   // first successor edge
-    const int qn = e0 / HN, hn = e0 % HN;                        // its role in the next step: predecessor qn of butterfly hn
-    const bool local = hn / HNC == rank;                         // which this CTA owns itself, or another
-    uint32_t dst[NWD];                                           // where each store goes (tile 0, buffer 0)
+    const int e0 = PL::first_edge(rank, tid);                    // first successor edge
+    const int qn = e0 / HN;                                      // its role in the next step: predecessor qn of butterfly e0 % HN
+    bool local[NBASE];                                           // which this CTA owns itself, or another
+    uint32_t dst[NBASE];                                         // where the words go (tile 0, buffer 0)
 #pragma unroll
-    for (int w = 0; w < NWD; ++w) {
-        dst[w] = smem_u32(cost + qn * HNC + slot(hn % HNC + w * SV));
-        if (!local) dst[w] = map_to_rank(dst[w], hn / HNC);
+    for (int b = 0; b < NBASE; ++b) {
+        const int hn = (e0 + b * PL::BASE_EDGE) % HN;
+        local[b] = PL::owner(hn) == rank;
+        dst[b] = smem_u32(cost + qn * HNC + PL::slot(hn));
+        if (!local[b]) dst[b] = map_to_rank(dst[b], PL::owner(hn));
     }
-    const uint32_t dst_bar = map_to_rank(smem_u32(mbar), hn / HNC);   // the consumer's mbarriers
-    const float* const src = cost + slot(hl0);
-    const uint32_t row_off = MR::pos(uint32_t(e0));              // in a metric row; a run's next edges follow NA apart
+    const uint32_t dst_bar = map_to_rank(smem_u32(mbar), PL::owner(e0 % HN));     // the consumer's mbarriers (one CTA consumes all of a run)
+    const float* const src = cost + PL::slot(e0 / Q);
+    const uint32_t row_off = PL::row_pos(uint32_t(e0));            // in a metric row; a run's next edges follow NA apart
     f32x2 cbv[NI * R][Q / 2];                                    // codebook values of (q = 2j, 2j+1) into each run's edges
 #pragma unroll
     for (int i = 0; i < NI * R; ++i) {
-        const uint32_t xb = uint32_t(e0 + i / R * (HI * Q) + i % R) * MUL + ADD;
+        const uint32_t xb = uint32_t(e0 + i / R * PL::ITEM_EDGE + i % R) * MUL + ADD;
 #pragma unroll
         for (int j = 0; j < Q / 2; ++j)
             cbv[i][j] = pack2(cb_from_x<CB>(xb + uint32_t((2 * j) * E) * MUL), cb_from_x<CB>(xb + uint32_t((2 * j + 1) * E) * MUL));
@@ -255,11 +324,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     float* row_tile0 = nullptr;                    // metric rows of the group's first tile
     int live = 0;                                  // tiles of the group that exist
 
-    // Bytes buffer b of a set of GS tiles receives from OTHER CTAs per step.  The owner of edge e = h*Q + l is bits of h that
-    // start K below the rank's own: with C <= Q they are all bits of hl, and each CTA keeps 1/C of what it produces.  A larger
-    // cluster's upper owner bits are the rank's lowest ones: a CTA keeps 1/Q if those agree with its uppermost bits, else nothing.
-    constexpr int kUp = C > Q ? C / Q : 1;
-    const uint32_t tile_bytes = uint32_t(EC) * 4 - (kUp == 1 || rank / (C / kUp) == rank % kUp ? uint32_t(EC) * 4 / (C / kUp) : 0u);
+    const uint32_t tile_bytes = PL::remote_bytes(rank);      // a tile's metrics that OTHER CTAs send each step
     bool timed_out = false;
 
     // All bytes of buffer b of set s have landed; then re-arm its mbarrier for the next use.
@@ -297,7 +362,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
         for (int q = 0; q < Q; ++q) ld_metrics<HB>(src + (T0 * 2 + CUR) * EC + q * HNC, cin[0][q]);
         static_for<GS * NI>([&](auto gc) __attribute__((always_inline)) {
             constexpr int gi = decltype(gc)::value, g = gi / NI, it = gi % NI, NX = gi + 1;
-            constexpr int OUT = (((T0 + g) * 2 + (CUR ^ 1)) * EC + it * DQ * HNC) * 4;
+            constexpr int OUT = ((T0 + g) * 2 + (CUR ^ 1)) * EC;
             float outv[R];
             static_for<R>([&](auto ic) __attribute__((always_inline)) {
                 constexpr int i = decltype(ic)::value;
@@ -307,7 +372,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                     unpack2(cand_cost2(w2[g], cbv[it * R + i][j], pack2(cin[gi & 1][2 * j][i / LU], cin[gi & 1][2 * j + 1][i / LU]), one2), c[2 * j], c[2 * j + 1]);
                 if constexpr (i == kAhead && NX < GS * NI) {
 #pragma unroll
-                    for (int q = 0; q < Q; ++q) ld_metrics<HB>(src + ((T0 + NX / NI) * 2 + CUR) * EC + NX % NI * HI + q * HNC, cin[NX & 1][q]);
+                    for (int q = 0; q < Q; ++q) ld_metrics<HB>(src + ((T0 + NX / NI) * 2 + CUR) * EC + NX % NI * PL::ITEM_SLOT + q * HNC, cin[NX & 1][q]);
                 }
                 outv[i] = min_tree<Q>(c);
                 if constexpr (gi == GS * NI - 1 && i == R - LU) {
@@ -326,12 +391,20 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                     // step_set proves it, and it is closed before the first store.
                     if (pending) cluster_wait_relaxed();
                     pending = false;
-                    if (local) st_local<OUT, SV>(dst[i / SV], outv + (i + 1 - SV));
-                    else st_remote<OUT, (2 * S + (CUR ^ 1)) * 8, SV>(dst[i / SV], outv + (i + 1 - SV), dst_bar);
+                    constexpr int wd = i / SV, b = PL::base(it, wd), AT = (OUT + PL::offset(it, wd)) * 4;
+                    const float* v = outv + (i + 1 - SV);
+                    float swapped[SV];
+                    if constexpr (PL::kSwap != 0 && wd % 2 != 0) {
+#pragma unroll
+                        for (int k = 0; k < SV; ++k) swapped[k] = v[k ^ PL::kSwap];
+                        v = swapped;
+                    }
+                    if (local[b]) st_local<AT, SV>(dst[b], v);
+                    else st_remote<AT, (2 * S + (CUR ^ 1)) * 8, SV>(dst[b], v, dst_bar);
                 }
             });
             if (row >= 0 && T0 + g < live) {
-                float* const rp = row_tile0 + (size_t(T0 + g) * ca.nrows + row) * E + row_off + it * (HI * Q >> MR::LB);
+                float* const rp = row_tile0 + (size_t(T0 + g) * ca.nrows + row) * E + row_off + it * PL::ITEM_ROW;
 #pragma unroll
                 for (int i = 0; i < R; ++i) rp[i * MR::NA] = outv[i];
             }
@@ -375,7 +448,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
         if (constrained && tid < G) {
             const int ov = (tid < live ? a.overlap[tile0 + tid] : 0) & (E - 1);
             const int qo = ov / HN, ho = ov % HN;                 // metric of edge ov is predecessor qo of butterfly ho
-            if (ho / HNC == rank) cost[(size_t(tid) * 2) * EC + qo * HNC + slot(ho % HNC)] = 0.0f;
+            if (PL::owner(ho) == rank) cost[(size_t(tid) * 2) * EC + qo * HNC + PL::slot(ho)] = 0.0f;
         }
         cluster.sync();   // every CTA's buffers are initialised before anyone stores into them
 
@@ -408,7 +481,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                 const float* fv = cost + (size_t(g) * 2) * EC;
                 unsigned long long key = ~0ull;
                 for (int i = tid; i < EC; i += NT) {
-                    const unsigned edge = unsigned(i / HNC) * HN + rank * HNC + unslot(i % HNC);
+                    const unsigned edge = unsigned(i / HNC) * HN + PL::butterfly(rank, i % HNC);
                     const unsigned long long k2 = (static_cast<unsigned long long>(__float_as_uint(fv[i])) << 32) | edge;
                     key = k2 < key ? k2 : key;
                 }
@@ -434,7 +507,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
         if (a.final_cost != nullptr && constrained && tid < live) {
             const int ov = a.overlap[tile0 + tid] & (E - 1);
             const int qo = ov / HN, ho = ov % HN;
-            if (ho / HNC == rank) a.final_cost[tile0 + tid] = cost[(size_t(tid) * 2) * EC + qo * HNC + slot(ho % HNC)];
+            if (PL::owner(ho) == rank) a.final_cost[tile0 + tid] = cost[(size_t(tid) * 2) * EC + qo * HNC + PL::slot(ho)];
         }
         cluster.sync();   // nobody may start re-initialising while a neighbour still reads or is written to
     }

@@ -10,7 +10,6 @@ cudaError_t launch_cluster_cb(const ClusterArgs& ca, int C, int G, cudaStream_t 
         case 801: return launch_cluster_variant<3, CB, 8, 1, 0, 256>(ca, stream);
         case 802: return launch_cluster_variant<3, CB, 8, 1, 1, 256>(ca, stream);
         case 401: return launch_cluster_variant<3, CB, 4, 1, 0, 512>(ca, stream);
-        case 402: return launch_cluster_variant<3, CB, 4, 1, 1, 512>(ca, stream);
         case 201: return launch_cluster_variant<3, CB, 2, 1, 0, 512>(ca, stream);
         case 202: return launch_cluster_variant<3, CB, 2, 1, 1, 512>(ca, stream);
         case 203: return launch_cluster_variant<3, CB, 2, 2, 1, 512>(ca, stream);

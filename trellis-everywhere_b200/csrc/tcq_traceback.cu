@@ -184,7 +184,8 @@ __device__ __forceinline__ uint32_t first_minimum(const float (&c)[N], float bes
     return qb;
 }
 
-template <int K, int CB>
+// OTHER: the rows' ancestors lie as in MetricRows::other_pos.
+template <int K, int CB, bool OTHER>
 __global__ void __launch_bounds__(WalkShape<K>::W * 32) tcq_walk_kernel(const TracebackArgs a) {
     using GE = Geo<K>;
     using MR = MetricRows<K>;
@@ -241,7 +242,7 @@ __global__ void __launch_bounds__(WalkShape<K>::W * 32) tcq_walk_kernel(const Tr
         return __fmul_rn(d, d);
     };
     int tau = a.t_end - D;                              // first of the trip's D steps
-    // metric(p): the metric of ancestor p before step tau.  kFirst: the trip that holds step 0; nodes before step 0 have the start
+    // metric(q * N1, p): the metric of ancestor q * N1 + p before step tau.  kFirst: the trip that holds step 0; nodes before step 0 have the start
     // metric of their edge.
     auto trip = [&](int buf, auto first_c, auto metric) {
         constexpr bool kFirst = decltype(first_c)::value;
@@ -251,7 +252,7 @@ __global__ void __launch_bounds__(WalkShape<K>::W * 32) tcq_walk_kernel(const Tr
 #pragma unroll
             for (int k = 0; k < QS; ++k) {
                 const uint32_t q = uint32_t(k + (SPLIT > 1 ? lane / N1 * QS : 0));
-                c1[i][k] = metric(q * N1 + uint32_t(tid + i * NT) % N1);
+                c1[i][k] = metric(q * N1, uint32_t(tid + i * NT) % N1);
             }
         // the emissions of every level, under the loads
         float em1[NPT][QS], em[D - 1][NP2][Q], em_root;
@@ -335,24 +336,24 @@ __global__ void __launch_bounds__(WalkShape<K>::W * 32) tcq_walk_kernel(const Tr
     int j = 0;
     for (; tau > 0 && tau + D > t_off; ++j, tau -= D) {
         const float* const row = rows + size_t(j) * E + (e >> (K * D)) * uint32_t(NA);     // the ancestors share the edge's bits above K*D
-        trip(j & 1, std::false_type{}, [&](uint32_t p) { return __ldg(row + p); });
+        trip(j & 1, std::false_type{}, [&](uint32_t pq, uint32_t p) { return __ldg(row + (OTHER ? MR::order(pq) | MR::order(p) : pq | p)); });
     }
     if (tau + D > t_off) {                         // tau <= 0
         const uint32_t g = e >> (K * D);
-        trip(j & 1, std::true_type{}, [&](uint32_t p) { return start_metric((p << LB) | g); });
+        trip(j & 1, std::true_type{}, [&](uint32_t pq, uint32_t p) { return start_metric(((pq + p) << LB) | g); });
     }
     __syncthreads();
     if (tid == 0 && a.e_out != nullptr) a.e_out[tile] = int(st[t_off] >> K);     // a trip may have gone past step t_off
     emit_outputs<K, NT>(a, tile, st, t_off, a.t_end, tid);
 }
 
-template <int K>
+template <int K, bool OTHER>
 cudaError_t launch_walk(const TracebackArgs& a, cudaStream_t stream) {
     const unsigned grid = unsigned(a.n), block = WalkShape<K>::W * 32;
     switch (a.codebook) {
-        case kCb1Mad:  tcq_walk_kernel<K, kCb1Mad><<<grid, block, 0, stream>>>(a); break;
-        case kCb3Inst: tcq_walk_kernel<K, kCb3Inst><<<grid, block, 0, stream>>>(a); break;
-        case kCbMcg:   tcq_walk_kernel<K, kCbMcg><<<grid, block, 0, stream>>>(a); break;
+        case kCb1Mad:  tcq_walk_kernel<K, kCb1Mad, OTHER><<<grid, block, 0, stream>>>(a); break;
+        case kCb3Inst: tcq_walk_kernel<K, kCb3Inst, OTHER><<<grid, block, 0, stream>>>(a); break;
+        case kCbMcg:   tcq_walk_kernel<K, kCbMcg, OTHER><<<grid, block, 0, stream>>>(a); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -365,9 +366,9 @@ cudaError_t launch_traceback(int K, const TracebackArgs& a, cudaStream_t stream)
     const unsigned grid = unsigned((a.n + kWarpsPerCta - 1) / kWarpsPerCta);
     if (a.rows != nullptr) {
         switch (K) {
-            case 2: return launch_walk<2>(a, stream);
-            case 3: return launch_walk<3>(a, stream);
-            case 4: return launch_walk<4>(a, stream);
+            case 2: return launch_walk<2, false>(a, stream);
+            case 3: return a.other_order ? launch_walk<3, true>(a, stream) : launch_walk<3, false>(a, stream);
+            case 4: return launch_walk<4, false>(a, stream);
             default: return cudaErrorInvalidValue;
         }
     }

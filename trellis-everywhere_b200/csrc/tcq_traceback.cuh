@@ -9,6 +9,7 @@ struct TracebackArgs {
     const unsigned char* bp;   // [n][bp_steps][E*K/8] packed backpointers of the LAST bp_steps steps, or nullptr with `rows`
     const float* rows;         // [n][nrows][E] metric rows (MetricRows) of the cluster step kernel, or nullptr
     int nrows;
+    int other_order;           // the rows' ancestors lie as in MetricRows::other_pos
     const float* w;            // with `rows`: the pass's weights, as its ForwardArgs gave them
     const float* w_add;
     int roll;
