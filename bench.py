@@ -60,7 +60,7 @@ CODEBOOK = "3inst"
 MATRIX = (4096, 4096)
 T_SEQ = 256
 STATE_EVALS_PER_WEIGHT = 2 * 65536            # two passes x 2^16 add-compare-select per step
-LANE_OPS_PER_EVAL = 3                         # fsub, fmul, fadd; the minimum runs on another pipe beside them and does not bind
+LANE_OPS_PER_EVAL = 2                         # fsub and ffma (large batches form candidates with a fused multiply-add); the minimum runs on another pipe beside them
 WORKLOAD = ("config 2: 4096x4096 fp32 matrix, N(0,0.02^2) + 1% outliers x20, incoherence-processed, "
             "65536 tiles of 256, K=3, L=16, 3INST")
 
@@ -284,8 +284,8 @@ def check_parity(torch, qtip, lib, _lib, tiles, last, dev, cid) -> dict:
     ok_packed = np.array_equal(last.packed[idx].cpu().numpy().view(np.uint32), O.pack_bits(bits, K_BITS))
     ok_dq = np.array_equal(last.dq[idx].cpu().numpy().view(np.uint32), dq.view(np.uint32))
     ok_sse = np.array_equal(last.sse[idx].cpu().numpy().view(np.uint32), sse.view(np.uint32))
-    # the launches the roofline leg times: one full chunk through the pass-level entry point (same launch code and
-    # tile-group shape as tcq_forward_pass), states of 64 spread tiles against the oracle's passes
+    # the launches the roofline leg times: one full chunk through the pass-level entry point (the same launch code;
+    # candidates are rounded operation by operation there, which the timed launches leave to the walk), states of 64 spread tiles against the oracle's passes
     chunk = min(n, 6 * torch.cuda.get_device_properties(dev).multi_processor_count)
     s1 = qtip.viterbi_pass_b200(tiles[:chunk], K_BITS, None, cid, roll=128)
     jdx = torch.linspace(0, chunk - 1, min(64, chunk), device=dev).round().long()
@@ -513,7 +513,7 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
             "peak_source": f"{sms} SMs x 128 fp32/int lanes x {sm_max_mhz:.0f} MHz (max SM clock of MEASURED_PEAKS.json"
                            f"{'' if peaks else '; file absent, nominal clock used'}); the path does no tensor-core or "
                            "HBM-bound work, so the measured HBM/bf16 peaks do not bound it",
-            "algorithmic": "3 fp32 lane-ops (fsub, fmul, fadd) x 65536 state evaluations per tile-step; the minimum runs on the "
+            "algorithmic": "2 fp32 lane-ops (fsub, ffma) x 65536 state evaluations per tile-step; the minimum runs on the "
                            "compare/select pipe beside them",
             "launch_ms": {"pass1": kern_ms[0], "pass2": kern_ms[1]}, "tiles_per_launch": chunk,
             "frac_at_sampled_clock": (achieved / (sms * 128 * ck["sm_mhz"] * 1e6)) if ck.get("sm_mhz") else None,

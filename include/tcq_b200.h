@@ -193,7 +193,9 @@ TCQ_API int tcq_selftest_wait_timeout(const float *w, int64_t n_tiles, int K, vo
  * Number of kernel launches tcq_encode_tb issues for n_tiles with a workspace of
  * ws_bytes (four per chunk: step kernel and traceback for each of the two passes;
  * six or twelve where the workspace holds a half or a quarter of a path only, and
- * half as many again where a sweep is two launches of different shape),
+ * half as many again where a sweep is two launches of different shape; and two for
+ * the tiles to sweep again, of which there are few or none, in batches that are swept
+ * with fused candidates: 149 tiles or more at K = 3 and 4),
  * or a negative TCQ_E_* code.  No reference counterpart; used for accounting.
  */
 TCQ_API int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes);

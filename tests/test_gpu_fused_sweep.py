@@ -1,0 +1,85 @@
+"""Sweeps with fused candidates (batches of 149 tiles and more at K = 3 and 4): the square and the sum are one operation there, and the walk
+and a second kernel see to it that the codes are those of the rounded operations.  TCQ_FORWARD_KERNEL=cluster2 runs every
+batch with the rounded operations; the two must agree bit for bit, whatever the tiles."""
+import numpy as np
+import pytest
+import torch
+
+from conftest import same_bits
+
+NAMES = ("1mad", "3inst", "mcg")
+
+
+def _tiles(n, lut, seed):
+    """Tiles of every kind by turns: Gaussian at several scales, coarse grids and few levels (ties and near-ties everywhere), zero,
+    constant and periodic tiles, the codebook's own values, beyond its range, below the normal range, sums that
+    overflow, NaN and infinite weights."""
+    g = torch.Generator().manual_seed(seed)
+    w = torch.randn(n, 256, generator=g)
+    i = torch.arange(n) % 24
+    w *= torch.tensor([1.24] * 6 + [0.2, 0.01, 2.5, 30.0] + [1.24] * 14)[i][:, None]
+    w[i == 10], w[i == 11] = (w[i == 10] * 4).round() / 4, w[i == 11].sign()
+    w[i == 12], w[i == 13] = 0.0, 0.5
+    w[i == 14, ::2] = 0.0
+    w[i == 15] = lut[torch.randint(0, 65536, (int((i == 15).sum()), 256), generator=g)]
+    w[i == 16], w[i == 17], w[i == 18] = w[i == 16] * 1e-20, 1e18, -1.9e19
+    w[i == 19, 10], w[i == 20, 200], w[i == 21] = float("nan"), float("inf"), float("nan")
+    w[i == 22, 64:] = 0.0
+    w[i == 23] = w[i == 23][:, :8].repeat(1, 32)
+    return w
+
+
+def _both(q, monkeypatch, call):
+    got = call()
+    monkeypatch.setenv("TCQ_FORWARD_KERNEL", "cluster2")
+    want = call()
+    monkeypatch.delenv("TCQ_FORWARD_KERNEL")
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    return got
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (3, 4))
+@pytest.mark.parametrize("name", NAMES)
+@pytest.mark.parametrize("n", (149, 300, 445, 900))       # one launch and two, one chunk and two; 450 tiles to sweep again in the last
+def test_codes_are_those_of_the_rounded_operations(monkeypatch, K, name, n):
+    from trellis_b200 import qtip as q
+    w = _tiles(n, q.codebook_lut(name, "cpu"), 10 * n + K).cuda()
+    _both(q, monkeypatch, lambda: q.encode(w, K, name, want_bits=True))
+    rows, comp = w.reshape(n, 16, 16).permute(2, 0, 1).reshape(16, 16 * n).contiguous(), torch.randn(16, 16 * n, device="cuda") * 0.05
+
+    def row_block():
+        wq, err = torch.empty_like(rows), torch.empty_like(rows)
+        packed, sse = torch.empty(n, 8 * K, dtype=torch.int32, device="cuda"), torch.empty(n, device="cuda")
+        q.encode_rows(rows, comp, K, name, wq, err, packed, sse)
+        return wq, err, packed, sse
+
+    _both(q, monkeypatch, row_block)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (3, 4))
+def test_a_large_batch_of_ordinary_tiles(oracle, luts, monkeypatch, K):
+    """20 000 Gaussian tiles (some hundred of them with another path within the limit), and a sample against the oracle."""
+    from trellis_b200 import qtip as q
+    w = torch.randn(20000, 256, generator=torch.Generator().manual_seed(K)) * 1.24
+    got = _both(q, monkeypatch, lambda: q.encode(w.cuda(), K, "mcg", want_bits=True))
+    idx = np.arange(0, 20000, 500)
+    bits, dq, sse = oracle.viterbi_tb(w.numpy()[idx], K, luts["mcg"], with_sse=True)
+    assert np.array_equal(got.bits.cpu().numpy()[idx], bits) and same_bits(got.dq.cpu().numpy()[idx], dq) and same_bits(got.sse.cpu().numpy()[idx], sse)
+
+
+def test_the_bound_between_fused_and_rounded_sums():
+    """|A - F| <= (2 t + 2) u H of the limit (fused_limit), over random, repeated and graded terms; A as the fused operation gives it (the
+    square is exact in 64 bits, the sum there rounds 2^29 times finer)."""
+    rng = np.random.default_rng(1)
+    for d in (rng.normal(size=(256, 2000)), np.repeat(rng.normal(size=(1, 2000)), 256, 0), rng.normal(size=(256, 2000)) * np.logspace(-4, 2, 256)[:, None],
+              np.tile(rng.normal(size=(8, 2000)), (32, 1)) * 0.17, rng.normal(size=(256, 2000)) ** 9):
+        d = d.astype(np.float32)
+        A, F = np.zeros(2000, np.float32), np.zeros(2000, np.float32)
+        for t in range(256):
+            A = (d[t].astype(np.float64) ** 2 + A).astype(np.float32)
+            F = d[t] * d[t] + F
+            H = 2.0 ** np.floor(np.log2(np.maximum((A * np.float32(1.0005)).astype(np.float64), 1e-30)))
+            assert (np.abs(A.astype(np.float64) - F) <= (2 * (t + 1) + 2) * 2.0 ** -24 * H).all()

@@ -82,8 +82,13 @@ constexpr ClusterShape kShapes2[] = {{16, 1, 100}, {8, 1, 120}, {8, 2, 156}, {4,
 constexpr ClusterShape kShapes3[] = {{8, 1, 107}, {8, 2, 150}, {4, 1, 152}, {2, 1, 203}, {2, 2, 325}, {2, 3, 440}, {2, 4, 540}, {2, 5, 665}, {2, 6, 786}};
 constexpr ClusterShape kShapes4[] = {{8, 1, 105}, {4, 1, 142}, {2, 1, 205}, {2, 2, 338}, {2, 3, 447}, {2, 4, 548}, {2, 5, 680}, {2, 6, 804}};
 
+// With fused candidates (two SMs per cluster only).
+constexpr ClusterShape kFusedShapes3[] = {{2, 1, 172}, {2, 2, 285}, {2, 3, 362}, {2, 4, 457}, {2, 5, 553}, {2, 6, 660}};
+constexpr ClusterShape kFusedShapes4[] = {{2, 1, 172}, {2, 2, 299}, {2, 3, 370}, {2, 4, 461}, {2, 5, 590}, {2, 6, 661}};
+
 struct ShapeList { const ClusterShape* s; int n; };
-ShapeList shapes(int K) {
+ShapeList shapes(int K, bool fused = false) {
+    if (fused) return K == 3 ? ShapeList{kFusedShapes3, int(std::size(kFusedShapes3))} : ShapeList{kFusedShapes4, int(std::size(kFusedShapes4))};
     return K == 2 ? ShapeList{kShapes2, int(std::size(kShapes2))} : K == 3 ? ShapeList{kShapes3, int(std::size(kShapes3))} : ShapeList{kShapes4, int(std::size(kShapes4))};
 }
 bool has_cluster_size(int K, int C) {
@@ -95,8 +100,8 @@ bool has_cluster_size(int K, int C) {
 // some GPCs over: 33, 15 and 7 of them run at once on a B200's 148 SMs.)  only: this cluster size (0: any).
 constexpr long long kTilesOf16 = 16;              // clusters of sixteen are for the smallest batches, no larger than this (key_words)
 struct Sweep { ClusterShape shape; double us; };
-Sweep pick_cluster(long long n, int K, int only) {
-    const auto [s, ns] = shapes(K);
+Sweep pick_cluster(long long n, int K, int only, bool fused) {
+    const auto [s, ns] = shapes(K, fused);
     Sweep best{{2, 2, 0}, 1e300};
     for (int i = 0; i < ns; ++i) {
         if (only != 0 ? s[i].C != only : s[i].C > 8 && n > kTilesOf16) continue;
@@ -114,18 +119,18 @@ Sweep pick_cluster(long long n, int K, int only) {
 // 2282 -> 1991.  5 us: a launch.  Only where it promises 4 %: the table is not better than that (256 tiles at K = 2, where it
 // promises 2 %, took 3 % longer).
 struct SweepPlan { ClusterShape first, second; long long n_first; double us; };
-SweepPlan plan_sweep(long long n, int K) {
+SweepPlan plan_sweep(long long n, int K, bool fused = false) {
     const int asked = kernel_asked_for(), only = asked > 1 ? asked : 0;
-    const Sweep one = pick_cluster(n, K, only);
+    const Sweep one = pick_cluster(n, K, only, fused);
     const SweepPlan whole{one.shape, one.shape, n, one.us};
     if (only != 0 && only != 2) return whole;
     SweepPlan best = whole;
     best.us *= 0.96;
-    const auto [s, ns] = shapes(K);
+    const auto [s, ns] = shapes(K, fused);
     for (int i = 0; i < ns; ++i) {
         const long long round = s[i].C == 2 ? (long long)clusters_at_once(2) * s[i].G : 0;
         if (round < 1 || n <= round || n % round == 0) continue;
-        const Sweep rest = pick_cluster(n % round, K, 2);
+        const Sweep rest = pick_cluster(n % round, K, 2, fused);
         const double us = double(n / round) * s[i].us + rest.us + 5.0;
         if (us < best.us) best = SweepPlan{s[i], rest.shape, n / round * round, us};
     }
@@ -184,7 +189,25 @@ struct Workspace {
     unsigned long long* keys;
     unsigned int* status;
     long long chunk;
+    // Sweeps with fused candidates (see plan_fused)
+    bool fused;
+    long long span;             // tiles that go through pass 1 before any goes through pass 2 (their overlaps are kept)
+    int* list;                  // [span] tiles to sweep again
+    int* counts;                // their numbers after the walks of pass 1 and of pass 2
 };
+
+// Batches from here on are swept with fused candidates, and the tiles whose path that does not settle again (one in a thousand, by a
+// kernel of its own after the walks of each pass).  Smaller ones are bound by the exchange between SMs and not by arithmetic, and there a
+// tile swept again, 0.2 ms, is a larger part of a call: 148 tiles at K = 3 would gain 4 %.  At K = 2 the metric rows bind as well (a sweep of 444
+// tiles 1115 -> 1022 us), and the longer walk takes most of the gain: 150 tiles 1220 -> 1230 us a call, 1000 tiles 5431 -> 5372.
+constexpr int kFusedFrom = 149;
+constexpr int kListedC = 4;
+constexpr long long kSpan = 1 << 18;               // the full-speed size holds the overlaps of so many tiles
+bool plan_fused(long long n, int K, const Workspace& wk) {
+    return K >= 3 && n >= kFusedFrom && wk.part == kT && kernel_asked_for() == 0 && wk.chunk >= (n < 2 * kFusedFrom ? n : 2 * kFusedFrom) && clusters_at_once(kListedC) > 0;
+}
+// Tiles of a chunk: whole rounds of the largest shape (six tiles a cluster), which has the most tiles per time.
+long long fused_chunk() { return 12LL * clusters_at_once(2); }
 
 // Largest chunk of at most `want` tiles; `need(chunk)` bytes, about per_tile each.
 template <typename Need>
@@ -237,7 +260,8 @@ void plan_rows(long long n, size_t ws_bytes, int K, int num_sms, long long* chun
     }
 }
 
-int carve(void* ws, size_t ws_bytes, long long n, int K, int num_sms, Workspace* out) {
+// fusible: whether the caller can do with sweeps with fused candidates.
+int carve(void* ws, size_t ws_bytes, long long n, int K, int num_sms, Workspace* out, bool fusible) {
     if (ws == nullptr) return TCQ_E_NULL_POINTER;
     if (reinterpret_cast<uintptr_t>(ws) % kAlign) return TCQ_E_MISALIGNED;
     if (kernel_asked_for() > 1 && !has_cluster_size(K, kernel_asked_for())) return TCQ_E_BAD_ARGUMENT;
@@ -257,6 +281,22 @@ int carve(void* ws, size_t ws_bytes, long long n, int K, int num_sms, Workspace*
             out->overlap = reinterpret_cast<int*>(out->keys + key_words(chunk, K));
             out->edge = out->overlap + chunk;
             out->rows = reinterpret_cast<float*>(base + beside_rows_bytes(chunk, K));
+            if (fusible && plan_fused(n, K, *out)) {
+                // as above, with the overlaps and the list of a span in all that the rows of a chunk leave over
+                const long long c = n <= chunk ? n : fused_chunk() < chunk ? fused_chunk() : chunk;
+                const size_t rows = size_t(c) * rows_bytes_per_tile(K, kT), keys = 64 + size_t(c) * 2 * kFusedKeys * sizeof(unsigned long long);
+                const size_t left = (ws_bytes - rows) / kAlign * kAlign;
+                const long long span = left < keys ? 0 : (long long)((left - keys) / (2 * sizeof(int)));
+                if (span >= c) {
+                    out->fused = true;
+                    out->chunk = c;
+                    out->span = n < span ? n : span / c * c;
+                    out->counts = reinterpret_cast<int*>(base + 16);
+                    out->overlap = reinterpret_cast<int*>(base + keys);
+                    out->list = out->overlap + out->span;
+                    out->rows = reinterpret_cast<float*>(base + align_up(keys + size_t(out->span) * 2 * sizeof(int)));
+                }
+            }
             return TCQ_OK;
         }
     }
@@ -282,13 +322,16 @@ cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& 
     t->e_start = a.overlap != nullptr ? a.overlap : wk.e_final;
     t->keys = nullptr;
     if (wk.clustered) {
-        const SweepPlan plan = plan_sweep(a.n, K);
-        ClusterArgs ca{a, wk.rows, rows_for(K, a.bp_steps), a.overlap == nullptr && a.steps == kT ? wk.keys : nullptr, 0, nullptr};
+        const SweepPlan plan = plan_sweep(a.n, K, wk.fused);
+        ClusterArgs ca{a, wk.rows, rows_for(K, wk.fused ? kT : a.bp_steps), a.overlap == nullptr && a.steps == kT ? wk.keys : nullptr};
+        ca.form = wk.fused ? StepForm::kFused : StepForm::kRounded;
+        ca.counts = wk.counts;
         t->rows = wk.rows;
         t->nrows = ca.nrows;
         t->other_order = K == 3 && plan.first.C == 2;      // (both launches of a sweep have as many CTAs per cluster)
         t->keys = ca.keys;
-        t->nkeys = plan.first.C;
+        t->nkeys = plan.first.C * (wk.fused ? kFusedKeys : 1);
+        t->fused = wk.fused;
         auto launch = [&](const ClusterShape& shape) -> cudaError_t {
             ca.at_once = clusters_at_once(shape.C);
             if (ca.at_once < 1) return cudaErrorNotSupported;
@@ -308,9 +351,9 @@ cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& 
         if (ca.f.w_add != nullptr) ca.f.w_add += at * tile_step;
         if (ca.f.overlap != nullptr) ca.f.overlap += at;
         if (ca.f.final_cost != nullptr) ca.f.final_cost += at;
-        ca.f.flags &= ~kFwdResetStatus;            // the first launch has cleared the status word
+        ca.f.flags &= ~(kFwdResetStatus | kFwdResetCounts);      // the first launch has cleared them
         ca.rows += size_t(at) * ca.nrows * (size_t(1) << (kL - K));
-        if (ca.keys != nullptr) ca.keys += at * plan.first.C;
+        if (ca.keys != nullptr) ca.keys += at * t->nkeys;
         return launch(plan.second);
     }
     t->bp = wk.bp;
@@ -344,10 +387,39 @@ int pass(int K, int codebook, ForwardArgs f, int walk, TracebackArgs out, const 
     return TCQ_OK;
 }
 
+// The tiles of a span that the walks of a pass have listed, swept and walked again with every operation rounded: one kernel, which ends
+// at once if there are none.  f, t: the pass and its outputs from the span's first tile on.
+int listed(int K, int codebook, ForwardArgs f, int walk, TracebackArgs t, const Workspace& wk, const int* count, cudaStream_t s, const char* what) {
+    f.steps = kT;
+    f.bp_steps = walk;
+    ClusterArgs ca{f, wk.rows, rows_for(K, walk), f.overlap == nullptr ? wk.keys : nullptr};
+    ca.at_once = clusters_at_once(kListedC);
+    if (ca.at_once > wk.chunk) ca.at_once = int(wk.chunk);         // rows of one tile per cluster
+    ca.f.n = f.n < ca.at_once ? f.n : ca.at_once;
+    ca.form = StepForm::kListed;
+    ca.list = wk.list;
+    ca.list_count = count;
+    t.rows = wk.rows;
+    t.nrows = ca.nrows;
+    t.w = f.w;
+    t.w_add = f.w_add;
+    t.ld = f.ld;
+    t.roll = f.roll;
+    t.overlap = t.e_start = f.overlap;
+    t.keys = ca.keys;
+    t.nkeys = kListedC;
+    t.bp_steps = walk;
+    t.t_end = kT;
+    t.codebook = codebook;
+    ca.walk = t;
+    const cudaError_t err = K == 3 ? launch_forward_cluster<3>(codebook, ca, kListedC, 1, s) : launch_forward_cluster<4>(codebook, ca, kListedC, 1, s);
+    return err == cudaSuccess ? TCQ_OK : cuda_fail(err, what);
+}
+
 // Launches of an encode for a chunk of n tiles: a sweep (of one or two launches) and a walk for each part of the two passes.
 int launches_of_chunk(long long n, int K, const Workspace& wk) {
     const int parts = (wk.part >= 128 ? 1 : 2) + 256 / wk.part;
-    return parts * (wk.clustered && plan_sweep(n, K).n_first < n ? 3 : 2);
+    return parts * (wk.clustered && plan_sweep(n, K, wk.fused).n_first < n ? 3 : 2);
 }
 
 int check_common(int K, int codebook, long long n) {
@@ -381,23 +453,21 @@ int encode_core(const EncodeIO& io, int K, int codebook, void* ws, size_t ws_byt
     int rc, num_sms = 0;
     if ((rc = current_num_sms(&num_sms)) != TCQ_OK) return rc;
     Workspace wk;
-    if ((rc = carve(ws, ws_bytes, io.n, K, num_sms, &wk)) != TCQ_OK) return rc;
-    // start of chunk c0 inside w / w_add / wq / err: whole tiles (1 KiB each) or 16 columns of the row block per tile
+    if ((rc = carve(ws, ws_bytes, io.n, K, num_sms, &wk, true)) != TCQ_OK) return rc;
+    // start of tile c0 inside w / w_add / wq / err: whole tiles (1 KiB each) or 16 columns of the row block per tile
     const long long tile_step = io.ld > 0 ? 16 : kT;
-    for (long long c0 = 0; c0 < io.n; c0 += wk.chunk) {
-        const long long cn = io.n - c0 < wk.chunk ? io.n - c0 : wk.chunk;
-        const float* w = io.w + c0 * tile_step;
-        const float* w_add = io.w_add ? io.w_add + c0 * tile_step : nullptr;
-        // pass 1: tile rotated by half its length, free start; only the second half of the path is needed, to
-        // reach the state at rotated position 128 (qtip.py:138-141)
-        ForwardArgs f1{w, w_add, io.ld, cn, nullptr, kT / 2, 0, 0, wk.bp, wk.e_final, nullptr, 1.0f, 0, wk.status,
-                       c0 == 0 ? kFwdResetStatus : 0};
-        TracebackArgs t1{};
-        t1.e_out = wk.overlap;
-        if ((rc = pass(K, codebook, f1, kT / 2, t1, wk, num_sms, s, "pass 1")) != TCQ_OK) return rc;
-        // pass 2: true order, start and end tied to the overlap (qtip.py:142)
-        ForwardArgs f2{w, w_add, io.ld, cn, wk.overlap, 0, 0, 0, wk.bp, nullptr, io.sse ? io.sse + c0 : nullptr, 1.0f, 0,
-                       wk.status, kFwdCheckFinite};
+    // pass 1 over cn tiles from c0 on: tile rotated by half its length, free start; only the second half of the path is needed, to
+    // reach the state at rotated position 128 (qtip.py:138-141)
+    auto forward_1 = [&](long long c0, long long cn) {
+        return ForwardArgs{io.w + c0 * tile_step, io.w_add ? io.w_add + c0 * tile_step : nullptr, io.ld, cn, nullptr, kT / 2, 0, 0, wk.bp, wk.e_final, nullptr, 1.0f, 0,
+                           wk.status, c0 == 0 ? kFwdResetStatus : 0};
+    };
+    // pass 2: true order, start and end tied to the overlap (qtip.py:142)
+    auto forward_2 = [&](long long c0, long long cn, const int* overlap) {
+        return ForwardArgs{io.w + c0 * tile_step, io.w_add ? io.w_add + c0 * tile_step : nullptr, io.ld, cn, overlap, 0, 0, 0, wk.bp, nullptr, io.sse ? io.sse + c0 : nullptr, 1.0f, 0,
+                           wk.status, kFwdCheckFinite};
+    };
+    auto outputs = [&](long long c0) {
         TracebackArgs t{};
         t.bits = io.bits ? reinterpret_cast<long long*>(io.bits) + c0 * kT : nullptr;
         t.dq = io.dq ? io.dq + c0 * kT : nullptr;
@@ -405,8 +475,47 @@ int encode_core(const EncodeIO& io, int K, int codebook, void* ws, size_t ws_byt
         t.packed_stride = io.packed_stride;
         t.wq = io.wq ? io.wq + c0 * tile_step : nullptr;
         t.err = io.err ? io.err + c0 * tile_step : nullptr;
-        t.src = w;
-        if ((rc = pass(K, codebook, f2, kT, t, wk, num_sms, s, "pass 2")) != TCQ_OK) return rc;
+        t.src = io.w + c0 * tile_step;
+        return t;
+    };
+    if (!wk.fused) {
+        for (long long c0 = 0; c0 < io.n; c0 += wk.chunk) {
+            const long long cn = io.n - c0 < wk.chunk ? io.n - c0 : wk.chunk;
+            TracebackArgs t1{};
+            t1.e_out = wk.overlap;
+            if ((rc = pass(K, codebook, forward_1(c0, cn), kT / 2, t1, wk, num_sms, s, "pass 1")) != TCQ_OK) return rc;
+            if ((rc = pass(K, codebook, forward_2(c0, cn, wk.overlap), kT, outputs(c0), wk, num_sms, s, "pass 2")) != TCQ_OK) return rc;
+        }
+        return TCQ_OK;
+    }
+    // Both passes of a whole span one after the other, so that the tiles that a pass has to sweep again, few and anywhere, go together.
+    for (long long s0 = 0; s0 < io.n; s0 += wk.span) {
+        const long long sn = io.n - s0 < wk.span ? io.n - s0 : wk.span;
+        for (int second = 0; second < 2; ++second) {
+            for (long long c0 = 0; c0 < sn; c0 += wk.chunk) {
+                const long long cn = sn - c0 < wk.chunk ? sn - c0 : wk.chunk;
+                ForwardArgs f = second ? forward_2(s0 + c0, cn, wk.overlap + c0) : forward_1(s0 + c0, cn);
+                if (!second && c0 == 0) f.flags |= kFwdResetCounts;
+                f.final_cost = nullptr;            // the walk sums it up by the defined operations
+                TracebackArgs t{};
+                if (second) {
+                    t = outputs(s0 + c0);
+                    t.sse = io.sse ? io.sse + s0 + c0 : nullptr;
+                } else {
+                    t.e_out = wk.overlap + c0;
+                }
+                t.again = wk.list;
+                t.again_count = wk.counts + second;
+                t.first_tile = int(c0);
+                if ((rc = pass(K, codebook, f, second ? kT : kT / 2, t, wk, num_sms, s, second ? "pass 2" : "pass 1")) != TCQ_OK) return rc;
+            }
+            ForwardArgs f = second ? forward_2(s0, sn, wk.overlap) : forward_1(s0, sn);
+            f.flags = 0;
+            TracebackArgs t{};
+            if (second) t = outputs(s0);
+            else t.e_out = wk.overlap;
+            if ((rc = listed(K, codebook, f, second ? kT : kT / 2, t, wk, wk.counts + second, s, second ? "pass 2, listed tiles" : "pass 1, listed tiles")) != TCQ_OK) return rc;
+        }
     }
     return TCQ_OK;
 }
@@ -456,7 +565,8 @@ size_t tcq_workspace_bytes(int64_t n_tiles, int K) {
     }
     const long long n = n_tiles < 1 ? 1 : n_tiles;
     const size_t bp = bp_ws_bytes(n < bp_chunk(num_sms) ? n : bp_chunk(num_sms), K);
-    const size_t rows = rows_ws_bytes(n < rows_chunk(num_sms) ? n : rows_chunk(num_sms), K, kT);
+    size_t rows = rows_ws_bytes(n < rows_chunk(num_sms) ? n : rows_chunk(num_sms), K, kT);
+    if (n > rows_chunk(num_sms)) rows += align_up(2 * sizeof(int) * size_t((n < kSpan ? n : kSpan) - rows_chunk(num_sms)));
     return rows > bp ? rows : bp;
 }
 
@@ -516,7 +626,7 @@ int tcq_viterbi_pass(const float* w, int64_t n_tiles, int K, int codebook, const
     int num_sms = 0;
     if ((rc = current_num_sms(&num_sms)) != TCQ_OK) return rc;
     Workspace wk;
-    if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
+    if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk, false)) != TCQ_OK) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(wk.status, 0, sizeof(unsigned int), s) != cudaSuccess) return cuda_fail(cudaGetLastError(), "status reset");
 
@@ -542,7 +652,7 @@ int tcq_forward_pass(const float* w, int64_t n_tiles, int K, int codebook, const
     int num_sms = 0;
     if ((rc = current_num_sms(&num_sms)) != TCQ_OK) return rc;
     Workspace wk;
-    if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
+    if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk, true)) != TCQ_OK) return rc;
     if (bp_chunk_for(n_tiles, ws_bytes, K, num_sms) < n_tiles) return TCQ_E_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(wk.status, 0, sizeof(unsigned int), s) != cudaSuccess) return cuda_fail(cudaGetLastError(), "status reset");
@@ -565,7 +675,7 @@ int tcq_workspace_status(const void* ws, size_t ws_bytes, int64_t n_tiles, int K
     int rc = current_num_sms(&num_sms);
     if (rc != TCQ_OK) return rc;
     Workspace wk;
-    if ((rc = carve(const_cast<void*>(ws), ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
+    if ((rc = carve(const_cast<void*>(ws), ws_bytes, n_tiles, K, num_sms, &wk, true)) != TCQ_OK) return rc;
     unsigned int host = 0;
     cudaError_t err = cudaMemcpyAsync(&host, wk.status, sizeof(host), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream));
     if (err == cudaSuccess) err = cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
@@ -583,14 +693,14 @@ int tcq_selftest_wait_timeout(const float* w, int64_t n_tiles, int K, void* ws, 
     int num_sms = 0;
     if ((rc = current_num_sms(&num_sms)) != TCQ_OK) return rc;
     Workspace wk;
-    if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
+    if ((rc = carve(ws, ws_bytes, n_tiles, K, num_sms, &wk, false)) != TCQ_OK) return rc;
     if (bp_ws_bytes(n_tiles, K) > ws_bytes) return TCQ_E_WORKSPACE;
     if (!cluster_available()) return TCQ_E_BAD_ARGUMENT;   // the single-CTA kernel has no bounded waits to test
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(wk.status, 0, sizeof(unsigned int), s) != cudaSuccess) return cuda_fail(cudaGetLastError(), "status reset");
     // the buffers of the final metrics are told to expect 16 bytes more than the cluster will ever send
     ForwardArgs f{w, nullptr, 0, n_tiles, nullptr, 0, 0, kT, nullptr, nullptr, nullptr, 1.0f, 16, wk.status, 0};
-    ClusterArgs ca{f, nullptr, 0, nullptr, clusters_at_once(2), nullptr};
+    ClusterArgs ca{f, nullptr, 0, nullptr, clusters_at_once(2)};
     cudaError_t err = K == 2   ? launch_forward_cluster<2>(kCbMcg, ca, 2, 2, s)
                       : K == 3 ? launch_forward_cluster<3>(kCbMcg, ca, 2, 2, s)
                                : launch_forward_cluster<4>(kCbMcg, ca, 2, 2, s);
@@ -606,9 +716,13 @@ int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes) {
     if (rc != TCQ_OK) return rc;
     Workspace wk;
     alignas(256) static unsigned char dummy[256];          // carve() only does pointer arithmetic on it
-    if ((rc = carve(dummy, ws_bytes, n_tiles, K, num_sms, &wk)) != TCQ_OK) return rc;
-    const int64_t whole = n_tiles / wk.chunk, rest = n_tiles % wk.chunk;
-    return whole * launches_of_chunk(wk.chunk, K, wk) + (rest > 0 ? launches_of_chunk(rest, K, wk) : 0);
+    if ((rc = carve(dummy, ws_bytes, n_tiles, K, num_sms, &wk, true)) != TCQ_OK) return rc;
+    auto of_span = [&](int64_t n) {
+        const int64_t whole = n / wk.chunk, rest = n % wk.chunk;
+        return whole * launches_of_chunk(wk.chunk, K, wk) + (rest > 0 ? launches_of_chunk(rest, K, wk) : 0) + (wk.fused ? 2 : 0);
+    };
+    if (!wk.fused) return of_span(n_tiles);
+    return n_tiles / wk.span * of_span(wk.span) + (n_tiles % wk.span > 0 ? of_span(n_tiles % wk.span) : 0);
 }
 
 int tcq_decode_packed(const uint32_t* packed, int64_t n_tiles, int K, int codebook, float* dq, void* stream) {

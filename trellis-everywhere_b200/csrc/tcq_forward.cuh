@@ -41,6 +41,7 @@ namespace tcq {
 // ForwardArgs::flags
 constexpr int kFwdResetStatus = 1;   // clear the status word at kernel start (the first launch of a call only)
 constexpr int kFwdCheckFinite = 2;   // flag NaN / infinite weights in the status word
+constexpr int kFwdResetCounts = 4;   // clear ClusterArgs::counts at kernel start
 
 struct ForwardArgs {
     const float* w;          // [n,256] tiles, or (ld > 0) a 16-row block of a row-major matrix
@@ -281,15 +282,68 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_kernel(const ForwardArgs a)
     }
 }
 
+// The walk back over a pass (tcq_walk.cuh, tcq_traceback.cu).
+struct TracebackArgs {
+    const unsigned char* bp;   // [n][bp_steps][E*K/8] packed backpointers of the LAST bp_steps steps, or nullptr with `rows`
+    const float* rows;         // [n][nrows][E] metric rows (MetricRows) of the cluster step kernel, or nullptr
+    int nrows;
+    int other_order;           // the rows' ancestors lie as in MetricRows::other_pos
+    const float* w;            // with `rows`: the pass's weights, as its ForwardArgs gave them
+    const float* w_add;
+    int roll;
+    const int* overlap;        // with `rows`: the pass's forced edge, or nullptr (unconstrained)
+    long long n;               // tiles
+    int bp_steps;              // steps walked: 256 (whole pass), 128 (second half only), or with `rows` any part of 64 steps or more
+    int t_end;                 // the walk starts after step t_end - 1 (256 unless a part of a pass is walked)
+    int codebook;              // used for dq
+    const int* e_start;        // [n] edge after step t_end - 1 (argmin edge, or the forced overlap); or nullptr with `keys`
+    const unsigned long long* keys;  // [n][nkeys] partial minima (metric bits << 32 | edge) whose smallest gives the start edge
+    int nkeys;
+    int* e_out;                // [n] out: edge BEFORE the first walked step (the overlap when bp_steps = 128), or nullptr; may be e_start
+    long long* states;         // [n,256] out (only the walked steps are written), or nullptr
+    long long* bits;           // [n,256] out: state & (2^K - 1), or nullptr
+    float* dq;                 // [n,256] out: codebook value of each state, or nullptr
+    uint32_t* packed;          // [n][packed_stride] out: exporter word layout, 8K words per tile (needs bp_steps = 256), or nullptr
+    long long packed_stride;   // words from one tile's packed codes to the next tile's (>= 8K)
+    // LDLQ row-block outputs (need bp_steps = 256); all three share the layout [16][ld], tile i = columns 16i..16i+15
+    float* wq;                 // out: reconstruction, or nullptr
+    float* err;                // out: src - reconstruction, or nullptr
+    const float* src;          // in: the uncompensated block (read only when err != nullptr)
+    long long ld;              // 0: tiles
+    // after a sweep with fused candidates (StepForm)
+    int fused;
+    float* sse;                // [n] out: the path's cost, or nullptr (whole passes tied to the overlap only)
+    int* again;                // out: tiles that have to be swept again with every operation rounded, in no order, first_tile added, and
+    int* again_count;          // their number
+    int first_tile;
+};
+
+// How the cluster kernel forms a candidate, (w - c)^2 + metric.
+//   kRounded  every operation rounded by itself, the encoder's definition.
+//   kFused    the square and the sum as one multiply-add: two fp32 instructions where there were three.  The metrics then differ from
+//             the defined ones by a few ulp, within a bound that the walk knows: where no other path comes within it of the one
+//             it is on, the path is the defined one, and where one does the walk settles it with rounded sums or lists the tile (tcq_walk.cuh).
+//   kListed   rounded, for the tiles that walks have listed, with the walk in the same kernel: one cluster takes a tile at a time.
+enum class StepForm : int { kRounded, kFused, kListed };
+
 // Cluster kernel (tcq_forward_cluster.cuh): the pass, and where its metric rows and final minima go.
 struct ClusterArgs {
     ForwardArgs f;              // bp, bp_steps and e_final are not used
-    float* rows;                // [n][nrows][E] out: metric rows (MetricRows), the last nrows of the pass
+    float* rows;                // [n][nrows][E] out: metric rows (MetricRows), the last nrows of the pass (kListed: those of one tile per cluster)
     int nrows;
-    unsigned long long* keys;   // [n][C] out: per-CTA (metric bits << 32 | edge) minima of the final metrics, or nullptr
+    unsigned long long* keys;   // [n][C] out: per-CTA (metric bits << 32 | edge) minima of the final metrics, or nullptr (kFused: [n][C][kFusedKeys])
     int at_once;                // launches: how many such clusters the device runs at once (the grid is no larger)
     int* query;                 // host, with f.n == 0: receives that number, 0 if the device cannot schedule such a cluster
+    StepForm form;
+    int* counts;                // kFused with kFwdResetCounts: two words to clear
+    const int* list;            // kListed: the tiles, and how many (f.n: the most that the grid is made for)
+    const int* list_count;
+    TracebackArgs walk;         // kListed: the walk's arguments but for rows and keys
 };
+// kFused leaves of each CTA's final metrics the minimum and up to three others that may be the minimum of the defined ones; the
+// last word is kTooMany if there are more.
+constexpr int kFusedKeys = 4;
+constexpr unsigned long long kTooMany = ~0ull - 1;
 
 // Host-side launchers, implemented once per K in tcq_forward_k{2,3,4}.cu.
 // Cluster form: clusters of C CTAs that advance G tiles.  With f.n == 0 nothing is launched: it asks how many the device

@@ -8,8 +8,15 @@
 // formed at all: one edge of 2^(16-K) per step lies on the path that the traceback walks, so the
 // argmin is worth having for that one only.  Every D-th step's path metrics go to HBM instead of every
 // step's argmins, and the traceback re-derives the D argmins between two such rows from the
-// Q^D metrics its edge can have come from (tcq_traceback.cu), with the same operations in the same
+// Q^D metrics its edge can have come from (tcq_walk.cuh), with the same operations in the same
 // order, so that the codes are those of the recorded argmins bit for bit.
+//
+// Three forms (StepForm).  What bounds a large batch is the fp32 pipe: subtract, square, add for each of 65536 states, tile and
+// step, 29.3 clocks per eight candidates and warp in registers alone.  kFused makes the square and the sum one operation, 21.7
+// clocks, and leaves it to the walk to find the path of the rounded sums (sweeps of 296 / 370 / 444 tiles: K = 3 566 / 697 / 806 -> 468 / 562 / 671 us,
+// K = 4 559 / 696 / 817 -> 477 / 569 / 674; what limits it then is operands of packed instructions as well as issue: fewer
+// instructions with the same operands are no faster).  kListed is the rounded form for the tiles that walks have listed, one at a time
+// on four SMs, with the walk behind it in the same launch: 3 us when there is none, 0.17 ms for a few.
 //
 //   * CTA r owns the butterflies h in [r * HN/C, (r+1) * HN/C): it needs the path metrics
 //     old[q * HN + h] for all q (E/C values per tile, in ITS shared memory, layout [Q][HN/C])
@@ -40,7 +47,7 @@
 
 #include <type_traits>
 
-#include "tcq_forward.cuh"
+#include "tcq_walk.cuh"
 
 namespace tcq {
 
@@ -263,8 +270,9 @@ constexpr size_t cluster_smem_bytes() {
 }
 
 // GA, GB: tiles of the two sets that alternate (GB = 0: one set, for the smallest batches).
-template <int K, int CB, int C, int GA, int GB, int NT>
+template <int K, int CB, int C, int GA, int GB, int NT, StepForm F>
 __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const ClusterArgs ca) {
+    static_assert(F != StepForm::kListed || (GA == 1 && GB == 0), "one listed tile at a time");
     using GE = Geo<K>;
     using MR = MetricRows<K>;
     using IT = ClusterItem<K, C, NT>;
@@ -317,7 +325,8 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
             cbv[i][j] = pack2(cb_from_x<CB>(xb + uint32_t((2 * j) * E) * MUL), cb_from_x<CB>(xb + uint32_t((2 * j + 1) * E) * MUL));
     }
 
-    const long long ngroups = (a.n + G - 1) / G;
+    const long long n = F == StepForm::kListed ? (long long)*ca.list_count : a.n;
+    const long long ngroups = (n + G - 1) / G;
     const long long nclusters = gridDim.x / C;
     const long long cluster_id = blockIdx.x / C;
 
@@ -356,7 +365,14 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
         // tile's own beginning.  How far ahead is a matter of registers: from the start where the item is a part of a
         // butterfly (K = 4), in the tile's second half with two tiles a set at K = 3 (558 us for 256 tiles, 577 from the
         // end), at the end otherwise (804 us for 444 tiles with three a set; 847 and spills in the second half).
-        constexpr int kAhead = LU < Q ? 0 : GS == 2 && K == 3 ? R * 5 / 8 : R - 1;
+        // With fused candidates at K = 3: in the second half for the shapes with three a set (444 tiles 672 us, from the start 704, from the
+        // end 722), early with two (296 tiles 469 us, in the second half 488).
+                // Alone on its two SMs a tile at K = 2 has them one edge earlier (74 tiles 264 us, 273 at the end; more tiles: no difference).
+        constexpr int kAhead = LU < Q                                ? 0
+                               : F == StepForm::kFused && K == 3     ? (GA == 3 ? 5 : 2)
+                               : F == StepForm::kRounded && GS == 2 && K == 3 ? R * 5 / 8
+                               : F == StepForm::kRounded && G == 1 && C == 2 && K == 2 ? R - 2
+                                                                     : R - 1;
         float cin[2][Q][HB];
 #pragma unroll
         for (int q = 0; q < Q; ++q) ld_metrics<HB>(src + (T0 * 2 + CUR) * EC + q * HNC, cin[0][q]);
@@ -368,8 +384,10 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                 constexpr int i = decltype(ic)::value;
                 float c[Q];
 #pragma unroll
-                for (int j = 0; j < Q / 2; ++j)
-                    unpack2(cand_cost2(w2[g], cbv[it * R + i][j], pack2(cin[gi & 1][2 * j][i / LU], cin[gi & 1][2 * j + 1][i / LU]), one2), c[2 * j], c[2 * j + 1]);
+                for (int j = 0; j < Q / 2; ++j) {
+                    const f32x2 from = pack2(cin[gi & 1][2 * j][i / LU], cin[gi & 1][2 * j + 1][i / LU]);
+                    unpack2(F == StepForm::kFused ? fused_cost2(w2[g], cbv[it * R + i][j], from) : cand_cost2(w2[g], cbv[it * R + i][j], from, one2), c[2 * j], c[2 * j + 1]);
+                }
                 if constexpr (i == kAhead && NX < GS * NI) {
 #pragma unroll
                     for (int q = 0; q < Q; ++q) ld_metrics<HB>(src + ((T0 + NX / NI) * 2 + CUR) * EC + NX % NI * PL::ITEM_SLOT + q * HNC, cin[NX & 1][q]);
@@ -414,6 +432,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     };
 
     if ((a.flags & kFwdResetStatus) && blockIdx.x == 0 && tid == 0 && a.status != nullptr) atomicExch(a.status, 0u);
+    if (F == StepForm::kFused && (a.flags & kFwdResetCounts) && blockIdx.x == 0 && tid < 2) ca.counts[tid] = 0;
 
     // ---- mbarriers: the arrivals of the re-arming thread and of every warp (its local stores) plus the bytes of the remote
     //      stores, per phase ----
@@ -430,9 +449,10 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     }
 
     for (long long grp = cluster_id; grp < ngroups; grp += nclusters) {
-        const long long tile0 = grp * G;
-        live = int(a.n - tile0 < G ? a.n - tile0 : G);
-        row_tile0 = ca.rows + size_t(tile0) * ca.nrows * E;
+        const long long tile0 = F == StepForm::kListed ? (long long)ca.list[grp] : grp * G;
+        const long long slot0 = F == StepForm::kListed ? cluster_id : tile0;       // whose rows and keys
+        live = F == StepForm::kListed ? 1 : int(n - tile0 < G ? n - tile0 : G);
+        row_tile0 = ca.rows + size_t(slot0) * ca.nrows * E;
         // ---- weights and initial metrics (src/trellis/qtip.py:161-165) ----
         for (int i = tid; i < G * kT; i += NT) {
             int t = i & 255;
@@ -480,10 +500,16 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
             for (int g = 0; g < G; ++g) {
                 const float* fv = cost + (size_t(g) * 2) * EC;
                 unsigned long long key = ~0ull;
-                for (int i = tid; i < EC; i += NT) {
+                auto take = [&](int i) {
                     const unsigned edge = unsigned(i / HNC) * HN + PL::butterfly(rank, i % HNC);
                     const unsigned long long k2 = (static_cast<unsigned long long>(__float_as_uint(fv[i])) << 32) | edge;
                     key = k2 < key ? k2 : key;
+                };
+                if constexpr (F == StepForm::kFused) {     // (unrolled, it takes registers from the step: 370 tiles at K = 3 586 us instead of 567)
+#pragma unroll 1
+                    for (int i = tid; i < EC; i += NT) take(i);
+                } else {
+                    for (int i = tid; i < EC; i += NT) take(i);
                 }
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) {
@@ -499,15 +525,39 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                         const unsigned long long o = __shfl_xor_sync(0xffffffffu, k2, off);
                         k2 = o < k2 ? o : k2;
                     }
-                    if (tid == 0 && g < live) ca.keys[(tile0 + g) * C + rank] = k2;
+                    if (F != StepForm::kFused && tid == 0 && g < live) ca.keys[(slot0 + g) * C + rank] = k2;
+                    if (F == StepForm::kFused && tid < kFusedKeys) red[48 + tid] = tid == 0 ? k2 : ~0ull;
+                    if (F == StepForm::kFused && tid == 0) red[56] = 0;
                 }
                 __syncthreads();
+                if constexpr (F == StepForm::kFused) {     // and who may be below it by the defined sums
+                    const float limit = fused_limit(__uint_as_float(unsigned(red[48] >> 32)), kT);
+#pragma unroll 1
+                    for (int i = tid; i < EC; i += NT)
+                        if (!(fv[i] > limit)) {
+                            const unsigned edge = unsigned(i / HNC) * HN + PL::butterfly(rank, i % HNC);
+                            if (edge == unsigned(red[48])) continue;
+                            const unsigned at = atomicAdd(reinterpret_cast<unsigned*>(red + 56), 1u) + 1;
+                            if (at < kFusedKeys) red[48 + at] = (static_cast<unsigned long long>(__float_as_uint(fv[i])) << 32) | edge;
+                        }
+                    __syncthreads();
+                    if (tid < kFusedKeys && g < live)
+                        ca.keys[((slot0 + g) * C + rank) * kFusedKeys + tid] = tid == kFusedKeys - 1 && *reinterpret_cast<unsigned*>(red + 56) >= kFusedKeys ? kTooMany : red[48 + tid];
+                    __syncthreads();
+                }
             }
         }
         if (a.final_cost != nullptr && constrained && tid < live) {
             const int ov = a.overlap[tile0 + tid] & (E - 1);
             const int qo = ov / HN, ho = ov % HN;
             if (PL::owner(ho) == rank) a.final_cost[tile0 + tid] = cost[(size_t(tid) * 2) * EC + qo * HNC + PL::slot(ho)];
+        }
+        if constexpr (F == StepForm::kListed) {
+            __shared__ WalkShared<K, false> walk_shared;
+            __threadfence();                        // the rows and keys of every CTA, before one of them walks
+            cluster.sync();
+            if (rank == 0 && tid < WalkShape<K>::W * 32) walk_tile<K, CB, false, false, true>(ca.walk, tile0, slot0, walk_shared);
+            __syncwarp();
         }
         cluster.sync();   // nobody may start re-initialising while a neighbour still reads or is written to
     }

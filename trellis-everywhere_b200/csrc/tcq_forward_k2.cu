@@ -8,6 +8,7 @@ template <int CB>
 cudaError_t launch_cluster_cb(const ClusterArgs& ca, int C, int G, cudaStream_t stream) {
     // The shapes of pick_cluster.  Clusters of eight have 512 threads here (16 states each) and 256 at K = 3 and 4 (32 states):
     // 9 to 30 tiles 8 % faster at K = 2 (24 tiles 421 -> 388 us a call), 7-20 % slower for one tile at K = 3 and 4.
+    if (ca.form != StepForm::kRounded) return cudaErrorInvalidValue;
     switch (100 * C + G) {
         case 1601: return launch_cluster_variant<2, CB, 16, 1, 0, 256>(ca, stream);
         case 801: return launch_cluster_variant<2, CB, 8, 1, 0, 512>(ca, stream);

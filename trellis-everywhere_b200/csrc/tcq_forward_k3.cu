@@ -6,6 +6,17 @@ namespace tcq {
 namespace {
 template <int CB>
 cudaError_t launch_cluster_cb(const ClusterArgs& ca, int C, int G, cudaStream_t stream) {
+    if (ca.form == StepForm::kListed) return launch_cluster_variant<3, CB, 4, 1, 0, 512, StepForm::kListed>(ca, stream);
+    if (ca.form == StepForm::kFused)
+        switch (G) {
+            case 1: return launch_cluster_variant<3, CB, 2, 1, 0, 512, StepForm::kFused>(ca, stream);
+            case 2: return launch_cluster_variant<3, CB, 2, 1, 1, 512, StepForm::kFused>(ca, stream);
+            case 3: return launch_cluster_variant<3, CB, 2, 2, 1, 512, StepForm::kFused>(ca, stream);
+            case 4: return launch_cluster_variant<3, CB, 2, 2, 2, 512, StepForm::kFused>(ca, stream);
+            case 5: return launch_cluster_variant<3, CB, 2, 3, 2, 512, StepForm::kFused>(ca, stream);
+            case 6: return launch_cluster_variant<3, CB, 2, 3, 3, 512, StepForm::kFused>(ca, stream);
+            default: return cudaErrorInvalidValue;
+        }
     switch (100 * C + G) {                       // the shapes of pick_cluster
         case 801: return launch_cluster_variant<3, CB, 8, 1, 0, 256>(ca, stream);
         case 802: return launch_cluster_variant<3, CB, 8, 1, 1, 256>(ca, stream);

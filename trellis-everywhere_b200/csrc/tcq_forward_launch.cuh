@@ -48,9 +48,9 @@ constexpr size_t kOneCtaPerSm = 116 * 1024;        // dynamic shared memory of w
 
 // Cluster form with clusters of C CTAs and tile sets of GA and GB.  A launch uses at most as many clusters as the device runs at
 // once, which depends on C only (one CTA fills an SM in every instantiation) and is asked for in a call of its own.
-template <int K, int CB, int C, int GA, int GB, int NT>
+template <int K, int CB, int C, int GA, int GB, int NT, StepForm F = StepForm::kRounded>
 static cudaError_t launch_cluster_variant(const ClusterArgs& ca, cudaStream_t stream) {
-    auto kern = tcq_forward_cluster_kernel<K, CB, C, GA, GB, NT>;
+    auto kern = tcq_forward_cluster_kernel<K, CB, C, GA, GB, NT, F>;
     // Never less than half of what an SM has: two small CTAs on one SM leave another SM idle, and a step takes as long as
     // the slowest CTA of its cluster.
     constexpr size_t need = cluster_smem_bytes<K, C, GA, GB>(), smem = need < kOneCtaPerSm ? kOneCtaPerSm : need;

@@ -1,4 +1,5 @@
-// Traceback kernel: walks the packed backpointers written by the Viterbi step
+// Traceback kernels.  tcq_walk_kernel is the walk over the metric rows of the cluster step kernel (tcq_walk.cuh);
+// tcq_traceback_kernel walks the packed backpointers written by the single-CTA Viterbi step
 // kernel from the last step to the first and emits, per tile, the state path and
 // everything derived from it (symbols, packed code words, reconstruction).
 //
@@ -18,6 +19,7 @@
 #include <type_traits>
 
 #include "tcq_traceback.cuh"
+#include "tcq_walk.cuh"
 
 namespace tcq {
 
@@ -36,46 +38,6 @@ __device__ __forceinline__ uint32_t bp_entry(const unsigned char* row, uint32_t 
     const uint32_t b1 = b0 + 1 < ROWB ? b0 + 1 : b0;
     const uint32_t v = uint32_t(row[b0]) | (uint32_t(row[b1]) << 8);
     return (v >> (bit & 7)) & (Q - 1);
-}
-
-// Outputs of one tile over the steps that were walked, by NT threads, from the states in shared memory.
-template <int K, int NT>
-__device__ __forceinline__ void emit_outputs(const TracebackArgs& a, long long tile, const uint16_t* st, int t_off, int t_end, int tid) {
-    constexpr uint32_t Q = Geo<K>::Q;
-    if (a.states != nullptr)
-        for (int t = t_off + tid; t < t_end; t += NT) a.states[tile * kT + t] = (long long)st[t];
-    if (a.bits != nullptr)
-        for (int t = t_off + tid; t < t_end; t += NT) a.bits[tile * kT + t] = (long long)(st[t] & (Q - 1));
-    if (a.dq != nullptr)
-        for (int t = t_off + tid; t < t_end; t += NT) a.dq[tile * kT + t] = cb_value_rt(a.codebook, st[t]);
-    if (a.wq != nullptr) {
-        // LDLQ row-block layout (src/trellis/ldlq.py:142-143): weight t of this tile is element
-        // [t & 15][16 * tile + (t >> 4)] of a 16-row block; j walks along the matrix rows so that a
-        // half-warp writes 64 contiguous bytes.  err = src - reconstruction is the block error the
-        // recursion feeds back (ldlq.py:90,97), formed here instead of by a separate pass over the block.
-        for (int j = tid; j < kT; j += NT) {
-            const int t = ((j & 15) << 4) | (j >> 4);
-            if (t < t_off || t >= t_end) continue;
-            const float v = cb_value_rt(a.codebook, st[t]);
-            const long long off = (long long)(j >> 4) * a.ld + tile * 16 + (j & 15);
-            a.wq[off] = v;
-            if (a.err != nullptr) a.err[off] = __fsub_rn(a.src[off], v);
-        }
-    }
-    if (a.packed != nullptr) {
-        // (whole words: a part of a pass is a multiple of 64 steps)
-        // word j holds stream bits 32j .. 32j+31; stream bit p is bit (p % K) of symbol 255 - p / K
-        for (uint32_t j = uint32_t(kT - t_end) * K / 32 + tid; j < uint32_t(kT - t_off) * K / 32; j += NT) {
-            uint32_t word = 0;
-#pragma unroll 8
-            for (uint32_t b = 0; b < 32; ++b) {
-                const uint32_t p = 32 * j + b;
-                const uint32_t t = (kT - 1) - p / K;
-                word |= ((uint32_t(st[t]) >> (p % K)) & 1u) << b;
-            }
-            a.packed[tile * a.packed_stride + j] = word;
-        }
-    }
 }
 
 template <int K, int DEPTH>
@@ -159,201 +121,21 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) tcq_traceback_kernel(const 
     emit_outputs<K, 32>(a, tile, st, t_off, kT, lane);
 }
 
-// Walk over metric rows (MetricRows, left by the cluster step kernel): one CTA of W warps per tile.
-//
-// Per trip the walk takes D steps back.  It reads the NA = Q^D metrics, contiguous in the row, that the current edge can
-// have come from, forms the candidates of the first of the D steps for the Q^(D-1) nodes above them exactly as the step
-// kernel does (same operations, same order, lowest q among equals), and so on up the tree to the current edge; each node
-// carries the q's chosen below it, so the root holds the whole path.  Candidates per step and tile, those that warps and lanes form
-// more than once included: 1/100, 1/180, 1/450 of the step kernel's (K = 2, 3, 4).
-//
-// What bounds it is the latency of one trip, whose address the trip before decides.  So the first level is spread over
-// the CTA (one barrier per trip, two buffers); the other levels are small and every warp does them for itself; and the
-// emission costs of all levels, which depend on the edge only, are formed while the metrics are on their way.
-template <int K> struct WalkShape {
-    static constexpr int W = K == 2 ? 4 : K == 3 ? 2 : 1;      // warps
-    static constexpr int SPLIT = K == 4 ? 2 : 1;               // lanes that share a first-level node
-};
-
-// Lowest q whose candidate is the minimum (Q-1 if no candidate compares equal: not-a-number weights), as the step kernels choose.
-template <int N>
-__device__ __forceinline__ uint32_t first_minimum(const float (&c)[N], float best) {
-    uint32_t qb = N - 1;
-#pragma unroll
-    for (int q = N - 2; q >= 0; --q) qb = c[q] == best ? uint32_t(q) : qb;
-    return qb;
+// One CTA of WalkShape<K>::W warps per tile, twice as many after fused sweeps (tcq_walk.cuh).
+// (six CTAs on an SM: 888 tiles walk at once)
+template <int K, int CB, bool OTHER, bool FUSED>
+__global__ void __launch_bounds__(WalkShape<K>::W * (FUSED ? 64 : 32), FUSED ? 6 : 1) tcq_walk_kernel(const TracebackArgs a) {
+    __shared__ WalkShared<K, FUSED> sh;
+    walk_tile<K, CB, OTHER, FUSED, false>(a, blockIdx.x, blockIdx.x, sh);
 }
 
-// OTHER: the rows' ancestors lie as in MetricRows::other_pos.
-template <int K, int CB, bool OTHER>
-__global__ void __launch_bounds__(WalkShape<K>::W * 32) tcq_walk_kernel(const TracebackArgs a) {
-    using GE = Geo<K>;
-    using MR = MetricRows<K>;
-    constexpr uint32_t Q = GE::Q, E = GE::E;
-    constexpr int SH = kL - K, D = MR::D, LB = MR::LB, NA = MR::NA;
-    constexpr int W = WalkShape<K>::W, NT = W * 32, SPLIT = WalkShape<K>::SPLIT;
-    constexpr int N1 = NA / int(Q);                // first-level nodes
-    constexpr int NPT = N1 * SPLIT / NT;           // ... per thread
-    constexpr int QS = int(Q) / SPLIT;             // candidates of a node that one thread forms
-    constexpr int N2 = D >= 3 ? N1 / int(Q) : 1;   // second-level nodes
-    constexpr int NP2 = N2 > 32 ? N2 / 32 : 1;     // ... per lane
-    static_assert(NPT * NT == N1 * SPLIT && (SPLIT == 1 || (W == 1 && N1 * SPLIT == 32)), "first-level nodes must divide over the threads");
-    __shared__ uint16_t st[kT];
-    __shared__ float wv_pad[kT + 8];               // by step; the first trip may also look (in vain) at the steps before 0
-    float* const wv = wv_pad + 8;
-    __shared__ float val1[2][N1];                  // first level: minima and their q, double buffered over trips
-    __shared__ uint32_t path1[2][N1];
-    __shared__ float val[W][D > 2 ? D - 2 : 1][N2];       // levels 2 .. D-1, one copy per warp
-    __shared__ uint32_t path[W][D > 2 ? D - 2 : 1][N2];
-    const int tid = threadIdx.x, lane = tid & 31, wrp = tid >> 5;
-    const long long tile = blockIdx.x;
-
-    ForwardArgs fw{};
-    fw.w = a.w;
-    fw.w_add = a.w_add;
-    fw.ld = a.ld;
-    for (int i = tid; i < kT; i += NT) {
-        int t;
-        const float x = load_weight(fw, tile, i, t);
-        wv[(t - a.roll) & (kT - 1)] = x;
-    }
-    if (tid < 8) wv_pad[tid] = 0.0f;
-    uint32_t e;
-    if (a.keys != nullptr) {            // argmin of the final metrics, left as per-CTA partial minima by the step kernel
-        unsigned long long k = a.keys[tile * a.nkeys];
-        for (int i = 1; i < a.nkeys; ++i) {
-            const unsigned long long o = a.keys[tile * a.nkeys + i];
-            k = o < k ? o : k;
-        }
-        e = uint32_t(k) & (E - 1);
-    } else {
-        e = uint32_t(a.e_start[tile]) & (E - 1);
-    }
-    const uint32_t ov = a.overlap != nullptr ? uint32_t(a.overlap[tile]) & (E - 1) : ~0u;
-    // metric of edge x before step 0
-    auto start_metric = [&](uint32_t x) { return a.overlap == nullptr ? 0.0f : x == ov ? 0.0f : __uint_as_float(kInfBits); };
-    const int t_off = a.t_end - a.bp_steps;
-    const float* const rows = a.rows + size_t(tile) * a.nrows * E;
-    __syncthreads();
-
-    // emission cost of state (q, y) at weight w
-    auto emission = [](float w, uint32_t q, uint32_t y) {
-        const float d = __fsub_rn(w, cb_value<CB>((q << SH) | y));
-        return __fmul_rn(d, d);
-    };
-    int tau = a.t_end - D;                              // first of the trip's D steps
-    // metric(q * N1, p): the metric of ancestor q * N1 + p before step tau.  kFirst: the trip that holds step 0; nodes before step 0 have the start
-    // metric of their edge.
-    auto trip = [&](int buf, auto first_c, auto metric) {
-        constexpr bool kFirst = decltype(first_c)::value;
-        float c1[NPT][QS];
-#pragma unroll
-        for (int i = 0; i < NPT; ++i)
-#pragma unroll
-            for (int k = 0; k < QS; ++k) {
-                const uint32_t q = uint32_t(k + (SPLIT > 1 ? lane / N1 * QS : 0));
-                c1[i][k] = metric(q * N1, uint32_t(tid + i * NT) % N1);
-            }
-        // the emissions of every level, under the loads
-        float em1[NPT][QS], em[D - 1][NP2][Q], em_root;
-#pragma unroll
-        for (int i = 0; i < NPT; ++i)
-#pragma unroll
-            for (int k = 0; k < QS; ++k) {
-                const uint32_t q = uint32_t(k + (SPLIT > 1 ? lane / N1 * QS : 0)), p = uint32_t(tid + i * NT) % N1;
-                em1[i][k] = emission(wv[tau], q, (p << (LB + K)) | (e >> ((D - 1) * K)));
-            }
-#pragma unroll
-        for (int d = 2; d < D; ++d) {
-            const int M = 1 << ((D - d) * K);      // nodes of this level
-#pragma unroll
-            for (int i = 0; i < (M > 32 ? M / 32 : 1); ++i)
-#pragma unroll
-                for (uint32_t q = 0; q < Q; ++q)
-                    em[d - 2][i][q] = emission(wv[tau + d - 1], q, (uint32_t((lane + 32 * i) & (M - 1)) << (LB + d * K)) | (e >> ((D - d) * K)));
-        }
-        em_root = emission(wv[tau + D - 1], uint32_t(lane) & (Q - 1), e);
-
-        // first level
-#pragma unroll
-        for (int i = 0; i < NPT; ++i) {
-#pragma unroll
-            for (int k = 0; k < QS; ++k) c1[i][k] = __fadd_rn(em1[i][k], c1[i][k]);
-            float best = min_of<QS>(c1[i]);
-            uint32_t qb = first_minimum<QS>(c1[i], best);
-            if constexpr (SPLIT == 2) {
-                const float bo = __shfl_xor_sync(0xffffffffu, best, N1);
-                const uint32_t qo = __shfl_xor_sync(0xffffffffu, qb, N1);
-                const bool upper = lane >= N1;
-                const float b0 = upper ? bo : best, b1 = upper ? best : bo;
-                const uint32_t q0 = upper ? qo : qb, q1 = (upper ? qb : qo) + QS;
-                best = fminf(b0, b1);
-                qb = b0 == best ? q0 : b1 == best ? q1 : Q - 1;
-            }
-            const int p = (tid + i * NT) % N1;
-            if constexpr (kFirst)
-                if (tau < 0) best = start_metric((uint32_t(p) << (LB + K)) | (e >> ((D - 1) * K)));
-            val1[buf][p] = best;
-            path1[buf][p] = qb;
-        }
-        if constexpr (W > 1) __syncthreads();
-        else __syncwarp();
-        const float* vin = val1[buf];
-        const uint32_t* pin = path1[buf];
-#pragma unroll
-        for (int d = 2; d < D; ++d) {
-            const int M = 1 << ((D - d) * K);
-#pragma unroll
-            for (int i = 0; i < (M > 32 ? M / 32 : 1); ++i) {
-                const uint32_t p = uint32_t((lane + 32 * i) & (M - 1));
-                float c[Q];
-#pragma unroll
-                for (uint32_t q = 0; q < Q; ++q) c[q] = __fadd_rn(em[d - 2][i][q], vin[q * uint32_t(M) + p]);
-                float best = min_of<int(Q)>(c);
-                const uint32_t qb = first_minimum<int(Q)>(c, best);
-                if constexpr (kFirst)
-                    if (tau + d - 1 < 0) best = start_metric((p << (LB + d * K)) | (e >> ((D - d) * K)));
-                val[wrp][d - 2][p] = best;
-                path[wrp][d - 2][p] = pin[qb * uint32_t(M) + p] | (qb << ((d - 1) * K));
-            }
-            __syncwarp();
-            vin = val[wrp][d - 2];
-            pin = path[wrp][d - 2];
-        }
-        // the root: one candidate per lane.  Candidates are non-negative (or not a number), so their bits order like the values.
-        const float c = __fadd_rn(em_root, vin[uint32_t(lane) & (Q - 1)]);
-        const float best = __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(c)));
-        const uint32_t eq = __ballot_sync(0xffffffffu, c == best);
-        const uint32_t qb = eq != 0 ? uint32_t(__ffs(int(eq)) - 1) : Q - 1;
-        const uint32_t whole = pin[qb] | (qb << ((D - 1) * K));       // q of step tau + i at bits i*K
-#pragma unroll
-        for (int i = D - 1; i >= 0; --i) {
-            const uint32_t s = (((whole >> (i * K)) & (Q - 1)) << SH) | e;
-            if (tid == 0 && (!kFirst || tau + i >= 0)) st[tau + i] = uint16_t(s);
-            e = s >> K;
-        }
-    };
-    int j = 0;
-    for (; tau > 0 && tau + D > t_off; ++j, tau -= D) {
-        const float* const row = rows + size_t(j) * E + (e >> (K * D)) * uint32_t(NA);     // the ancestors share the edge's bits above K*D
-        trip(j & 1, std::false_type{}, [&](uint32_t pq, uint32_t p) { return __ldg(row + (OTHER ? MR::order(pq) | MR::order(p) : pq | p)); });
-    }
-    if (tau + D > t_off) {                         // tau <= 0
-        const uint32_t g = e >> (K * D);
-        trip(j & 1, std::true_type{}, [&](uint32_t pq, uint32_t p) { return start_metric(((pq + p) << LB) | g); });
-    }
-    __syncthreads();
-    if (tid == 0 && a.e_out != nullptr) a.e_out[tile] = int(st[t_off] >> K);     // a trip may have gone past step t_off
-    emit_outputs<K, NT>(a, tile, st, t_off, a.t_end, tid);
-}
-
-template <int K, bool OTHER>
+template <int K, bool OTHER, bool FUSED>
 cudaError_t launch_walk(const TracebackArgs& a, cudaStream_t stream) {
-    const unsigned grid = unsigned(a.n), block = WalkShape<K>::W * 32;
+    const unsigned grid = unsigned(a.n), block = WalkShape<K>::W * (FUSED ? 64 : 32);
     switch (a.codebook) {
-        case kCb1Mad:  tcq_walk_kernel<K, kCb1Mad, OTHER><<<grid, block, 0, stream>>>(a); break;
-        case kCb3Inst: tcq_walk_kernel<K, kCb3Inst, OTHER><<<grid, block, 0, stream>>>(a); break;
-        case kCbMcg:   tcq_walk_kernel<K, kCbMcg, OTHER><<<grid, block, 0, stream>>>(a); break;
+        case kCb1Mad:  tcq_walk_kernel<K, kCb1Mad, OTHER, FUSED><<<grid, block, 0, stream>>>(a); break;
+        case kCb3Inst: tcq_walk_kernel<K, kCb3Inst, OTHER, FUSED><<<grid, block, 0, stream>>>(a); break;
+        case kCbMcg:   tcq_walk_kernel<K, kCbMcg, OTHER, FUSED><<<grid, block, 0, stream>>>(a); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -366,9 +148,9 @@ cudaError_t launch_traceback(int K, const TracebackArgs& a, cudaStream_t stream)
     const unsigned grid = unsigned((a.n + kWarpsPerCta - 1) / kWarpsPerCta);
     if (a.rows != nullptr) {
         switch (K) {
-            case 2: return launch_walk<2, false>(a, stream);
-            case 3: return a.other_order ? launch_walk<3, true>(a, stream) : launch_walk<3, false>(a, stream);
-            case 4: return launch_walk<4, false>(a, stream);
+            case 2: return launch_walk<2, false, false>(a, stream);
+            case 3: return a.fused ? launch_walk<3, true, true>(a, stream) : a.other_order ? launch_walk<3, true, false>(a, stream) : launch_walk<3, false, false>(a, stream);
+            case 4: return a.fused ? launch_walk<4, false, true>(a, stream) : launch_walk<4, false, false>(a, stream);
             default: return cudaErrorInvalidValue;
         }
     }
