@@ -504,8 +504,8 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
         avg_kernel_ms = sum(kern_ms) / 2
         evals_per_launch = chunk * T_SEQ * 65536
         achieved = evals_per_launch * LANE_OPS_PER_EVAL / (avg_kernel_ms * 1e-3)
-        # metric rows of every 5th / 3rd / 2nd step, 4 bytes an edge: mean of the two passes
-        row_bytes = chunk * {2: (26 + 51) / 2, 3: (43 + 85) / 2, 4: (64 + 127) / 2}[K_BITS] * (1 << (16 - K_BITS)) * 4
+        # metric rows of every 5th / 3rd / 2nd step, 4 bytes an edge: mean of the two passes (with fused candidates both leave those of all steps)
+        row_bytes = chunk * {2: (26 + 51) / 2, 3: 85, 4: 127}[K_BITS] * (1 << (16 - K_BITS)) * 4
         ck = clocks.summary()
         roofline = {
             "bound": "alu", "kernel": f"Viterbi step kernel (tcq_forward_cluster_kernel, K={K_BITS}, {CODEBOOK}, 2 CTAs per cluster)",

@@ -201,7 +201,7 @@ struct Workspace {
 // tile swept again, 0.2 ms, is a larger part of a call: 148 tiles at K = 3 would gain 4 %.  At K = 2 the metric rows bind as well (a sweep of 444
 // tiles 1115 -> 1022 us), and the longer walk takes most of the gain: 150 tiles 1220 -> 1230 us a call, 1000 tiles 5431 -> 5372.
 constexpr int kFusedFrom = 149;
-constexpr int kListedC = 4;
+constexpr int kListedC = 2;                        // (with four SMs a tile, a few tiles take 0.17 ms instead of 0.25, and a batch of nothing but ties longer)
 constexpr long long kSpan = 1 << 18;               // the full-speed size holds the overlaps of so many tiles
 bool plan_fused(long long n, int K, const Workspace& wk) {
     return K >= 3 && n >= kFusedFrom && wk.part == kT && kernel_asked_for() == 0 && wk.chunk >= (n < 2 * kFusedFrom ? n : 2 * kFusedFrom) && clusters_at_once(kListedC) > 0;
@@ -408,6 +408,7 @@ int listed(int K, int codebook, ForwardArgs f, int walk, TracebackArgs t, const 
     t.overlap = t.e_start = f.overlap;
     t.keys = ca.keys;
     t.nkeys = kListedC;
+    t.other_order = K == 3;
     t.bp_steps = walk;
     t.t_end = kT;
     t.codebook = codebook;

@@ -16,7 +16,7 @@
 // clocks, and leaves it to the walk to find the path of the rounded sums (sweeps of 296 / 370 / 444 tiles: K = 3 566 / 697 / 806 -> 468 / 562 / 671 us,
 // K = 4 559 / 696 / 817 -> 477 / 569 / 674; what limits it then is operands of packed instructions as well as issue: fewer
 // instructions with the same operands are no faster).  kListed is the rounded form for the tiles that walks have listed, one at a time
-// on four SMs, with the walk behind it in the same launch: 3 us when there is none, 0.17 ms for a few.
+// on two SMs, with the walk behind it in the same launch: 3 us when there is none.
 //
 //   * CTA r owns the butterflies h in [r * HN/C, (r+1) * HN/C): it needs the path metrics
 //     old[q * HN + h] for all q (E/C values per tile, in ITS shared memory, layout [Q][HN/C])
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     }
 
     const long long n = F == StepForm::kListed ? (long long)*ca.list_count : a.n;
-    const long long ngroups = (n + G - 1) / G;
+    const long long ngroups = ((F == StepForm::kRounded ? a.n : n) + G - 1) / G;
     const long long nclusters = gridDim.x / C;
     const long long cluster_id = blockIdx.x / C;
 
@@ -385,8 +385,12 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
                 float c[Q];
 #pragma unroll
                 for (int j = 0; j < Q / 2; ++j) {
-                    const f32x2 from = pack2(cin[gi & 1][2 * j][i / LU], cin[gi & 1][2 * j + 1][i / LU]);
-                    unpack2(F == StepForm::kFused ? fused_cost2(w2[g], cbv[it * R + i][j], from) : cand_cost2(w2[g], cbv[it * R + i][j], from, one2), c[2 * j], c[2 * j + 1]);
+                    if constexpr (F == StepForm::kFused) {
+                        const f32x2 from = pack2(cin[gi & 1][2 * j][i / LU], cin[gi & 1][2 * j + 1][i / LU]);
+                        unpack2(fused_cost2(w2[g], cbv[it * R + i][j], from), c[2 * j], c[2 * j + 1]);
+                    } else {
+                        unpack2(cand_cost2(w2[g], cbv[it * R + i][j], pack2(cin[gi & 1][2 * j][i / LU], cin[gi & 1][2 * j + 1][i / LU]), one2), c[2 * j], c[2 * j + 1]);
+                    }
                 }
                 if constexpr (i == kAhead && NX < GS * NI) {
 #pragma unroll
@@ -451,7 +455,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     for (long long grp = cluster_id; grp < ngroups; grp += nclusters) {
         const long long tile0 = F == StepForm::kListed ? (long long)ca.list[grp] : grp * G;
         const long long slot0 = F == StepForm::kListed ? cluster_id : tile0;       // whose rows and keys
-        live = F == StepForm::kListed ? 1 : int(n - tile0 < G ? n - tile0 : G);
+        live = F == StepForm::kListed ? 1 : F == StepForm::kFused ? int(n - tile0 < G ? n - tile0 : G) : int(a.n - tile0 < G ? a.n - tile0 : G);
         row_tile0 = ca.rows + size_t(slot0) * ca.nrows * E;
         // ---- weights and initial metrics (src/trellis/qtip.py:161-165) ----
         for (int i = tid; i < G * kT; i += NT) {
@@ -500,16 +504,20 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
             for (int g = 0; g < G; ++g) {
                 const float* fv = cost + (size_t(g) * 2) * EC;
                 unsigned long long key = ~0ull;
-                auto take = [&](int i) {
-                    const unsigned edge = unsigned(i / HNC) * HN + PL::butterfly(rank, i % HNC);
-                    const unsigned long long k2 = (static_cast<unsigned long long>(__float_as_uint(fv[i])) << 32) | edge;
-                    key = k2 < key ? k2 : key;
-                };
                 if constexpr (F == StepForm::kFused) {     // (unrolled, it takes registers from the step: 370 tiles at K = 3 586 us instead of 567)
+                    auto take = [&](int i) {
+                        const unsigned edge = unsigned(i / HNC) * HN + PL::butterfly(rank, i % HNC);
+                        const unsigned long long k2 = (static_cast<unsigned long long>(__float_as_uint(fv[i])) << 32) | edge;
+                        key = k2 < key ? k2 : key;
+                    };
 #pragma unroll 1
                     for (int i = tid; i < EC; i += NT) take(i);
                 } else {
-                    for (int i = tid; i < EC; i += NT) take(i);
+                    for (int i = tid; i < EC; i += NT) {
+                        const unsigned edge = unsigned(i / HNC) * HN + PL::butterfly(rank, i % HNC);
+                        const unsigned long long k2 = (static_cast<unsigned long long>(__float_as_uint(fv[i])) << 32) | edge;
+                        key = k2 < key ? k2 : key;
+                    }
                 }
 #pragma unroll
                 for (int off = 16; off > 0; off >>= 1) {
@@ -556,7 +564,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
             __shared__ WalkShared<K, false> walk_shared;
             __threadfence();                        // the rows and keys of every CTA, before one of them walks
             cluster.sync();
-            if (rank == 0 && tid < WalkShape<K>::W * 32) walk_tile<K, CB, false, false, true>(ca.walk, tile0, slot0, walk_shared);
+            if (rank == 0 && tid < WalkShape<K>::W * 32) walk_tile<K, CB, K == 3 && C == 2, false, true>(ca.walk, tile0, slot0, walk_shared);
             __syncwarp();
         }
         cluster.sync();   // nobody may start re-initialising while a neighbour still reads or is written to
