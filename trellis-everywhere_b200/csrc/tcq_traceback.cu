@@ -129,8 +129,40 @@ __global__ void __launch_bounds__(WalkShape<K>::W * (FUSED ? 64 : 32), FUSED ? 6
     walk_tile<K, CB, OTHER, FUSED, false>(a, blockIdx.x, blockIdx.x, sh);
 }
 
+// The same with rows fetched ahead (Ring): from three tiles on, whose rows are far enough away for it (one or two: 270 us a call at K = 3 without, 276
+// with it; 3 / 8 / 24 / 74 tiles 288 / 289 / 391 / 506 without, 278 / 274 / 381 / 480 with it), until the bytes of all tiles bind: at K = 4 one tile
+// per SM still gains (148 tiles 819 -> 791), at K = 3, whose rows are twice as long, it loses (771 -> 781), at K = 2 from 96 on (881 -> 893; 64 tiles 602 -> 594).
+constexpr bool in_ring(int K, long long n) { return n >= 3 && n <= (K == 2 ? 74 : K == 3 ? 96 : 148); }
+template <int K, int CB, bool OTHER>
+__global__ void __launch_bounds__(WalkShape<K>::W * 32) tcq_walk_ring_kernel(const TracebackArgs a) {
+    extern __shared__ __align__(128) float walk_ring[];
+    __shared__ WalkShared<K, false> sh;
+    walk_tile<K, CB, OTHER, false, false, true>(a, blockIdx.x, blockIdx.x, sh, walk_ring);
+}
+
+template <int K, int CB, bool OTHER>
+cudaError_t launch_ring(const TracebackArgs& a, cudaStream_t stream) {
+    static bool optin[64] = {};                    // per device ordinal: the shared-memory opt-in has been made
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    if (dev < 0 || dev >= 64 || !optin[dev]) {
+        if ((err = cudaFuncSetAttribute(tcq_walk_ring_kernel<K, CB, OTHER>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(Ring<K>::kBytes))) != cudaSuccess) return err;
+        if (dev >= 0 && dev < 64) optin[dev] = true;
+    }
+    tcq_walk_ring_kernel<K, CB, OTHER><<<unsigned(a.n), WalkShape<K>::W * 32, Ring<K>::kBytes, stream>>>(a);
+    return cudaGetLastError();
+}
+
 template <int K, bool OTHER, bool FUSED>
 cudaError_t launch_walk(const TracebackArgs& a, cudaStream_t stream) {
+    if constexpr (!FUSED)
+        if (in_ring(K, a.n)) switch (a.codebook) {
+            case kCb1Mad:  return launch_ring<K, kCb1Mad, OTHER>(a, stream);
+            case kCb3Inst: return launch_ring<K, kCb3Inst, OTHER>(a, stream);
+            case kCbMcg:   return launch_ring<K, kCbMcg, OTHER>(a, stream);
+            default: return cudaErrorInvalidValue;
+        }
     const unsigned grid = unsigned(a.n), block = WalkShape<K>::W * (FUSED ? 64 : 32);
     switch (a.codebook) {
         case kCb1Mad:  tcq_walk_kernel<K, kCb1Mad, OTHER, FUSED><<<grid, block, 0, stream>>>(a); break;

@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "tcq_forward.cuh"
+#include "tcq_mbarrier.cuh"
 
 namespace tcq {
 
@@ -85,6 +86,15 @@ __device__ __forceinline__ float fused_limit(float best, int t) {
 }
 constexpr float kFusedMax = 1e37f;
 
+// A tile's rows lie one after another whatever the path, so where few tiles walk, each on an SM of its own, their CTAs fetch whole rows ahead
+// (32 KiB at K = 3) and find a trip's metrics in shared memory: the latency of L2 or HBM leaves the chain of trips.  16 times as many bytes
+// are read, 2.8 MB a tile and walk, so it is for few tiles only.
+template <int K> struct Ring {
+    static constexpr int E = Geo<K>::E, kRows = 192 * 1024 / (E * 4);
+    static constexpr size_t kBytes = size_t(kRows) * E * 4 + 16 * 8;       // rows, then an mbarrier each and the waits' flag
+    static_assert(kRows <= 14, "the flag is the sixteenth word");
+};
+
 template <int K, bool FUSED>
 struct WalkShared {
     static constexpr int D = MetricRows<K>::D, W = WalkShape<K>::W, N1 = MetricRows<K>::NA >> K, N2 = D >= 3 ? N1 >> K : 1;
@@ -122,8 +132,11 @@ struct WalkShared {
 // the trips that get marked.  Its waits for the first group are bounded by the clock.
 // What this does not settle (marks on the other path too, another winner, more than a few marks, costs above 1e37 or not a
 // number) lists the tile in a.again: one tile in 10 000, and every tile of ties, such as one of zeros.
-template <int K, int CB, bool OTHER, bool FUSED, bool COHERENT>
-__device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile, long long slot, WalkShared<K, FUSED>& sh) {
+//
+// RING: rows come to shared memory ahead of the walk; `ring` is Ring<K>::kBytes of it.
+template <int K, int CB, bool OTHER, bool FUSED, bool COHERENT, bool RING = false>
+__device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile, long long slot, WalkShared<K, FUSED>& sh, float* ring = nullptr) {
+    static_assert(!RING || !FUSED, "the second group would need rows of its own");
     using GE = Geo<K>;
     using MR = MetricRows<K>;
     constexpr uint32_t Q = GE::Q, E = GE::E;
@@ -358,7 +371,40 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
     };
     // ... where its metrics are: rows, or before step 0
     auto row_of = [&](uint32_t e, int j) { return rows + size_t(j) * E + (e >> (K * D)) * uint32_t(NA); };    // the ancestors share the edge's bits above K*D
+    [[maybe_unused]] unsigned long long* const full = reinterpret_cast<unsigned long long*>(ring + (RING ? Ring<K>::kRows * int(E) : 0));
+    [[maybe_unused]] bool lost = false;            // RING: a row did not come; the walk goes on from global memory
+    [[maybe_unused]] int ring_rows = 0;            // rows that the walk reads
+    [[maybe_unused]] auto fetch = [&](int j) {
+        const uint32_t bar = smem_u32(full + j % Ring<K>::kRows);
+        mbar_expect(bar, E * 4);
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                     ::"r"(smem_u32(ring + j % Ring<K>::kRows * int(E))), "l"(rows + size_t(j) * E), "r"(uint32_t(E) * 4), "r"(bar) : "memory");
+    };
+    if constexpr (RING) {
+        while (a.t_end - D * (ring_rows + 1) > 0 && a.t_end - D * ring_rows > t_off) ++ring_rows;
+        if (tid == 0) {
+            for (int i = 0; i < Ring<K>::kRows; ++i) mbar_init(smem_u32(full + i), 1);
+            *reinterpret_cast<unsigned int*>(full + 15) = 0;
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            for (int i = 0; i < Ring<K>::kRows && i < ring_rows; ++i) fetch(i);
+        }
+        sync();
+    }
     auto row_trip = [&](int buf, auto now_c, int tau, uint32_t e, int j) __attribute__((always_inline)) {
+        if constexpr (RING) {
+            if (!lost) {
+                const bool came = mbar_wait(smem_u32(full + j % Ring<K>::kRows), uint32_t(j / Ring<K>::kRows) & 1u, reinterpret_cast<volatile unsigned int*>(full + 15));
+                lost = __any_sync(0xffffffffu, !came);
+            }
+            if (!lost) {
+                const float* const row = ring + j % Ring<K>::kRows * int(E) + (e >> (K * D)) * uint32_t(NA);
+                const uint32_t whole = trip(buf, std::false_type{}, now_c, tau, e, [&](uint32_t pq, uint32_t p) { return row[OTHER ? MR::order(pq) | MR::order(p) : pq | p]; });
+                // every thread has its metrics: the trip's barrier lies behind it
+                if (tid == 0 && j + Ring<K>::kRows < ring_rows) fetch(j + Ring<K>::kRows);
+                return whole;
+            }
+        }
         const float* const row = row_of(e, j);
         return trip(buf, std::false_type{}, now_c, tau, e, [&](uint32_t pq, uint32_t p) { return load(row + (OTHER ? MR::order(pq) | MR::order(p) : pq | p)); });
     };
