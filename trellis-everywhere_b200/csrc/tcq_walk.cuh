@@ -4,6 +4,7 @@
 #include <type_traits>
 
 #include "tcq_forward.cuh"
+#include "tcq_handoff.cuh"
 #include "tcq_mbarrier.cuh"
 
 namespace tcq {
@@ -114,7 +115,7 @@ struct WalkShared {
     uint16_t other[FUSED ? kT : 1];                // states of another path
     uint32_t todo[FUSED ? kMaxTodo : 1][3];        // such paths: the last step that they do not share, the state there, q's of the trip before it
     int go_on;                                     // the second group's orders
-    volatile int trips;                            // taken by the first group (kAllTrips: the walk is over and `cost` complete)
+    int trips;                                     // taken by the first group (kAllTrips: the walk is over and `cost` complete), published (tcq_handoff.cuh)
     int verdict;                                   // of the second group on the marks: kOther | kApart
     static constexpr int kAllTrips = 1 << 20, kOther = 1, kApart = 2;
 };
@@ -421,10 +422,7 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
             if (tid == 0 && (!first || tau + i >= 0)) st[tau + i] = uint16_t(s);
             e = s >> K;
         }
-        if (FUSED && behind && tid == 0 && j % 4 == 3) {   // (a fence every trip: 4 to 7 us a walk)
-            __threadfence_block();
-            sh.trips = j + 1;
-        }
+        if (FUSED && behind && tid == 0 && j % 4 == 3) handoff_publish(sh.trips, j + 1);   // (every trip: 4 to 7 us a walk)
     };
     auto walk = [&]() __attribute__((always_inline)) {     // back to step `lo`, or a little further
         for (; tau > 0 && tau + D > lo; ++j, tau -= D) take(row_trip(j & 1, std::false_type{}, tau, e, j), false);
@@ -482,13 +480,12 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
         };
         // Whether the first group has taken so many trips: it need not have at once where the second one is behind it.
         auto taken = [&](int trips) -> bool {
-            if (who == 0 || sh.trips >= trips) return true;
+            if (who == 0 || handoff_count(sh.trips) >= trips) return true;
             const long long t0 = clock64();
-            while (sh.trips < trips) {
+            while (handoff_count(sh.trips) < trips) {
                 __nanosleep(200);
-                if (clock64() - t0 > 500000000ll) return sh.trips >= trips;
+                if (clock64() - t0 > 500000000ll) return handoff_count(sh.trips) >= trips;
             }
-            __threadfence_block();
             return true;
         };
         bool apart = false;                        // another path does not meet the one found as far as that is known
@@ -635,10 +632,7 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
             if (who == 0) {
                 if (sums) sum_up();
                 if (tied && tid == 0 && a.sse != nullptr) a.sse[tile] = sh.cost[kT];
-                if (behind && !deep && tid == 0) {
-                    __threadfence_block();
-                    sh.trips = sh.kAllTrips;
-                }
+                if (behind && !deep && tid == 0) handoff_publish(sh.trips, sh.kAllTrips);
                 again = sums && !(sh.cost[kT] < kFusedMax);
                 if (tied) again = again || uint32_t(found[0]) >> K != ov;
                 else again = again || !(end_metric < kFusedMax) || __ballot_sync(0xffffffffu, key == kTooMany) != 0;
