@@ -190,6 +190,14 @@ TCQ_API int tcq_workspace_status(const void *ws, size_t ws_bytes, int64_t n_tile
 TCQ_API int tcq_selftest_wait_timeout(const float *w, int64_t n_tiles, int K, void *ws, size_t ws_bytes, void *stream);
 
 /*
+ * Self-test of the bounded waits of the walks: tcq_encode_tb with the MCG codebook, with a limit of nothing on every wait of the
+ * second group of warps that walks a tile for the first one (batches of 149 tiles and more at K = 3 and 4; there are no
+ * others to test elsewhere).  Tiles whose wait runs out are swept again, so the codes are those of tcq_encode_tb.
+ * At most 2000 tiles (TCQ_E_BAD_COUNT).  No reference counterpart.
+ */
+TCQ_API int tcq_selftest_walk_waits(const float *w, int64_t n_tiles, int K, uint32_t *packed, void *ws, size_t ws_bytes, void *stream);
+
+/*
  * Number of kernel launches tcq_encode_tb issues for n_tiles with a workspace of
  * ws_bytes (four per chunk: step kernel and traceback for each of the two passes;
  * six or twelve where the workspace holds a half or a quarter of a path only, and

@@ -70,6 +70,30 @@ def test_a_large_batch_of_ordinary_tiles(oracle, luts, monkeypatch, K):
     assert np.array_equal(got.bits.cpu().numpy()[idx], bits) and same_bits(got.dq.cpu().numpy()[idx], dq) and same_bits(got.sse.cpu().numpy()[idx], sse)
 
 
+def _listed(ws):
+    """How many tiles the walks of the two passes of a span have listed (the words that tcq_capi.cu's `counts` names)."""
+    return ws[16:24].view(torch.int32).tolist()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (3, 4))
+def test_a_walk_that_does_not_wait_lists_its_tile(K):
+    """The second group of warps gives up at once where the first has not come far enough, now one warp of it first and now the other: the
+    tiles are swept again, nothing hangs, and the codes are the same."""
+    from trellis_b200 import qtip as q
+    n, lib = 600, q._lib.lib()
+    w = (torch.randn(n, 256, generator=torch.Generator().manual_seed(K)) * 1.24).cuda()
+    ws = torch.zeros(int(lib.tcq_workspace_bytes(n, K)), dtype=torch.uint8, device="cuda")
+    stream, want, got = torch.cuda.current_stream().cuda_stream, *torch.zeros(2, n, 8 * K, dtype=torch.int32, device="cuda")
+    assert lib.tcq_encode_tb(w.data_ptr(), n, K, 2, want.data_ptr(), None, None, None, ws.data_ptr(), ws.numel(), stream) == 0
+    assert max(_listed(ws)) <= n // 100
+    for _ in range(5):
+        got.zero_()
+        assert lib.tcq_selftest_walk_waits(w.data_ptr(), n, K, got.data_ptr(), ws.data_ptr(), ws.numel(), stream) == 0
+        assert torch.equal(got, want) and min(_listed(ws)) > n // 2
+    assert lib.tcq_workspace_status(ws.data_ptr(), ws.numel(), n, K, stream) == 0
+
+
 def test_the_bound_between_fused_and_rounded_sums():
     """|A - F| <= (2 t + 2) u H of the limit (fused_limit), over random, repeated and graded terms; A as the fused operation gives it (the
     square is exact in 64 bits, the sum there rounds 2^29 times finer)."""

@@ -13,9 +13,15 @@ def handoff(tmp_path_factory):
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
     subprocess.check_call(["g++", "-std=c++20", "-O2", "-g", "-fsanitize=thread", "-isystem", os.path.join(cuda, "include"), "-o", exe,
                            os.path.join(ROOT, "tests", "handoff.cpp"), "-pthread"])
-    return lambda: subprocess.run([exe], capture_output=True, text=True, timeout=300)
+    return lambda what: subprocess.run([exe, what], capture_output=True, text=True, timeout=300)
 
 
 def test_what_was_written_before_the_count_is_there(handoff):
-    r = handoff()
+    r = handoff("order")
     assert r.returncode == 0 and "data race" not in r.stderr, r.stderr[:2000]
+
+
+def test_all_threads_leave_a_wait_with_the_same_outcome(handoff):
+    """The clock of one follower runs out; the other, whose clock does not, then sees the count and still has to give up with it."""
+    r = handoff("limit")
+    assert r.returncode == 0 and "data race" not in r.stderr, r.stdout + r.stderr[:2000]

@@ -445,6 +445,7 @@ struct EncodeIO {
     float* sse;
     float* wq;
     float* err;
+    bool hurry;                // see TracebackArgs
 };
 
 // The launch sequence of the tail-biting encoder (src/trellis/qtip.py:135-144) per workspace chunk:
@@ -508,6 +509,7 @@ int encode_core(const EncodeIO& io, int K, int codebook, void* ws, size_t ws_byt
                 t.again = wk.list;
                 t.again_count = wk.counts + second;
                 t.first_tile = int(c0);
+                t.hurry = io.hurry;
                 if ((rc = pass(K, codebook, f, second ? kT : kT / 2, t, wk, num_sms, s, second ? "pass 2" : "pass 1")) != TCQ_OK) return rc;
             }
             ForwardArgs f = second ? forward_2(s0, sn, wk.overlap) : forward_1(s0, sn);
@@ -706,6 +708,21 @@ int tcq_selftest_wait_timeout(const float* w, int64_t n_tiles, int K, void* ws, 
                       : K == 3 ? launch_forward_cluster<3>(kCbMcg, ca, 2, 2, s)
                                : launch_forward_cluster<4>(kCbMcg, ca, 2, 2, s);
     return err == cudaSuccess ? TCQ_OK : cuda_fail(err, "forward (self-test)");
+}
+
+int tcq_selftest_walk_waits(const float* w, int64_t n_tiles, int K, uint32_t* packed, void* ws, size_t ws_bytes, void* stream) {
+    const int rc = check_common(K, kCbMcg, n_tiles);
+    if (rc != TCQ_OK) return rc;
+    if (n_tiles < 1 || n_tiles > 2000) return TCQ_E_BAD_COUNT;
+    if (w == nullptr || packed == nullptr) return TCQ_E_NULL_POINTER;
+    if (misaligned(w, 16) || misaligned(packed, 4)) return TCQ_E_MISALIGNED;
+    EncodeIO io{};
+    io.w = w;
+    io.n = n_tiles;
+    io.packed = packed;
+    io.packed_stride = kT * K / 32;
+    io.hurry = true;
+    return encode_core(io, K, kCbMcg, ws, ws_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int64_t tcq_encode_launches(int64_t n_tiles, int K, size_t ws_bytes) {

@@ -316,6 +316,7 @@ struct TracebackArgs {
     int* again;                // out: tiles that have to be swept again with every operation rounded, in no order, first_tile added, and
     int* again_count;          // their number
     int first_tile;
+    int hurry;                 // self-test: the waits of the walk give up at once
 };
 
 // How the cluster kernel forms a candidate, (w - c)^2 + metric.

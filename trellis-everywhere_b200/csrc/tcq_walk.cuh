@@ -86,6 +86,7 @@ __device__ __forceinline__ float fused_limit(float best, int t) {
     return __fadd_rn(__fmaf_rn(h, float(4 * t + 16) * 0x1p-24f, best), 1e-30f);
 }
 constexpr float kFusedMax = 1e37f;
+constexpr long long kWalkWaitCycles = 500000000LL;        // of the second group for the first, a quarter of a second where microseconds are due
 
 // A tile's rows lie one after another whatever the path, so where few tiles walk, each on an SM of its own, their CTAs fetch whole rows ahead
 // (32 KiB at K = 3) and find a trip's metrics in shared memory: the latency of L2 or HBM leaves the chain of trips.  16 times as many bytes
@@ -130,7 +131,7 @@ struct WalkShared {
 // their rounded sums from where they meet (one tile in 200 of the first pass is walked back to its beginning for that).
 // Other paths cost as long as they are to walk, so a second group of warps walks them at the same time: where the pass may end with one
 // of two edges (one tile in 25 of the first pass) it walks from the second edge; otherwise it goes behind the first group and takes up
-// the trips that get marked.  Its waits for the first group are bounded by the clock.
+// the trips that get marked.  Its waits for the first group are bounded by the clock; a tile whose wait runs out is listed.
 // What this does not settle (marks on the other path too, another winner, more than a few marks, costs above 1e37 or not a
 // number) lists the tile in a.again: one tile in 10 000, and every tile of ties, such as one of zeros.
 //
@@ -478,16 +479,20 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
             }
             return f;
         };
-        // Whether the first group has taken so many trips: it need not have at once where the second one is behind it.
-        auto taken = [&](int trips) -> bool {
-            if (who == 0 || handoff_count(sh.trips) >= trips) return true;
-            const long long t0 = clock64();
-            while (handoff_count(sh.trips) < trips) {
-                __nanosleep(200);
-                if (clock64() - t0 > 500000000ll) return handoff_count(sh.trips) >= trips;
+        // Whether the first group has taken so many trips, which it need not have at once where the second one is behind it.
+        struct Follower {
+            __device__ static long long clock() { return clock64(); }
+            __device__ static void pause() { __nanosleep(200); }
+            __device__ static bool all(bool x) {           // of the second group
+                x = __all_sync(0xffffffffu, x);
+                if constexpr (W == 1) return x;
+                uint32_t every;
+                asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.and.pred p, 2, %2, p;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                             : "=r"(every) : "r"(uint32_t(x)), "n"(NT) : "memory");
+                return every != 0;
             }
-            return true;
-        };
+        } follower;
+        auto taken = [&](int trips) -> bool { return who == 0 || handoff_wait(follower, sh.trips, trips, a.hurry ? 0 : kWalkWaitCycles); };
         bool apart = false;                        // another path does not meet the one found as far as that is known
         int trips = 0;
         auto any_trip = [&](int tau, uint32_t e) -> uint32_t {
