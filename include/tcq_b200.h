@@ -83,12 +83,13 @@ TCQ_API size_t tcq_workspace_min_bytes(int K);
  * Replaces viterbi_tb (src/trellis/qtip.py:124-144) and viterbi_tb_triton
  * (src/trellis/viterbi_triton.py:121-129), with pack_bits_np
  * (scripts/export_packed_8b.py:52-62) fused into the traceback.
- *   w       [n_tiles,256] fp32, 16-byte aligned, never written
+ *   w       [n_tiles,256] fp32, 16-byte aligned, only read
  *   packed  [n_tiles, 8*K] u32: bit kb of symbol t at bit (255-t)*K+kb   (required)
  *   bits    [n_tiles,256] int64 symbols (< 2^K), or NULL
  *   dq      [n_tiles,256] fp32 reconstruction codebook[state_t], or NULL
  *   sse     [n_tiles] fp32 sum_t (w_t-dq_t)^2 accumulated in time order, or NULL
  *   ws      scratch, 256-byte aligned, ws_bytes >= tcq_workspace_min_bytes(K)
+ * dq may be w itself (the reconstruction takes the weights' place); no output may overlap w or another output otherwise.
  */
 TCQ_API int tcq_encode_tb(const float *w, int64_t n_tiles, int K, int codebook, uint32_t *packed, int64_t *bits,
                   float *dq, float *sse, void *ws, size_t ws_bytes, void *stream);

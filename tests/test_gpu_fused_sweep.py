@@ -70,6 +70,23 @@ def test_a_large_batch_of_ordinary_tiles(oracle, luts, monkeypatch, K):
     assert np.array_equal(got.bits.cpu().numpy()[idx], bits) and same_bits(got.dq.cpu().numpy()[idx], dq) and same_bits(got.sse.cpu().numpy()[idx], sse)
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (2, 3, 4))
+@pytest.mark.parametrize("n", (100, 300, 1000))
+def test_the_reconstruction_may_take_the_weights_place(K, n):
+    """dq over w, with tiles that are swept again among the others, at full scratch and (paths walked in parts) at little."""
+    from trellis_b200 import qtip as q
+    w, lib = _tiles(n, q.codebook_lut("mcg", "cpu"), n + K).cuda(), q._lib.lib()
+    want = q.encode(w, K, "mcg")
+    for ws_bytes in (int(lib.tcq_workspace_bytes(n, K)), n // 5 * int(lib.tcq_workspace_min_bytes(K))):
+        ws, x = torch.zeros(ws_bytes, dtype=torch.uint8, device="cuda"), w.clone()
+        packed, sse = torch.zeros(n, 8 * K, dtype=torch.int32, device="cuda"), torch.zeros(n, device="cuda")
+        assert lib.tcq_encode_tb(x.data_ptr(), n, K, 2, packed.data_ptr(), None, x.data_ptr(), sse.data_ptr(), ws.data_ptr(), ws_bytes,
+                                 torch.cuda.current_stream().cuda_stream) == 0
+        assert torch.equal(packed, want.packed) and torch.equal(x.view(torch.int32), want.dq.view(torch.int32))
+        assert torch.equal(sse.view(torch.int32), want.sse.view(torch.int32))
+
+
 def _listed(ws):
     """How many tiles the walks of the two passes of a span have listed (the words that tcq_capi.cu's `counts` names)."""
     return ws[16:24].view(torch.int32).tolist()

@@ -636,7 +636,6 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
             const bool alone = !behind || deep;
             if (who == 0) {
                 if (sums) sum_up();
-                if (tied && tid == 0 && a.sse != nullptr) a.sse[tile] = sh.cost[kT];
                 if (behind && !deep && tid == 0) handoff_publish(sh.trips, sh.kAllTrips);
                 again = sums && !(sh.cost[kT] < kFusedMax);
                 if (tied) again = again || uint32_t(found[0]) >> K != ov;
@@ -673,7 +672,11 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
             if (tid == 0) sh.go_on = 0;
             both();
         }
-        if (again && tid == 0) a.again[atomicAdd(a.again_count, 1)] = a.first_tile + int(tile);
+        if (again) {                               // no outputs: they may lie over the weights, which the sweep to come reads again
+            if (tid == 0) a.again[atomicAdd(a.again_count, 1)] = a.first_tile + int(tile);
+            return;
+        }
+        if (tied && tid == 0 && a.sse != nullptr) a.sse[tile] = sh.cost[kT];
     }
     if (tid == 0 && a.e_out != nullptr) a.e_out[tile] = int(st[t_off] >> K);     // a trip may have gone past step t_off
     emit_outputs<K, NT>(a, tile, st, t_off, a.t_end, tid);

@@ -237,6 +237,7 @@ def encode_rows(src: torch.Tensor, comp: Optional[torch.Tensor], K: int, codeboo
     encoded, and written back in the same layout: ``wq`` the reconstruction, ``err = src - wq``.
     ``packed``: int32 view ``[n_out/16, 8K]`` whose rows may be strided (a column of the matrix's
     ``[n_out/16, k_in/16, 8K]`` code array).  All tensors on one CUDA device; nothing synchronises.
+    ``wq`` and ``err`` must not overlap ``src``, ``comp`` or each other.
     """
     if src.dim() != 2 or src.shape[0] != 16 or src.shape[1] % 16:
         raise ValueError(f"expected a (16, n_out) block with n_out % 16 == 0, got {tuple(src.shape)}")
