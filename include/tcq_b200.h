@@ -191,9 +191,11 @@ TCQ_API int tcq_workspace_status(const void *ws, size_t ws_bytes, int64_t n_tile
 TCQ_API int tcq_selftest_wait_timeout(const float *w, int64_t n_tiles, int K, void *ws, size_t ws_bytes, void *stream);
 
 /*
- * Self-test of the bounded waits of the walks: tcq_encode_tb with the MCG codebook, with a limit of nothing on every wait of the
- * second group of warps that walks a tile for the first one (batches of 149 tiles and more at K = 3 and 4; there are no
- * others to test elsewhere).  Tiles whose wait runs out are swept again, so the codes are those of tcq_encode_tb.
+ * Self-test of the bounded waits of the walks: tcq_encode_tb with the MCG codebook, with a limit of nothing on every wait of a
+ * walk.  Batches of 149 tiles and more at K = 3 and 4: those of the second group of warps that walks a tile for the first one; tiles whose
+ * wait runs out are swept again.  Batches of 3 to 74 / 96 / 148 tiles (K = 2 / 3 / 4): those for rows fetched ahead into shared memory;
+ * the walk goes on without them, ends when the copies on their way have landed (a wait with a limit of its own), and
+ * tcq_workspace_status must report TCQ_E_DEVICE_TIMEOUT.  The codes are those of tcq_encode_tb in both.
  * At most 2000 tiles (TCQ_E_BAD_COUNT).  No reference counterpart.
  */
 TCQ_API int tcq_selftest_walk_waits(const float *w, int64_t n_tiles, int K, uint32_t *packed, void *ws, size_t ws_bytes, void *stream);

@@ -25,3 +25,22 @@ def test_rows_in_the_ring(oracle, luts, K, n):
         assert lib.tcq_encode_tb(wd.data_ptr(), n, K, 1, packed.data_ptr(), b.data_ptr(), d.data_ptr(), s.data_ptr(), ws.data_ptr(), ws_bytes, stream) == 0
         assert np.array_equal(b.cpu().numpy()[idx], bits)
         assert same_bits(d.cpu().numpy()[idx], dq) and same_bits(s.cpu().numpy()[idx], sse)
+
+
+@pytest.mark.parametrize("K", KS)
+@pytest.mark.parametrize("n", (3, 8, 74))
+def test_rows_that_do_not_come_in_time(K, n):
+    """The walk waits for no row: it reads them from global memory, the status word says so, and the CTA ends after its copies.
+    The calls that follow on the same SMs are sound."""
+    from trellis_b200 import qtip as q
+    lib, stream = q._lib.lib(), torch.cuda.current_stream().cuda_stream
+    w = (torch.randn(n, 256, generator=torch.Generator().manual_seed(n + K)) * 1.2).cuda()
+    want = q.encode(w, K, "mcg").packed
+    for ws_bytes in (int(lib.tcq_workspace_bytes(n, K)), n * int(lib.tcq_workspace_min_bytes(K))):
+        ws, packed = torch.zeros(ws_bytes, dtype=torch.uint8, device="cuda"), torch.zeros(n, 8 * K, dtype=torch.int32, device="cuda")
+        assert lib.tcq_selftest_walk_waits(w.data_ptr(), n, K, packed.data_ptr(), ws.data_ptr(), ws_bytes, stream) == 0
+        assert lib.tcq_workspace_status(ws.data_ptr(), ws_bytes, n, K, stream) == -10          # TCQ_E_DEVICE_TIMEOUT
+        assert torch.equal(packed, want)
+        packed.zero_()
+        assert lib.tcq_encode_tb(w.data_ptr(), n, K, 2, packed.data_ptr(), None, None, None, ws.data_ptr(), ws_bytes, stream) == 0
+        assert lib.tcq_workspace_status(ws.data_ptr(), ws_bytes, n, K, stream) == 0 and torch.equal(packed, want)

@@ -318,6 +318,7 @@ cudaError_t forward(int K, int codebook, const ForwardArgs& a, const Workspace& 
     t->w_add = a.w_add;
     t->ld = a.ld;
     t->roll = a.roll;
+    t->status = a.status;
     t->overlap = a.overlap;
     t->e_start = a.overlap != nullptr ? a.overlap : wk.e_final;
     t->keys = nullptr;
@@ -478,6 +479,7 @@ int encode_core(const EncodeIO& io, int K, int codebook, void* ws, size_t ws_byt
         t.wq = io.wq ? io.wq + c0 * tile_step : nullptr;
         t.err = io.err ? io.err + c0 * tile_step : nullptr;
         t.src = io.w + c0 * tile_step;
+        t.hurry = io.hurry;
         return t;
     };
     if (!wk.fused) {
@@ -485,6 +487,7 @@ int encode_core(const EncodeIO& io, int K, int codebook, void* ws, size_t ws_byt
             const long long cn = io.n - c0 < wk.chunk ? io.n - c0 : wk.chunk;
             TracebackArgs t1{};
             t1.e_out = wk.overlap;
+            t1.hurry = io.hurry;
             if ((rc = pass(K, codebook, forward_1(c0, cn), kT / 2, t1, wk, num_sms, s, "pass 1")) != TCQ_OK) return rc;
             if ((rc = pass(K, codebook, forward_2(c0, cn, wk.overlap), kT, outputs(c0), wk, num_sms, s, "pass 2")) != TCQ_OK) return rc;
         }

@@ -317,6 +317,7 @@ struct TracebackArgs {
     int* again_count;          // their number
     int first_tile;
     int hurry;                 // self-test: the waits of the walk give up at once
+    unsigned int* status;      // bit 0: a row of the ring did not come (ForwardArgs), or nullptr
 };
 
 // How the cluster kernel forms a candidate, (w - c)^2 + metric.

@@ -374,7 +374,8 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
     // ... where its metrics are: rows, or before step 0
     auto row_of = [&](uint32_t e, int j) { return rows + size_t(j) * E + (e >> (K * D)) * uint32_t(NA); };    // the ancestors share the edge's bits above K*D
     [[maybe_unused]] unsigned long long* const full = reinterpret_cast<unsigned long long*>(ring + (RING ? Ring<K>::kRows * int(E) : 0));
-    [[maybe_unused]] bool lost = false;            // RING: a row did not come; the walk goes on from global memory
+    [[maybe_unused]] bool lost = RING && a.hurry;  // RING: a row did not come; the walk goes on from global memory
+    [[maybe_unused]] int lost_at = 0;              // ... this row
     [[maybe_unused]] int ring_rows = 0;            // rows that the walk reads
     [[maybe_unused]] auto fetch = [&](int j) {
         const uint32_t bar = smem_u32(full + j % Ring<K>::kRows);
@@ -398,6 +399,7 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
             if (!lost) {
                 const bool came = mbar_wait(smem_u32(full + j % Ring<K>::kRows), uint32_t(j / Ring<K>::kRows) & 1u, reinterpret_cast<volatile unsigned int*>(full + 15));
                 lost = __any_sync(0xffffffffu, !came);
+                lost_at = j;
             }
             if (!lost) {
                 const float* const row = ring + j % Ring<K>::kRows * int(E) + (e >> (K * D)) * uint32_t(NA);
@@ -680,6 +682,14 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
     }
     if (tid == 0 && a.e_out != nullptr) a.e_out[tile] = int(st[t_off] >> K);     // a trip may have gone past step t_off
     emit_outputs<K, NT>(a, tile, st, t_off, a.t_end, tid);
+    if constexpr (RING)
+        if (lost) {
+            if (lane == 0 && a.status != nullptr) atomicOr(a.status, 1u);
+            // The copies that are still on their way: the next CTA on this SM must not find them in its shared memory.
+            const long long t0 = clock64();
+            for (int i = lost_at; tid == 0 && i < ring_rows && i < lost_at + Ring<K>::kRows; ++i)
+                while (!mbar_try_wait(smem_u32(full + i % Ring<K>::kRows), uint32_t(i / Ring<K>::kRows) & 1u) && clock64() - t0 < kMbarWaitCycles) {}
+        }
 }
 
 }  // namespace tcq
