@@ -3,7 +3,9 @@
 // launch_plan_runtime.cpp.  Built and run by test_launch_plan.py.  Arguments, in order:
 //   fail N             the next N occupancy queries fail
 //   encode K N BYTES   tcq_encode_tb of N tiles with BYTES of scratch (0: what tcq_workspace_bytes says)
-//   shapes K           the shapes that a launch may have
+//   pass K N BYTES     tcq_viterbi_pass, unconstrained, likewise
+//   size K N 0         what tcq_workspace_bytes says
+//   shapes K           the shapes that a launch may have, by form
 // Each launch, each call's status and each shape is printed on a line.
 #include <cstdio>
 #include <cstdlib>
@@ -19,6 +21,7 @@ extern int g_failing_queries;
 // What a call puts where in its scratch: complaints about bytes outside, and about bytes that another buffer holds.
 constexpr uintptr_t kScratch = 1 << 22;
 static size_t g_scratch_bytes = 0;
+static long long g_span = 0;           // tiles whose walks have shared a list so far
 struct Use { std::string what; uintptr_t begin, end; };
 static std::vector<Use> g_uses;
 static void use(const std::string& what, const void* p, size_t bytes) {
@@ -36,10 +39,18 @@ static cudaError_t cluster(int K, const ClusterArgs& ca, int C, int G) {
     // queries go through the real launcher (of the size with the smallest kernel for all but one)
     if (ca.f.n <= 0) return C == 16 ? launch_cluster_variant<2, kCbMcg, 16, 1, 0, 256>(ca, nullptr) : C == 8 ? launch_cluster_variant<2, kCbMcg, 8, 1, 0, 512>(ca, nullptr)
                           : C == 4 ? launch_cluster_variant<2, kCbMcg, 4, 1, 0, 512>(ca, nullptr) : launch_cluster_variant<2, kCbMcg, 2, 1, 0, 512>(ca, nullptr);
-    std::printf("cluster K=%d C=%d G=%d n=%lld steps=%d\n", K, C, G, ca.f.n, ca.f.steps);
+    const char* const form = ca.form == StepForm::kFused ? "fused" : ca.form == StepForm::kListed ? "listed" : "rounded";
+    std::printf("cluster K=%d C=%d G=%d n=%lld steps=%d %s\n", K, C, G, ca.f.n, ca.f.steps, form);
+    const bool fused = ca.form == StepForm::kFused, listed = ca.form == StepForm::kListed;
+    if (listed && (C * ca.at_once > 148 || ca.f.n > ca.at_once)) std::printf("outside: more listed tiles than clusters\n");
     use("rows", ca.rows, ca.f.n * ca.nrows * (size_t(4) << (16 - K)));
-    if (ca.keys != nullptr) use("keys", ca.keys, ca.f.n * C * 8);
-    if (ca.f.overlap != nullptr) use("overlap", ca.f.overlap, ca.f.n * 4);
+    if (ca.keys != nullptr) use("keys", ca.keys, ca.f.n * C * 8 * (fused ? kFusedKeys : 1));
+    // (a listed tile's overlap lies anywhere in the span, whose walks have said how large it is)
+    if (ca.f.overlap != nullptr) use("overlap", ca.f.overlap, listed ? g_span * 4 : ca.f.n * 4);
+    if (fused) use("counts", ca.counts, 2 * sizeof(int));
+    if (listed) use("list", ca.list, g_span * 4), use("counts", ca.list_count, sizeof(int));
+    if (listed && ca.walk.keys != ca.keys) std::printf("outside: keys of the listed walk\n");
+    if (listed && ca.walk.e_out != nullptr) use("edges", ca.walk.e_out, g_span * 4);
     return cudaSuccess;
 }
 static cudaError_t cta(int K, const ForwardArgs& a) {
@@ -55,6 +66,12 @@ template <> cudaError_t launch_forward_cta<4>(int, const ForwardArgs& a, int, cu
 cudaError_t launch_traceback(int, const TracebackArgs& a, cudaStream_t) {
     std::printf("walk %s n=%lld keys=%d\n", a.rows != nullptr ? "rows" : "backpointers", a.n, a.keys != nullptr ? a.nkeys : 0);
     if (a.e_out != nullptr) use("edges", a.e_out, a.n * 4);
+    if (a.keys != nullptr) use("keys", a.keys, a.n * a.nkeys * 8);
+    if (a.fused) {
+        if (a.first_tile == 0) g_span = 0;
+        g_span = a.first_tile + a.n > g_span ? a.first_tile + a.n : g_span;
+        use("list", a.again, g_span * 4), use("counts", a.again_count, sizeof(int));
+    }
     return cudaSuccess;
 }
 cudaError_t launch_decode_packed(const uint32_t*, long long, int, int, float*, cudaStream_t) { return cudaErrorUnknown; }
@@ -77,16 +94,25 @@ int main(int argc, char** argv) {
             g_failing_queries = std::atoi(argv[i + 1]);
             i += 2;
         } else if (!std::strcmp(argv[i], "shapes")) {
-            const auto [s, n] = shapes(std::atoi(argv[i + 1]));
-            for (int j = 0; j < n; ++j) std::printf("C=%d G=%d\n", s[j].C, s[j].G);
+            const int K = std::atoi(argv[i + 1]);
+            for (bool fused : {false, true}) {
+                const auto [s, n] = shapes(K, fused);
+                for (int j = 0; j < n && (!fused || K > 2); ++j) std::printf("C=%d G=%d %s\n", s[j].C, s[j].G, fused ? "fused" : "rounded");
+            }
             i += 2;
+        } else if (!std::strcmp(argv[i], "size")) {
+            std::printf("%zu\n", tcq_workspace_bytes(std::atoll(argv[i + 2]), std::atoi(argv[i + 1])));
+            i += 4;
         } else {
             const int K = std::atoi(argv[i + 1]);
             const long long n = std::atoll(argv[i + 2]), bytes = std::atoll(argv[i + 3]);
             g_scratch_bytes = bytes > 0 ? size_t(bytes) : tcq_workspace_bytes(n, K);
             g_uses.clear();
-            std::printf("status %d\n", tcq_encode_tb(static_cast<float*>(address(1 << 20)), n, K, 2, static_cast<uint32_t*>(address(1 << 21)), nullptr, nullptr,
-                                                     nullptr, address(kScratch), g_scratch_bytes, nullptr));
+            g_span = 0;
+            const float* const w = static_cast<float*>(address(1 << 20));
+            std::printf("status %d\n", !std::strcmp(argv[i], "pass")
+                                           ? tcq_viterbi_pass(w, n, K, 2, nullptr, 0, static_cast<int64_t*>(address(1 << 21)), address(kScratch), g_scratch_bytes, nullptr)
+                                           : tcq_encode_tb(w, n, K, 2, static_cast<uint32_t*>(address(1 << 21)), nullptr, nullptr, nullptr, address(kScratch), g_scratch_bytes, nullptr));
             i += 4;
         }
     }

@@ -1,11 +1,14 @@
 """Sweeps with fused candidates (batches of 149 tiles and more at K = 3 and 4): the square and the sum are one operation there, and the walk
 and a second kernel see to it that the codes are those of the rounded operations.  TCQ_FORWARD_KERNEL=cluster2 runs every
 batch with the rounded operations; the two must agree bit for bit, whatever the tiles."""
+import os
+import subprocess
+
 import numpy as np
 import pytest
 import torch
 
-from conftest import same_bits
+from conftest import ROOT, same_bits
 
 NAMES = ("1mad", "3inst", "mcg")
 
@@ -42,7 +45,7 @@ def _both(q, monkeypatch, call):
 @pytest.mark.gpu
 @pytest.mark.parametrize("K", (3, 4))
 @pytest.mark.parametrize("name", NAMES)
-@pytest.mark.parametrize("n", (149, 300, 445, 900))       # one launch and two, one chunk and two; 450 tiles to sweep again in the last
+@pytest.mark.parametrize("n", (149, 300, 445, 900, 1000))       # one launch and two, one chunk and two (leaving 12 and 112 tiles over); hundreds of tiles to sweep again in the last
 def test_codes_are_those_of_the_rounded_operations(monkeypatch, K, name, n):
     from trellis_b200 import qtip as q
     w = _tiles(n, q.codebook_lut(name, "cpu"), 10 * n + K).cuda()
@@ -94,6 +97,52 @@ def _listed(ws):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("K", (3, 4))
+@pytest.mark.parametrize("n,size_for", ((700, 350), (1000, 888), (2700, 888)))         # two spans, two with a short one, four
+def test_batches_of_several_spans(monkeypatch, K, n, size_for):
+    """Scratch sized for fewer tiles: the lists, the overlaps and the counts of a span are those of the span before, used again."""
+    from trellis_b200 import qtip as q
+    lib = q._lib.lib()
+    w = _tiles(n, q.codebook_lut("1mad", "cpu"), n + K).cuda()
+    ws = torch.full((int(lib.tcq_workspace_bytes(size_for, K)),), 0x5A, dtype=torch.uint8, device="cuda")
+
+    def encode():
+        packed, dq, sse = torch.zeros(n, 8 * K, dtype=torch.int32, device="cuda"), torch.zeros(n, 256, device="cuda"), torch.zeros(n, device="cuda")
+        assert lib.tcq_encode_tb(w.data_ptr(), n, K, 0, packed.data_ptr(), None, dq.data_ptr(), sse.data_ptr(), ws.data_ptr(), ws.numel(),
+                                 torch.cuda.current_stream().cuda_stream) == 0
+        return packed, dq, sse
+
+    _both(q, monkeypatch, encode)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (3, 4))
+def test_what_the_walk_settles_and_what_it_lists(K):
+    """Of 20 000 Gaussian tiles 800 have a second edge at the end of pass 1, some hundred a marked node and some tens are walked back to the beginning:
+    no more than a few are listed, so each of these is settled and not left to the second sweep.  Tiles whose costs are above 1e37 are all listed
+    (of ties alone that does not hold in both passes: over zeros the free pass has one best path)."""
+    from trellis_b200 import qtip as q
+    lib, stream = q._lib.lib(), torch.cuda.current_stream().cuda_stream
+    for w, least, most in ((torch.randn(20000, 256, generator=torch.Generator().manual_seed(K)) * 1.24, 0, 20), (torch.full((300, 256), 1e18), 300, 300)):
+        n, w = w.shape[0], w.cuda()
+        ws, packed = torch.zeros(int(lib.tcq_workspace_bytes(n, K)), dtype=torch.uint8, device="cuda"), torch.zeros(n, 8 * K, dtype=torch.int32, device="cuda")
+        assert lib.tcq_encode_tb(w.data_ptr(), n, K, 2, packed.data_ptr(), None, None, None, ws.data_ptr(), ws.numel(), stream) == 0
+        assert all(least <= x <= most for x in _listed(ws)), _listed(ws)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (3, 4))
+@pytest.mark.parametrize("n", (200, 296, 370, 444))       # three to six tiles a cluster
+def test_single_passes_keep_the_rounded_shapes(K, n):
+    """tcq_viterbi_pass sweeps every batch with rounded operations; its two passes give the codes of an encode."""
+    from trellis_b200 import qtip as q
+    w = (torch.randn(n, 256, generator=torch.Generator().manual_seed(n + K)) * 1.24).cuda()
+    overlap = (q.viterbi_pass_b200(w, K, None, "mcg", roll=128)[:, 128] >> K).int()
+    states = q.viterbi_pass_b200(w, K, overlap, "mcg")
+    assert torch.equal(states & (2 ** K - 1), q.encode(w, K, "mcg", want_bits=True).bits)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (3, 4))
 def test_a_walk_that_does_not_wait_lists_its_tile(K):
     """The second group of warps gives up at once where the first has not come far enough, now one warp of it first and now the other: the
     tiles are swept again, nothing hangs, and the codes are the same."""
@@ -111,16 +160,38 @@ def test_a_walk_that_does_not_wait_lists_its_tile(K):
     assert lib.tcq_workspace_status(ws.data_ptr(), ws.numel(), n, K, stream) == 0
 
 
-def test_the_bound_between_fused_and_rounded_sums():
-    """|A - F| <= (2 t + 2) u H of the limit (fused_limit), over random, repeated and graded terms; A as the fused operation gives it (the
-    square is exact in 64 bits, the sum there rounds 2^29 times finer)."""
+@pytest.fixture(scope="module")
+def fused_limit(tmp_path_factory):
+    """fused_limit of tcq_walk.cuh: (smallest candidates, steps) -> limits."""
+    exe = str(tmp_path_factory.mktemp("limit") / "fused_limit")
+    subprocess.check_call([os.environ.get("NVCC", "nvcc"), "-gencode", "arch=compute_100a,code=sm_100a", "-std=c++17", "-O1", "-fmad=false",
+                           "-o", exe, os.path.join(ROOT, "tests", "fused_limit.cu")])
+
+    def run(best, t):
+        pairs = np.empty(best.size, [("best", np.float32), ("t", np.int32)])
+        pairs["best"], pairs["t"] = best.ravel(), t.ravel()
+        return np.frombuffer(subprocess.run([exe], input=pairs.tobytes(), check=True, capture_output=True).stdout, np.float32).reshape(best.shape)
+
+    return run
+
+
+def test_the_bound_between_fused_and_rounded_sums(fused_limit):
+    """|A - F| <= (2 t + 2) u H, and no more than half of what fused_limit adds, so that of two candidates one of which is beyond the other's limit
+    that one is the larger by the rounded sums too; over random, repeated and graded terms.  A as the fused operation gives it (the
+    square is exact in 64 bits, the sum there rounds 2^29 times finer).  The limit adds no more than it says."""
     rng = np.random.default_rng(1)
     for d in (rng.normal(size=(256, 2000)), np.repeat(rng.normal(size=(1, 2000)), 256, 0), rng.normal(size=(256, 2000)) * np.logspace(-4, 2, 256)[:, None],
               np.tile(rng.normal(size=(8, 2000)), (32, 1)) * 0.17, rng.normal(size=(256, 2000)) ** 9):
         d = d.astype(np.float32)
-        A, F = np.zeros(2000, np.float32), np.zeros(2000, np.float32)
+        A, F = np.zeros((256, 2000), np.float32), np.zeros((256, 2000), np.float32)
+        a = f = np.zeros(2000, np.float32)
         for t in range(256):
-            A = (d[t].astype(np.float64) ** 2 + A).astype(np.float32)
-            F = d[t] * d[t] + F
-            H = 2.0 ** np.floor(np.log2(np.maximum((A * np.float32(1.0005)).astype(np.float64), 1e-30)))
-            assert (np.abs(A.astype(np.float64) - F) <= (2 * (t + 1) + 2) * 2.0 ** -24 * H).all()
+            A[t] = a = (d[t].astype(np.float64) ** 2 + a).astype(np.float32)
+            F[t] = f = d[t] * d[t] + f
+        steps = np.broadcast_to(np.arange(1, 257, dtype=np.int32)[:, None], A.shape)
+        H = 2.0 ** np.floor(np.log2(np.maximum((A * np.float32(1.0005)).astype(np.float64), 1e-30)))
+        off = np.abs(A.astype(np.float64) - F)
+        assert (off <= (2 * steps + 2) * 2.0 ** -24 * H).all()
+        added = fused_limit(A, steps).astype(np.float64) - A
+        assert (2 * off <= added).all()
+        assert (added >= (4 * steps + 4) * 2.0 ** -24 * H).all() and (added <= (4 * steps + 18) * 2.0 ** -24 * H + 2e-30).all()

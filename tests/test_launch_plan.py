@@ -47,13 +47,16 @@ def test_a_cluster_size_that_a_rate_has_not_is_refused(plan):
 
 @pytest.mark.parametrize("K", KS)
 def test_every_shape_is_some_batch_s_and_every_switch_is_tested(plan, K):
-    """No shape is compiled that no batch takes, and the sizes of the GPU test hold both sides of every size at which another
-    shape, or another pair of shapes, takes over (up to two rounds of the largest, the tiles of one chunk)."""
-    lines = plan(*(x for n in range(1, 889) for x in ("encode", K, n, 0)))
-    calls = "\n".join(lines).split("status 0")[:-1]
-    taken = [tuple(re.findall(r"C=\d+ G=\d+", c)) for c in calls]
-    assert {s for t in taken for s in t} == set(plan("shapes", K))
-    switches = [n for n in range(2, 889) if taken[n - 1] != taken[n - 2]]
+    """No shape is compiled that no batch takes, in either form (at K = 3 and 4 the rounded shapes of three to six tiles are those of single passes, the
+    fused ones of one and two those of what a chunk leaves over), and the sizes of the GPU test hold both sides of every size at which another shape, or another pair of shapes, or the other form
+    takes over (up to two rounds of the largest, the tiles of one chunk)."""
+    shape = re.compile(r"(C=\d+ G=\d+) .* (rounded|fused|listed)")
+    of = lambda what: [[" ".join(x) for x in shape.findall(c)] for c in "\n".join(plan(*(x for n in range(1, 1037) for x in (what, K, n, 0)))).split("status 0")[:-1]]
+    encodes, passes = of("encode"), of("pass")
+    assert {s for t in encodes + passes for s in t} - {"C=2 G=1 listed"} == set(plan("shapes", K))
+    assert not any(s.endswith("rounded") for t in encodes[148:] for s in t) if K > 2 else all(s.endswith("rounded") for t in encodes for s in t)
+    assert all(s.endswith("rounded") for t in passes for s in t)
+    switches = [n for n in range(2, 889) if encodes[n - 1] != encodes[n - 2]]
     assert len(switches) >= 10 and {n - 1 for n in switches} | set(switches) <= set(SIZES[K])
 
 
@@ -70,6 +73,16 @@ def test_every_plan_stays_inside_its_scratch(plan, K):
         lines = plan(*(x for n in (1, 2, 7, 8, 15, 16, 17, 31, 64, 100, 101, 443, 888, 1000) for x in ("encode", K, n, size(n))))
         assert lines.count("status 0") == 14 and not [x for x in lines if x.startswith(("outside", "shared"))]
     assert not [x for x in plan("encode", 2, 100, 0, TCQ_FORWARD_KERNEL="cluster16") if x.startswith(("outside", "shared"))]
+
+
+@pytest.mark.parametrize("K", (3, 4))
+def test_spans_of_fused_batches_stay_inside_their_scratch(plan, K):
+    """Batches that go in several spans: scratch sized for fewer tiles than the batch has."""
+    for n, m, spans in ((700, 350, 2), (1000, 888, 2), (2700, 888, 4), (5000, 888, 6)):
+        lines = plan("encode", K, n, int(plan("size", K, m, 0)[0]))
+        walks = [int(re.search(r" n=(\d+) ", x).group(1)) for x in lines if x.startswith("walk")]
+        assert lines[-1] == "status 0" and not [x for x in lines if x.startswith(("outside", "shared"))]
+        assert sum(walks) == 2 * n and sum(x.endswith("listed") for x in lines) == 2 * spans
 
 
 @pytest.mark.parametrize("n,tiles", [(48, 24), (64, 32), (200, 67), (256, 128), (300, 150), (444, 222)])

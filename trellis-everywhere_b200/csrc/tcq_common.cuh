@@ -3,9 +3,14 @@
 //
 // Numerics contract (what makes the encoder bit-identical to the fp32 PyTorch
 // dynamic programme of the reference, src/trellis/qtip.py:147-196):
-//   * every fp32 operation of the path metric is an explicit round-to-nearest
-//     intrinsic (__fsub_rn, __fmul_rn, __fadd_rn), so nothing is contracted into
-//     a fused multiply-add, and the file is compiled with -fmad=false as well;
+//   * the path metric that decides is the one with every fp32 operation rounded by
+//     itself: explicit round-to-nearest operations (__fsub_rn, __fmul_rn, __fadd_rn,
+//     packed ones likewise), which nothing contracts (compiled with -fmad=false as well);
+//   * large batches at K = 3 and 4 are swept with the square and the sum as one
+//     multiply-add (StepForm::kFused).  These metrics differ from the defined ones by a
+//     bounded few ulp: the walk back takes from them only what lies outside that bound,
+//     compares rounded sums where it does not, and has the tile swept again with
+//     rounded operations where that settles nothing (tcq_walk.cuh), so the result is the defined path;
 //   * "infinity" is FLT_MAX / 4 (bit pattern 0x7E7FFFFF), as in qtip.py:159;
 //   * the minimum over the 2^K predecessors keeps the lowest index on ties.
 #pragma once

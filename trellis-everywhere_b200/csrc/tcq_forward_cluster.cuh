@@ -282,6 +282,8 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
             cbv[i][j] = pack2(cb_from_x<CB>(xb + uint32_t((2 * j) * E) * MUL), cb_from_x<CB>(xb + uint32_t((2 * j + 1) * E) * MUL));
     }
 
+    // (a.n and not n in the rounded form, here and in `live` below, and the key loop once more for it: written as one for all forms the compiler orders
+    // the rounded step at K = 2 differently and it takes 2 % longer, 222 / 444 tiles 574 / 1141 us instead of 554 / 1101)
     const long long n = F == StepForm::kListed ? (long long)*ca.list_count : a.n;
     const long long ngroups = ((F == StepForm::kRounded ? a.n : n) + G - 1) / G;
     const long long nclusters = gridDim.x / C;
@@ -324,7 +326,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
         // end), at the end otherwise (804 us for 444 tiles with three a set; 847 and spills in the second half).
         // With fused candidates at K = 3: in the second half for the shapes with three a set (444 tiles 672 us, from the start 704, from the
         // end 722), early with two (296 tiles 469 us, in the second half 488).
-                // Alone on its two SMs a tile at K = 2 has them one edge earlier (74 tiles 264 us, 273 at the end; more tiles: no difference).
+        // Alone on its two SMs a tile at K = 2 has them one edge earlier (74 tiles 264 us, 273 at the end; more tiles: no difference).
         constexpr int kAhead = LU < Q                                ? 0
                                : F == StepForm::kFused && K == 3     ? (GA == 3 ? 5 : 2)
                                : F == StepForm::kRounded && GS == 2 && K == 3 ? R * 5 / 8

@@ -1,6 +1,7 @@
 // The walk back over the metric rows of the cluster step kernel (tcq_forward_cluster.cuh), and what a tile's states become.
 #pragma once
 
+#include <cuda/std/bit>
 #include <type_traits>
 
 #include "tcq_forward.cuh"
@@ -81,9 +82,10 @@ __device__ __forceinline__ uint32_t first_minimum(const float (&c)[N], float bes
 // A by more than (4 t + 4) u H, its F is above that one's F as well (and no tie).  H is taken from the smallest candidate, a little
 // enlarged so that no sum in question reaches 2 H; twelve more u H cover the rounding of the limit itself, and 1e-30 what underflows (512
 // operations, 2^-150 each).  Above 1e37 sums may overflow: such tiles are swept again.
-__device__ __forceinline__ float fused_limit(float best, int t) {
-    const float h = __uint_as_float(__float_as_uint(__fmul_rn(best, 1.0005f)) & 0x7f800000u);
-    return __fadd_rn(__fmaf_rn(h, float(4 * t + 16) * 0x1p-24f, best), 1e-30f);
+// (Plain operators, which the build does not contract: the host computes the same, tests/fused_limit.cu.)
+__host__ __device__ __forceinline__ float fused_limit(float best, int t) {
+    const float h = cuda::std::bit_cast<float>(cuda::std::bit_cast<uint32_t>(best * 1.0005f) & 0x7f800000u);
+    return fmaf(h, float(4 * t + 16) * 0x1p-24f, best) + 1e-30f;
 }
 constexpr float kFusedMax = 1e37f;
 constexpr long long kWalkWaitCycles = 500000000LL;        // of the second group for the first, a quarter of a second where microseconds are due
