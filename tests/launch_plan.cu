@@ -42,7 +42,7 @@ static cudaError_t cluster(int K, const ClusterArgs& ca, int C, int G) {
     const char* const form = ca.form == StepForm::kFused ? "fused" : ca.form == StepForm::kListed ? "listed" : "rounded";
     std::printf("cluster K=%d C=%d G=%d n=%lld steps=%d %s\n", K, C, G, ca.f.n, ca.f.steps, form);
     const bool fused = ca.form == StepForm::kFused, listed = ca.form == StepForm::kListed;
-    if (listed && (C * ca.at_once > 148 || ca.f.n > ca.at_once)) std::printf("outside: more listed tiles than clusters\n");
+    if (listed && (C * ca.at_once > 148 || ca.f.n > G * ca.at_once)) std::printf("outside: more listed tiles than clusters\n");
     use("rows", ca.rows, ca.f.n * ca.nrows * (size_t(4) << (16 - K)));
     if (ca.keys != nullptr) use("keys", ca.keys, ca.f.n * C * 8 * (fused ? kFusedKeys : 1));
     // (a listed tile's overlap lies anywhere in the span, whose walks have said how large it is)

@@ -53,7 +53,7 @@ def test_every_shape_is_some_batch_s_and_every_switch_is_tested(plan, K):
     shape = re.compile(r"(C=\d+ G=\d+) .* (rounded|fused|listed)")
     of = lambda what: [[" ".join(x) for x in shape.findall(c)] for c in "\n".join(plan(*(x for n in range(1, 1037) for x in (what, K, n, 0)))).split("status 0")[:-1]]
     encodes, passes = of("encode"), of("pass")
-    assert {s for t in encodes + passes for s in t} - {"C=2 G=1 listed"} == set(plan("shapes", K))
+    assert {s for t in encodes + passes for s in t} - {"C=2 G=2 listed"} == set(plan("shapes", K))
     assert not any(s.endswith("rounded") for t in encodes[148:] for s in t) if K > 2 else all(s.endswith("rounded") for t in encodes for s in t)
     assert all(s.endswith("rounded") for t in passes for s in t)
     switches = [n for n in range(2, 889) if encodes[n - 1] != encodes[n - 2]]

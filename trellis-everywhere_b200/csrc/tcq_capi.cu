@@ -201,7 +201,7 @@ struct Workspace {
 // tile swept again, 0.2 ms, is a larger part of a call: 148 tiles at K = 3 would gain 4 %.  At K = 2 the metric rows bind as well (a sweep of 444
 // tiles 1115 -> 1022 us), and the longer walk takes most of the gain: 150 tiles 1220 -> 1230 us a call, 1000 tiles 5431 -> 5372.
 constexpr int kFusedFrom = 149;
-constexpr int kListedC = 2;                        // (with four SMs a tile, a few tiles take 0.17 ms instead of 0.25, and a batch of nothing but ties longer)
+constexpr int kListedC = 2, kListedG = 2;          // (with four SMs a tile, a few tiles take 0.17 ms instead of 0.25, and a batch of nothing but such tiles longer)
 constexpr long long kSpan = 1 << 18;               // the full-speed size holds the overlaps of so many tiles
 bool plan_fused(long long n, int K, const Workspace& wk) {
     return K >= 3 && n >= kFusedFrom && wk.part == kT && kernel_asked_for() == 0 && wk.chunk >= (n < 2 * kFusedFrom ? n : 2 * kFusedFrom) && clusters_at_once(kListedC) > 0;
@@ -395,8 +395,8 @@ int listed(int K, int codebook, ForwardArgs f, int walk, TracebackArgs t, const 
     f.bp_steps = walk;
     ClusterArgs ca{f, wk.rows, rows_for(K, walk), f.overlap == nullptr ? wk.keys : nullptr};
     ca.at_once = clusters_at_once(kListedC);
-    if (ca.at_once > wk.chunk) ca.at_once = int(wk.chunk);         // rows of one tile per cluster
-    ca.f.n = f.n < ca.at_once ? f.n : ca.at_once;
+    if (ca.at_once > wk.chunk / kListedG) ca.at_once = int(wk.chunk / kListedG);         // rows of two tiles per cluster
+    ca.f.n = kListedG * (f.n < ca.at_once ? f.n : ca.at_once);
     ca.form = StepForm::kListed;
     ca.list = wk.list;
     ca.list_count = count;
@@ -414,7 +414,7 @@ int listed(int K, int codebook, ForwardArgs f, int walk, TracebackArgs t, const 
     t.t_end = kT;
     t.codebook = codebook;
     ca.walk = t;
-    const cudaError_t err = K == 3 ? launch_forward_cluster<3>(codebook, ca, kListedC, 1, s) : launch_forward_cluster<4>(codebook, ca, kListedC, 1, s);
+    const cudaError_t err = K == 3 ? launch_forward_cluster<3>(codebook, ca, kListedC, kListedG, s) : launch_forward_cluster<4>(codebook, ca, kListedC, kListedG, s);
     return err == cudaSuccess ? TCQ_OK : cuda_fail(err, what);
 }
 

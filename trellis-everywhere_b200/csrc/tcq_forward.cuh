@@ -325,13 +325,14 @@ struct TracebackArgs {
 //   kFused    the square and the sum as one multiply-add: two fp32 instructions where there were three.  The metrics then differ from
 //             the defined ones by a few ulp, within a bound that the walk knows: where no other path comes within it of the one
 //             it is on, the path is the defined one, and where one does the walk settles it with rounded sums or lists the tile (tcq_walk.cuh).
-//   kListed   rounded, for the tiles that walks have listed, with the walk in the same kernel: one cluster takes a tile at a time.
+//   kListed   rounded, for the tiles that walks have listed, with the walk in the same kernel: a cluster takes one tile at a time, or two
+//             where there are more than clusters.
 enum class StepForm : int { kRounded, kFused, kListed };
 
 // Cluster kernel (tcq_forward_cluster.cuh): the pass, and where its metric rows and final minima go.
 struct ClusterArgs {
     ForwardArgs f;              // bp, bp_steps and e_final are not used
-    float* rows;                // [n][nrows][E] out: metric rows (MetricRows), the last nrows of the pass (kListed: those of one tile per cluster)
+    float* rows;                // [n][nrows][E] out: metric rows (MetricRows), the last nrows of the pass (kListed: those of two tiles per cluster)
     int nrows;
     unsigned long long* keys;   // [n][C] out: per-CTA (metric bits << 32 | edge) minima of the final metrics, or nullptr (kFused: [n][C][kFusedKeys])
     int at_once;                // launches: how many such clusters the device runs at once (the grid is no larger)

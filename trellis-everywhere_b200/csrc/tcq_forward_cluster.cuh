@@ -229,7 +229,7 @@ constexpr size_t cluster_smem_bytes() {
 // GA, GB: tiles of the two sets that alternate (GB = 0: one set, for the smallest batches).
 template <int K, int CB, int C, int GA, int GB, int NT, StepForm F>
 __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const ClusterArgs ca) {
-    static_assert(F != StepForm::kListed || (GA == 1 && GB == 0), "one listed tile at a time");
+    static_assert(F != StepForm::kListed || (GA == 1 && GB == 1 && C == 2), "each CTA walks a listed tile");
     using GE = Geo<K>;
     using MR = MetricRows<K>;
     using IT = ClusterItem<K, C, NT>;
@@ -285,9 +285,10 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     // (a.n and not n in the rounded form, here and in `live` below, and the key loop once more for it: written as one for all forms the compiler orders
     // the rounded step at K = 2 differently and it takes 2 % longer, 222 / 444 tiles 574 / 1141 us instead of 554 / 1101)
     const long long n = F == StepForm::kListed ? (long long)*ca.list_count : a.n;
-    const long long ngroups = ((F == StepForm::kRounded ? a.n : n) + G - 1) / G;
     const long long nclusters = gridDim.x / C;
     const long long cluster_id = blockIdx.x / C;
+    const int per = F == StepForm::kListed && n <= nclusters ? 1 : G;      // tiles of a group: while each cluster has one at most, one alone
+    const long long ngroups = ((F == StepForm::kRounded ? a.n : n) + per - 1) / per;
 
     float* row_tile0 = nullptr;                    // metric rows of the group's first tile
     int live = 0;                                  // tiles of the group that exist
@@ -412,14 +413,19 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
     }
 
     for (long long grp = cluster_id; grp < ngroups; grp += nclusters) {
-        const long long tile0 = F == StepForm::kListed ? (long long)ca.list[grp] : grp * G;
-        const long long slot0 = F == StepForm::kListed ? cluster_id : tile0;       // whose rows and keys
-        live = F == StepForm::kListed ? 1 : F == StepForm::kFused ? int(n - tile0 < G ? n - tile0 : G) : int(a.n - tile0 < G ? a.n - tile0 : G);
+        const long long tile0 = grp * per;
+        const long long slot0 = F == StepForm::kListed ? cluster_id * G : tile0;       // whose rows and keys
+        live = F != StepForm::kRounded ? int(n - tile0 < per ? n - tile0 : per) : int(a.n - tile0 < G ? a.n - tile0 : G);
+        const bool second = F != StepForm::kListed || live > 1;        // whether set 1 has a tile
+        auto tile_at = [&](int g) -> long long {
+            if constexpr (F == StepForm::kListed) return ca.list[tile0 + g];
+            else return tile0 + g;
+        };
         row_tile0 = ca.rows + size_t(slot0) * ca.nrows * E;
         // ---- weights and initial metrics (src/trellis/qtip.py:161-165) ----
         for (int i = tid; i < G * kT; i += NT) {
             int t = i & 255;
-            const float x = (i >> 8) < live ? load_weight(a, tile0 + (i >> 8), i & 255, t) : 0.0f;
+            const float x = (i >> 8) < live ? load_weight(a, tile_at(i >> 8), i & 255, t) : 0.0f;
             wv[(i & ~255) | t] = make_float2(x, x);
             if ((a.flags & kFwdCheckFinite) && !isfinite(x) && rank == 0 && a.status != nullptr) atomicOr(a.status, 2u);   // reported, never trapped on
         }
@@ -429,7 +435,7 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
         }
         __syncthreads();
         if (constrained && tid < G) {
-            const int ov = (tid < live ? a.overlap[tile0 + tid] : 0) & (E - 1);
+            const int ov = (tid < live ? a.overlap[tile_at(tid)] : 0) & (E - 1);
             const int qo = ov / HN, ho = ov % HN;                 // metric of edge ov is predecessor qo of butterfly ho
             if (PL::owner(ho) == rank) cost[(size_t(tid) * 2) * EC + qo * HNC + PL::slot(ho)] = 0.0f;
         }
@@ -447,15 +453,15 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
 #pragma unroll 1
         for (int t = 0; t < a.steps; t += 2) {
             const int row1 = MR::row_after(t + 1, a.steps, ca.nrows);
-            if constexpr (GB > 0) step_set(C1{}, C0{}, t, ph ^ 1u, MR::row_after(t, a.steps, ca.nrows), t == 0, true);
+            if constexpr (GB > 0) if (second) step_set(C1{}, C0{}, t, ph ^ 1u, MR::row_after(t, a.steps, ca.nrows), t == 0, true);
             step_set(C0{}, C1{}, t + 1, ph, row1, false, true);
-            if constexpr (GB > 0) step_set(C1{}, C1{}, t + 1, ph, row1, false, true);
+            if constexpr (GB > 0) if (second) step_set(C1{}, C1{}, t + 1, ph, row1, false, true);
             if (t + 2 < a.steps) step_set(C0{}, C0{}, t + 2, ph, MR::row_after(t + 2, a.steps, ca.nrows), false, true);
             ph ^= 1u;
         }
         cluster_wait_relaxed();             // closes the phase opened by the last step_set
         wait_buffer(0, 0, 1u, false);       // the last step wrote the final metrics into buffer 0
-        if constexpr (GB > 0) wait_buffer(1, 0, 1u, false);
+        if constexpr (GB > 0) if (second) wait_buffer(1, 0, 1u, false);
         __syncthreads();
 
         // ---- final metrics live in buffer 0 (an even number of steps), layout [Q][HNC] = edges q*HN + rank*HNC + hl ----
@@ -515,15 +521,15 @@ __global__ void __launch_bounds__(NT, 1) tcq_forward_cluster_kernel(const Cluste
             }
         }
         if (a.final_cost != nullptr && constrained && tid < live) {
-            const int ov = a.overlap[tile0 + tid] & (E - 1);
+            const int ov = a.overlap[tile_at(tid)] & (E - 1);
             const int qo = ov / HN, ho = ov % HN;
-            if (PL::owner(ho) == rank) a.final_cost[tile0 + tid] = cost[(size_t(tid) * 2) * EC + qo * HNC + PL::slot(ho)];
+            if (PL::owner(ho) == rank) a.final_cost[tile_at(tid)] = cost[(size_t(tid) * 2) * EC + qo * HNC + PL::slot(ho)];
         }
         if constexpr (F == StepForm::kListed) {
             __shared__ WalkShared<K, false> walk_shared;
             __threadfence();                        // the rows and keys of every CTA, before one of them walks
             cluster.sync();
-            if (rank == 0 && tid < WalkShape<K>::W * 32) walk_tile<K, CB, K == 3 && C == 2, false, true>(ca.walk, tile0, slot0, walk_shared);
+            if (rank < live && tid < WalkShape<K>::W * 32) walk_tile<K, CB, K == 3 && C == 2, false, true>(ca.walk, tile_at(rank), slot0 + rank, walk_shared);
             __syncwarp();
         }
         cluster.sync();   // nobody may start re-initialising while a neighbour still reads or is written to

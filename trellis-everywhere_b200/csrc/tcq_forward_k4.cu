@@ -6,7 +6,7 @@ namespace tcq {
 namespace {
 template <int CB>
 cudaError_t launch_cluster_cb(const ClusterArgs& ca, int C, int G, cudaStream_t stream) {
-    if (ca.form == StepForm::kListed) return launch_cluster_variant<4, CB, 2, 1, 0, 512, StepForm::kListed>(ca, stream);
+    if (ca.form == StepForm::kListed) return launch_cluster_variant<4, CB, 2, 1, 1, 512, StepForm::kListed>(ca, stream);
     if (ca.form == StepForm::kFused)
         switch (G) {
             case 1: return launch_cluster_variant<4, CB, 2, 1, 0, 512, StepForm::kFused>(ca, stream);
