@@ -5,7 +5,8 @@
 //   encode K N BYTES   tcq_encode_tb of N tiles with BYTES of scratch (0: what tcq_workspace_bytes says)
 //   pass K N BYTES     tcq_viterbi_pass, unconstrained, likewise
 //   size K N 0         what tcq_workspace_bytes says
-//   shapes K           the shapes that a launch may have, by form
+//   shapes K           the shapes that a launch may have
+//   forms K            the same by form
 // Each launch, each call's status and each shape is printed on a line.
 #include <cstdio>
 #include <cstdlib>
@@ -94,6 +95,10 @@ int main(int argc, char** argv) {
             g_failing_queries = std::atoi(argv[i + 1]);
             i += 2;
         } else if (!std::strcmp(argv[i], "shapes")) {
+            const auto [s, n] = shapes(std::atoi(argv[i + 1]));
+            for (int j = 0; j < n; ++j) std::printf("C=%d G=%d\n", s[j].C, s[j].G);
+            i += 2;
+        } else if (!std::strcmp(argv[i], "forms")) {
             const int K = std::atoi(argv[i + 1]);
             for (bool fused : {false, true}) {
                 const auto [s, n] = shapes(K, fused);

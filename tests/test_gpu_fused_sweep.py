@@ -45,7 +45,7 @@ def _both(q, monkeypatch, call):
 @pytest.mark.gpu
 @pytest.mark.parametrize("K", (3, 4))
 @pytest.mark.parametrize("name", NAMES)
-@pytest.mark.parametrize("n", (149, 300, 445, 900, 1000))       # one launch and two, one chunk and two (leaving 12 and 112 tiles over); hundreds of tiles to sweep again in the last
+@pytest.mark.parametrize("n", (149, 300, 445, 900))       # one launch and two, one chunk and two; 450 tiles to sweep again in the last
 def test_codes_are_those_of_the_rounded_operations(monkeypatch, K, name, n):
     from trellis_b200 import qtip as q
     w = _tiles(n, q.codebook_lut(name, "cpu"), 10 * n + K).cuda()
@@ -59,6 +59,13 @@ def test_codes_are_those_of_the_rounded_operations(monkeypatch, K, name, n):
         return wq, err, packed, sse
 
     _both(q, monkeypatch, row_block)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("K", (3, 4))
+def test_a_chunk_that_leaves_a_few_tiles_over(monkeypatch, K):
+    """112 tiles over, in the fused shapes of one and two tiles a cluster (900 above leave 12)."""
+    test_codes_are_those_of_the_rounded_operations(monkeypatch, K, "mcg", 1000)
 
 
 @pytest.mark.gpu
@@ -160,6 +167,21 @@ def test_a_walk_that_does_not_wait_lists_its_tile(K):
     assert lib.tcq_workspace_status(ws.data_ptr(), ws.numel(), n, K, stream) == 0
 
 
+def test_the_bound_between_fused_and_rounded_sums():
+    """|A - F| <= (2 t + 2) u H of the limit (fused_limit), over random, repeated and graded terms; A as the fused operation gives it (the
+    square is exact in 64 bits, the sum there rounds 2^29 times finer)."""
+    rng = np.random.default_rng(1)
+    for d in (rng.normal(size=(256, 2000)), np.repeat(rng.normal(size=(1, 2000)), 256, 0), rng.normal(size=(256, 2000)) * np.logspace(-4, 2, 256)[:, None],
+              np.tile(rng.normal(size=(8, 2000)), (32, 1)) * 0.17, rng.normal(size=(256, 2000)) ** 9):
+        d = d.astype(np.float32)
+        A, F = np.zeros(2000, np.float32), np.zeros(2000, np.float32)
+        for t in range(256):
+            A = (d[t].astype(np.float64) ** 2 + A).astype(np.float32)
+            F = d[t] * d[t] + F
+            H = 2.0 ** np.floor(np.log2(np.maximum((A * np.float32(1.0005)).astype(np.float64), 1e-30)))
+            assert (np.abs(A.astype(np.float64) - F) <= (2 * (t + 1) + 2) * 2.0 ** -24 * H).all()
+
+
 @pytest.fixture(scope="module")
 def fused_limit(tmp_path_factory):
     """fused_limit of tcq_walk.cuh: (smallest candidates, steps) -> limits."""
@@ -175,7 +197,7 @@ def fused_limit(tmp_path_factory):
     return run
 
 
-def test_the_bound_between_fused_and_rounded_sums(fused_limit):
+def test_the_limit_holds_the_bound_between_fused_and_rounded_sums(fused_limit):
     """|A - F| <= (2 t + 2) u H, and no more than half of what fused_limit adds, so that of two candidates one of which is beyond the other's limit
     that one is the larger by the rounded sums too; over random, repeated and graded terms.  A as the fused operation gives it (the
     square is exact in 64 bits, the sum there rounds 2^29 times finer).  The limit adds no more than it says."""

@@ -47,13 +47,25 @@ def test_a_cluster_size_that_a_rate_has_not_is_refused(plan):
 
 @pytest.mark.parametrize("K", KS)
 def test_every_shape_is_some_batch_s_and_every_switch_is_tested(plan, K):
+    """No shape is compiled that no batch takes, and the sizes of the GPU test hold both sides of every size at which another
+    shape, or another pair of shapes, takes over (up to two rounds of the largest, the tiles of one chunk)."""
+    lines = plan(*(x for n in range(1, 889) for x in ("encode", K, n, 0)))
+    calls = "\n".join(lines).split("status 0")[:-1]
+    taken = [tuple(re.findall(r"C=\d+ G=\d+", c)) for c in calls]
+    assert {s for t in taken for s in t} == set(plan("shapes", K))
+    switches = [n for n in range(2, 889) if taken[n - 1] != taken[n - 2]]
+    assert len(switches) >= 10 and {n - 1 for n in switches} | set(switches) <= set(SIZES[K])
+
+
+@pytest.mark.parametrize("K", KS)
+def test_every_form_is_some_batch_s_and_every_switch_is_tested(plan, K):
     """No shape is compiled that no batch takes, in either form (at K = 3 and 4 the rounded shapes of three to six tiles are those of single passes, the
     fused ones of one and two those of what a chunk leaves over), and the sizes of the GPU test hold both sides of every size at which another shape, or another pair of shapes, or the other form
     takes over (up to two rounds of the largest, the tiles of one chunk)."""
     shape = re.compile(r"(C=\d+ G=\d+) .* (rounded|fused|listed)")
     of = lambda what: [[" ".join(x) for x in shape.findall(c)] for c in "\n".join(plan(*(x for n in range(1, 1037) for x in (what, K, n, 0)))).split("status 0")[:-1]]
     encodes, passes = of("encode"), of("pass")
-    assert {s for t in encodes + passes for s in t} - {"C=2 G=2 listed"} == set(plan("shapes", K))
+    assert {s for t in encodes + passes for s in t} - {"C=2 G=2 listed"} == set(plan("forms", K))
     assert not any(s.endswith("rounded") for t in encodes[148:] for s in t) if K > 2 else all(s.endswith("rounded") for t in encodes for s in t)
     assert all(s.endswith("rounded") for t in passes for s in t)
     switches = [n for n in range(2, 889) if encodes[n - 1] != encodes[n - 2]]
