@@ -120,7 +120,7 @@ struct WalkShared {
     int go_on;                                     // the second group's orders
     int trips;                                     // taken by the first group (kAllTrips: the walk is over and `cost` complete), published (tcq_handoff.cuh)
     int verdict;                                   // of the second group on the marks: kOther | kApart
-    static constexpr int kAllTrips = 1 << 20, kOther = 1, kApart = 2;
+    static constexpr int kAllTrips = 1 << 20, kTold = 4, kOther = 1, kApart = 2;      // (told of every trip, a walk takes 4 to 7 us longer)
 };
 
 // The walk over one tile, by WalkShape<K>::W whole warps (threads 0 .. 32 W - 1 of the CTA), from the rows and partial minima of `slot`.
@@ -427,7 +427,7 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
             if (tid == 0 && (!first || tau + i >= 0)) st[tau + i] = uint16_t(s);
             e = s >> K;
         }
-        if (FUSED && behind && tid == 0 && j % 4 == 3) handoff_publish(sh.trips, j + 1);   // (every trip: 4 to 7 us a walk)
+        if (FUSED && behind && tid == 0 && j % sh.kTold == sh.kTold - 1) handoff_publish(sh.trips, j + 1);
     };
     auto walk = [&]() __attribute__((always_inline)) {     // back to step `lo`, or a little further
         for (; tau > 0 && tau + D > lo; ++j, tau -= D) take(row_trip(j & 1, std::false_type{}, tau, e, j), false);
@@ -496,7 +496,15 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
                 return every != 0;
             }
         } follower;
-        auto taken = [&](int trips) -> bool { return who == 0 || handoff_wait(follower, sh.trips, trips, a.hurry ? 0 : kWalkWaitCycles); };
+        // (The group waits for the next count that is told and remembers it: a barrier for that many trips.)
+        int seen = 0;
+        auto taken = [&](int trips) -> bool {
+            if (who == 0 || trips <= seen) return true;
+            const int told = (trips + sh.kTold - 1) / sh.kTold * sh.kTold;
+            if (!handoff_wait(follower, sh.trips, told, a.hurry ? 0 : kWalkWaitCycles)) return false;
+            seen = told;
+            return true;
+        };
         bool apart = false;                        // another path does not meet the one found as far as that is known
         int trips = 0;
         auto any_trip = [&](int tau, uint32_t e) -> uint32_t {
