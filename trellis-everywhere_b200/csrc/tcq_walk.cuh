@@ -102,7 +102,8 @@ template <int K> struct Ring {
 template <int K, bool FUSED>
 struct WalkShared {
     static constexpr int D = MetricRows<K>::D, W = WalkShape<K>::W, N1 = MetricRows<K>::NA >> K, N2 = D >= 3 ? N1 >> K : 1;
-    static constexpr int kMaxMarks = 16, kMaxTodo = 8;
+    // (kMaxTrips along other paths: of 100 000 Gaussian tiles one that was settled took more, and tiles of zeros at K = 4 take four times as many in vain)
+    static constexpr int kMaxMarks = 16, kMaxTodo = 8, kMaxTrips = 128;
     struct Walker {
         uint16_t st[kT];
         float val1[2][N1];                         // first level: minima and their q, double buffered over trips
@@ -514,7 +515,7 @@ __device__ __forceinline__ void walk_tile(const TracebackArgs& a, long long tile
         // Another path, from `e` before step t, the first of a trip: back to where it meets the path found, or to a beginning as good.
         // Returns the step before which they meet, or -1.
         auto follow = [&](uint32_t e, int t) -> int {
-            while (t > lo && ++trips <= 512) {
+            while (t > lo && ++trips <= sh.kMaxTrips) {
                 t -= D;
                 const uint32_t whole = any_trip(t, e);
                 if ((whole & kNear) || !taken((a.t_end - t + D - 1) / D)) return -1;
