@@ -31,8 +31,9 @@ Printed: ONE JSON line on rank 0 with
             forward-only entry point, against the fp32/INT lane-issue ceiling;
   cpu_baseline  the CPU oracle (a C port of the reference's PyTorch dynamic programme)
             on a bounded sample of the same tiles, all host threads (N = 1 only);
-  parity    64 tiles spread over the last timed step's output and 64 tiles of the launches the
-            roofline leg times, checked bit for bit against the CPU oracle after the timing.
+  parity    64 tiles spread over the last timed step's output and the state paths of 64 tiles of a
+            full chunk through the pass-level entry point, checked bit for bit against the CPU
+            oracle after the timing.
 
 ``--impl reference`` times the reference's own ``viterbi_tb`` (fp32 PyTorch DP, the staged copy under
 ``oracle/_ref``) on the host cores, rank 0 only, on tiles of the same workload, and prints the same kind of
@@ -272,7 +273,7 @@ def run_reference_triton(args) -> None:
 
 # ------------------------------------------------------------------------------------ B200 arm
 def check_parity(torch, qtip, lib, _lib, tiles, last, dev, cid) -> dict:
-    """After the timing: the last timed step's output and the roofline leg's launches against the CPU oracle."""
+    """After the timing: the last timed step's output and the two passes of one chunk against the CPU oracle."""
     import numpy as np
     from oracle import oracle as O
     O.build()
@@ -284,8 +285,8 @@ def check_parity(torch, qtip, lib, _lib, tiles, last, dev, cid) -> dict:
     ok_packed = np.array_equal(last.packed[idx].cpu().numpy().view(np.uint32), O.pack_bits(bits, K_BITS))
     ok_dq = np.array_equal(last.dq[idx].cpu().numpy().view(np.uint32), dq.view(np.uint32))
     ok_sse = np.array_equal(last.sse[idx].cpu().numpy().view(np.uint32), sse.view(np.uint32))
-    # the launches the roofline leg times: one full chunk through the pass-level entry point (the same launch code;
-    # candidates are rounded operation by operation there, which the timed launches leave to the walk), states of 64 spread tiles against the oracle's passes
+    # one full chunk through the pass-level entry point, whose candidates are rounded operation by operation (the roofline leg's launches have
+    # fused ones, and leave it to the walk to find the path of the rounded sums): states of 64 spread tiles against the oracle's passes
     chunk = min(n, 6 * torch.cuda.get_device_properties(dev).multi_processor_count)
     s1 = qtip.viterbi_pass_b200(tiles[:chunk], K_BITS, None, cid, roll=128)
     jdx = torch.linspace(0, chunk - 1, min(64, chunk), device=dev).round().long()
@@ -517,9 +518,9 @@ def run_b200(args, rank: int, local_rank: int, world: int) -> None:
                            "compare/select pipe beside them",
             "launch_ms": {"pass1": kern_ms[0], "pass2": kern_ms[1]}, "tiles_per_launch": chunk,
             "frac_at_sampled_clock": (achieved / (sms * 128 * ck["sm_mhz"] * 1e6)) if ck.get("sm_mhz") else None,
-            # ncu dram__bytes_read+write of a 444-tile launch pair against its metric rows
-            # (profiles/step_kernel_k3_3inst_444tiles_ncu_counters.md), scaled here by the tiles per launch
-            "traffic": 0.94 * row_bytes,
+            # ncu dram__bytes_read+write of an 888-tile launch pair against its metric rows
+            # (profiles/step_kernel_k3_fused_candidates_ncu_counters.md), scaled here by the tiles per launch
+            "traffic": 0.98 * row_bytes,
             "hbm": {"algorithmic_bytes_per_launch": row_bytes, "achieved_GBps": row_bytes / (avg_kernel_ms * 1e-3) / 1e9,
                     "peak_GBps": peaks.get("hbm_gbs"), "note": "path metrics of every third step (K = 3)"},
         }

@@ -124,7 +124,7 @@ def test_batches_of_several_spans(monkeypatch, K, n, size_for):
 @pytest.mark.gpu
 @pytest.mark.parametrize("K", (3, 4))
 def test_what_the_walk_settles_and_what_it_lists(K):
-    """Of 20 000 Gaussian tiles 800 have a second edge at the end of pass 1, some hundred a marked node and some tens are walked back to the beginning:
+    """Of 20 000 Gaussian tiles 400 have a second edge at the end of pass 1, a hundred or two a marked node in a pass and some twenty are walked back to the beginning:
     no more than a few are listed, so each of these is settled and not left to the second sweep.  Tiles whose costs are above 1e37 are all listed
     (of ties alone that does not hold in both passes: over zeros the free pass has one best path)."""
     from trellis_b200 import qtip as q

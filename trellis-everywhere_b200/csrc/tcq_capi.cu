@@ -196,10 +196,10 @@ struct Workspace {
     int* counts;                // their numbers after the walks of pass 1 and of pass 2
 };
 
-// Batches from here on are swept with fused candidates, and the tiles whose path that does not settle again (one in a thousand, by a
+// Batches from here on are swept with fused candidates, and the tiles whose path that does not settle again (one Gaussian tile in 10 000, by a
 // kernel of its own after the walks of each pass).  Smaller ones are bound by the exchange between SMs and not by arithmetic, and there a
-// tile swept again, 0.2 ms, is a larger part of a call: 148 tiles at K = 3 would gain 4 %.  At K = 2 the metric rows bind as well (a sweep of 444
-// tiles 1115 -> 1022 us), and the longer walk takes most of the gain: 150 tiles 1220 -> 1230 us a call, 1000 tiles 5431 -> 5372.
+// tile swept again, 0.25 ms, is a larger part of a call: 148 tiles at K = 3 would gain 4 %.  At K = 2 a sweep gains less (444
+// tiles 1115 -> 1022 us), and the longer walk takes most of it: 150 tiles 1220 -> 1230 us a call, 1000 tiles 5431 -> 5372.
 constexpr int kFusedFrom = 149;
 constexpr int kListedC = 2, kListedG = 2;          // (with four SMs a tile, a few tiles take 0.17 ms instead of 0.25, and a batch of nothing but such tiles longer)
 constexpr long long kSpan = 1 << 18;               // the full-speed size holds the overlaps of so many tiles

@@ -16,7 +16,7 @@
 // clocks, and leaves it to the walk to find the path of the rounded sums (sweeps of 296 / 370 / 444 tiles: K = 3 566 / 697 / 806 -> 468 / 562 / 671 us,
 // K = 4 559 / 696 / 817 -> 477 / 569 / 674; what limits it then is operands of packed instructions as well as issue: fewer
 // instructions with the same operands are no faster).  kListed is the rounded form for the tiles that walks have listed, one at a time
-// on two SMs, with the walk behind it in the same launch: 3 us when there is none.
+// on two SMs or, where there are more than clusters, two, with the walks behind it in the same launch: 3 us when there is none.
 //
 //   * CTA r owns the butterflies h in [r * HN/C, (r+1) * HN/C): it needs the path metrics
 //     old[q * HN + h] for all q (E/C values per tile, in ITS shared memory, layout [Q][HN/C])
@@ -184,7 +184,7 @@ struct ClusterPlace {
 
 // Two CTAs at K = 3: the owner is the majority of h9 h6 h3.  A step moves these bits up by one place and brings in one new one, so
 // most majorities stay: 1/4 of the metrics cross between the SMs, where 1/2 do with an owner that is a bit of its own (or any sum of
-// bits modulo two).  Sweep of 74 / 148 / 222 / 296 / 370 / 444 tiles: 230 / 363 / 469 / 596 / 727 / 828 -> 209 / 340 / 449 / 566 / 697 / 809 us;
+// bits modulo two).  Sweep of 74 / 148 / 222 / 296 / 370 / 444 tiles: 230 / 363 / 469 / 596 / 727 / 828 -> 207 / 339 / 449 / 566 / 697 / 806 us;
 // with nothing sent at all 183 / 330 / 433 / 556 / 688 / 801.  (At K = 2, majority of h11 h9 h7: 564 -> 568 us for 222 tiles, 561 with
 // nothing sent: there the network does not bind.)
 //   slot, from the top: number of the pattern h9 h6 h3 among those with its majority, h2, h8 h7 h5 h4, h1, h0 flipped by h2.

@@ -128,15 +128,15 @@ struct WalkShared {
 // OTHER: the rows' ancestors lie as in MetricRows::other_pos.  COHERENT: the rows were written by this kernel.
 //
 // FUSED: the metrics are those of fused candidates.  A node on the path where a second candidate is within fused_limit of the smallest marks
-// its trip; nothing else is done on the way.  Without a mark (97 tiles of 100) the path is the defined one.  With marks every such
+// its trip; nothing else is done on the way.  Without a mark (99 Gaussian tiles of 100) the path is the defined one.  With marks every such
 // candidate's own path is walked back until it meets the path found.  In the pass that looks for the overlap that is all as long as
 // they meet before the middle of the tile: the overlap is the same either way.  Otherwise, and in the other pass, the two are compared by
-// their rounded sums from where they meet (one tile in 200 of the first pass is walked back to its beginning for that).
+// their rounded sums from where they meet (one tile in 800 of the first pass is walked back to its beginning for that).
 // Other paths cost as long as they are to walk, so a second group of warps walks them at the same time: where the pass may end with one
-// of two edges (one tile in 25 of the first pass) it walks from the second edge; otherwise it goes behind the first group and takes up
+// of two edges (one tile in 36 to 75 of the first pass) it walks from the second edge; otherwise it goes behind the first group and takes up
 // the trips that get marked.  Its waits for the first group are bounded by the clock; a tile whose wait runs out is listed.
 // What this does not settle (marks on the other path too, another winner, more than a few marks, costs above 1e37 or not a
-// number) lists the tile in a.again: one tile in 10 000, and every tile of ties, such as one of zeros.
+// number) lists the tile in a.again: one Gaussian tile in 10 000, and some tiles of ties, such as one of zeros in the second pass.
 //
 // RING: rows come to shared memory ahead of the walk; `ring` is Ring<K>::kBytes of it.
 template <int K, int CB, bool OTHER, bool FUSED, bool COHERENT, bool RING = false>
